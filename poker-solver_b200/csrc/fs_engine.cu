@@ -805,7 +805,7 @@ class Solve {
     // then its reach; the root strategy is taken before the last traverser's
     // pass (the reference's last regret matching)
     cudaError_t iteration(bool keep_sigma) {
-        cudaError_t e = launch_bump(diter, stream);
+        cudaError_t e = launch_bump(diter, 1, stream);
         for (int t = 0; t < 2 && e == cudaSuccess; ++t) {
             if (t == 1) {
                 e = launch_root_strategy(c, P.first_edge[0], P.root_na, -1, P.H[P.root_player], dsnap, stream);

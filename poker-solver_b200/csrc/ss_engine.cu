@@ -197,7 +197,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     Blob b;
     size_t o_heads[SS_MAX_PLAYERS][TK_COUNT] = {};
     size_t o_reach[SS_MAX_PLAYERS], o_cfv[SS_MAX_PLAYERS], o_term[SS_MAX_PLAYERS][TK_COUNT],
-        o_rootfr[SS_MAX_PLAYERS];
+        o_rootfr[SS_MAX_PLAYERS], o_tree[SS_MAX_PLAYERS];
     for (int p = 0; p < np; ++p) {
         std::vector<ReachItem> all;
         for (auto &lv : P.reach_levels[p]) {
@@ -233,6 +233,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
             if (!P.term_heads[p][k].empty()) o_heads[p][k] = b.add(P.term_heads[p][k]);
         }
         o_rootfr[p] = b.add(P.root_fr[p]);
+        o_tree[p] = b.add(P.tree[p].blob);
     }
     const size_t o_fr_off = b.add(P.fr_off);
     const size_t o_fr_items = b.add(P.fr_items);
@@ -268,6 +269,9 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
                                                           : reinterpret_cast<const int *>(dbase + o_heads[p][k]);
         }
         root_fr[p] = reinterpret_cast<const int *>(dbase + o_rootfr[p]);
+        const TreePass &T = P.tree[p];
+        tree[p] = TreeRef{dbase + o_tree[p], static_cast<int>(T.blob.size()), T.o_items, T.o_chains, T.o_reach,
+                          T.o_rows, static_cast<int>(T.stages.size()), T.max_chains, T.threads};
     }
     dec_fe = reinterpret_cast<const int *>(dbase + o_dfe);
     dec_na = reinterpret_cast<const int *>(dbase + o_dna);

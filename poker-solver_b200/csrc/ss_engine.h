@@ -111,6 +111,10 @@ void inline_frontier(CfvItem &it, const std::vector<int> &fr_off, const std::vec
 // total is long: several warps share each of its hand chunks.
 constexpr int kCfvLongFrontier = 48;
 
+// warps that share one hand chunk of a value/regret item with a long frontier
+// (k_cfv), chains per edge of such an item (k_tree)
+constexpr int kCfvSplit = 4;
+
 // Order one level's value/regret items short, then long (stable within each
 // class); returns the number of long items.
 template <class Item, class FrontierRows>
@@ -118,6 +122,60 @@ inline int order_cfv_level(std::vector<Item> &v, FrontierRows rows) {
     auto mid = std::stable_partition(v.begin(), v.end(), [&](const Item &it) { return rows(it) < kCfvLongFrontier; });
     return static_cast<int>(v.end() - mid);
 }
+
+// One player's pass over the small levels of its tree in one launch (k_tree):
+// its value/regret levels bottom-up, then its reach levels top-down.  Every
+// hand is independent of the others there, so a block owns kTreeHands hands
+// and orders the levels with its own barriers instead of launches.  The pass
+// is a list of stages; a value/regret level is cut into tiles of at most
+// kTreeChains row chains.  A chain is the sum of the frontier rows
+// k0 + i * stride, i < n, of the pass's row list, in that order: one per edge, or kCfvSplit
+// interleaved ones per edge of an item with a long frontier, whose partial
+// sums are added in order -- the summation order of k_cfv in both cases.
+constexpr int kTreeHands = 8;
+constexpr int kTreeThreads = 1024;
+constexpr int kTreeChains = 1024;
+// The pass's tables are one blob (stages, items, chains, reach items, rows):
+// a block copies it to shared memory when it fits kTreeResident bytes.
+struct TreeChain {
+    int k0;       // into the pass's row list
+    int ns;       // rows << 4 | stride
+};
+struct alignas(16) TreeItem {
+    int first_edge, na, frozen, node;
+    float scale;
+    int part0;    // its first chain within the tile; edge a's chains follow at part0 + a * split
+    int split;    // chains per edge: 1 or kCfvSplit
+    int pad;
+};
+struct alignas(16) TreeReach {
+    int first_edge, na, parent_row, frozen;
+};
+enum TreeStageKind : int { TS_VALUE = 0, TS_REACH = 1 };
+struct alignas(16) TreeStage {
+    int kind;
+    int i0, i1;   // TS_VALUE: tree items; TS_REACH: reach items
+    int c0, c1;   // TS_VALUE: the tile's chains
+    int pad[3];
+};
+constexpr int kTreeResident = 64 * 1024;
+struct TreePass {
+    std::vector<TreeStage> stages;
+    std::vector<TreeChain> chains;
+    std::vector<TreeItem> items;
+    std::vector<TreeReach> reach;
+    std::vector<int> rows;
+    int cfv_from = 0;    // value/regret levels below this one have launches of their own (k_cfv)
+    int reach_to = 0;    // so have the reach levels from this one on (k_reach)
+    int threads = 0;     // block size, for the widest stage
+    int max_chains = 0;  // widest tile
+    // the blob and the offsets of its parts in it (bytes, multiples of 16)
+    std::vector<char> blob;
+    int o_items = 0, o_chains = 0, o_reach = 0, o_rows = 0;
+};
+void build_tree_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const std::vector<int> &cfv_nlong,
+                     const std::vector<std::vector<ReachItem>> &reach_levels, const std::vector<int> &fr_off,
+                     const std::vector<int> &fr_items, TreePass *out);
 
 // A three-way showdown's rank-order sweep is cut into at most this many runs
 // of tie groups, each swept by its own block from a directly computed state.
@@ -230,6 +288,7 @@ struct Plan {
     // with long frontiers come last, cfv_nlong of them
     std::vector<std::vector<CfvItem>> cfv_levels[SS_MAX_PLAYERS];
     std::vector<int> cfv_nlong[SS_MAX_PLAYERS];
+    TreePass tree[SS_MAX_PLAYERS];     // the small levels of both, in one launch per traverser
     // two-opponent terminals (TK_CR2): the items that start work (group leaders
     // that no chain head computes); the launch gets one block each.  (One block
     // per item, as for every other kind, keeps the one-opponent launches

@@ -211,7 +211,7 @@ __device__ __forceinline__ CfvHead cfv_head(const CfvItem *p) {
 template <int S>
 __global__ void __launch_bounds__(kCfvThreads, 8) k_cfv(DevCtx c0, const DevCtx *__restrict__ ctxs,
                                                      const CfvItem *__restrict__ items, int nchunk, int Hl,
-                                                     int trav) {
+                                                     int trav, int iter_add) {
     wait_prior_grid();
     const int it = blockIdx.x / nchunk;
     const int ch = blockIdx.x - it * nchunk;
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kCfvThreads, 8) k_cfv(DevCtx c0, const DevCtx 
             v1 += sigma(a, r.y, s1, inv1) * ev[a].y;
         }
     }
-    const int t = *V.iter;
+    const int t = *V.iter + iter_add;
     const float d = static_cast<float>(t) / (static_cast<float>(t) + 1.0f);
     const float w = static_cast<float>(t);
 #pragma unroll
@@ -389,6 +389,171 @@ __global__ void __launch_bounds__(kCfvThreads, 8) k_cfv(DevCtx c0, const DevCtx 
     // scale 1 on a single street (exact: the row equals v); below chance
     // nodes the row carries their 1 / cards weights for the parent's frontier
     st2(V.val + static_cast<size_t>(I.node) * HS + h0, make_float2(v0 * I.scale, v1 * I.scale));
+}
+
+// --------------------------------------------------------------------------
+// One player's value/regret levels (bottom-up) and reach levels (top-down)
+// near the root in one launch.  No hand depends on another here, so a block
+// owns 8 hands (one 32-byte sector of every row) and walks the levels between
+// its own barriers: a launch per level costs about 3.6 us of dependent-launch
+// latency, a stage of this kernel about one chain of loads.  Threads are
+// (slot, hand) pairs: in a value stage a slot sums one row chain into shared
+// memory, then a slot updates one item; in a reach stage a slot takes one
+// item.  Summation orders and expressions are those of k_cfv and k_reach.
+// What is left is the latency of the row loads, so everything that no kernel
+// writes (the pass's tables) comes to shared memory before the wait for the
+// previous kernel where it fits (kResident), the next chain's rows are loaded
+// while the last one's are added, and regret rows are prefetched into L1.
+// --------------------------------------------------------------------------
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+template <bool kResident>
+__global__ void __launch_bounds__(kTreeThreads, 1) k_tree(DevCtx c, TreeRef T, int H, int iter_add) {
+    extern __shared__ __align__(16) char smem[];
+    float *part = reinterpret_cast<float *>(smem);   // [chain of the tile][kTreeHands]
+    const char *tab = T.blob;
+    if constexpr (kResident) {
+        int4 *dst = reinterpret_cast<int4 *>(smem + static_cast<size_t>(T.max_chains) * kTreeHands * sizeof(float));
+        const int4 *src = reinterpret_cast<const int4 *>(T.blob);
+        for (int i = threadIdx.x; i < T.bytes / 16; i += blockDim.x) dst[i] = __ldg(src + i);
+        tab = reinterpret_cast<const char *>(dst);
+    }
+    wait_prior_grid();
+    if constexpr (kResident) __syncthreads();
+    const TreeStage *stages = reinterpret_cast<const TreeStage *>(tab);
+    const TreeItem *items = reinterpret_cast<const TreeItem *>(tab + T.o_items);
+    const int2 *chains = reinterpret_cast<const int2 *>(tab + T.o_chains);
+    const int4 *reach_items = reinterpret_cast<const int4 *>(tab + T.o_reach);
+    const int *rows = reinterpret_cast<const int *>(tab + T.o_rows);
+    const int hand = threadIdx.x & (kTreeHands - 1), slot = threadIdx.x / kTreeHands;
+    const int slots = blockDim.x / kTreeHands;
+    const int h = blockIdx.x * kTreeHands + hand;
+    const bool act = h < H;
+    const size_t HS = static_cast<size_t>(c.HS);
+    const float *val = c.val + h;
+    float *R = c.R + h, *S = c.S + h, *reach = c.reach + h;
+    const int t = *c.iter + iter_add;
+    const float d = static_cast<float>(t) / (static_cast<float>(t) + 1.0f);
+    const float w = static_cast<float>(t);
+    for (int si = 0; si < T.n_stages; ++si) {
+        const int4 sa = *reinterpret_cast<const int4 *>(stages + si);
+        if (sa.x == TS_VALUE) {
+            const int c0 = sa.w, c1 = stages[si].c1;
+            if (act) {
+                // this slot's first item: its regret and strategy-sum rows
+                if (sa.y + slot < sa.z) {
+                    const TreeItem &I = items[sa.y + slot];
+                    const size_t off = static_cast<size_t>(I.first_edge) * HS;
+                    for (int a = 0; a < I.na; ++a) {
+                        prefetch_l1(R + off + a * HS);
+                        prefetch_l1(S + off + a * HS);
+                    }
+                }
+                // rows i .. i + 7 of a chain (+0 past its end: the sum is the row-order sum)
+                auto load8 = [&](int2 C, int i, float x[8]) {
+                    const int n = C.y >> 4, st = C.y & 15;
+                    const int *fr = rows + C.x;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        x[j] = i + j < n ? val[static_cast<size_t>(fr[(i + j) * st]) * HS] : 0.f;
+                };
+                float x[8];
+                int ch = c0 + slot;
+                int2 C = ch < c1 ? chains[ch] : make_int2(0, 0);
+                load8(C, 0, x);
+                while (ch < c1) {
+                    const int nx = ch + slots;
+                    const int2 Cn = nx < c1 ? chains[nx] : make_int2(0, 0);
+                    float y[8];
+                    load8(Cn, 0, y);
+                    float e = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) e += x[j];
+                    for (int i = 8; i < C.y >> 4; i += 8) {
+                        load8(C, i, x);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) e += x[j];
+                    }
+                    part[(ch - c0) * kTreeHands + hand] = e;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) x[j] = y[j];
+                    C = Cn;
+                    ch = nx;
+                }
+            }
+            __syncthreads();
+            if (act) {
+                for (int it = sa.y + slot; it < sa.z; it += slots) {
+                    const int4 I0 = reinterpret_cast<const int4 *>(items + it)[0];
+                    const int4 I1 = reinterpret_cast<const int4 *>(items + it)[1];
+                    const int na = I0.y, frozen = I0.z, split = I1.z;
+                    const float *pp = part + I1.y * kTreeHands + hand;
+                    float *Rh = R + static_cast<size_t>(I0.x) * HS, *Sh = S + static_cast<size_t>(I0.x) * HS;
+                    float r[SS_MAX_ACTIONS], ev[SS_MAX_ACTIONS], sm[SS_MAX_ACTIONS];
+                    float sum = 0.f;
+#pragma unroll
+                    for (int a = 0; a < SS_MAX_ACTIONS; ++a)
+                        if (a < na) {
+                            r[a] = Rh[a * HS];
+                            sm[a] = Sh[a * HS];
+                        }
+#pragma unroll
+                    for (int a = 0; a < SS_MAX_ACTIONS; ++a)
+                        if (a < na) {
+                            float e = pp[a * split * kTreeHands];
+                            if (split > 1)
+                                for (int k = 1; k < kCfvSplit; ++k) e += pp[(a * split + k) * kTreeHands];
+                            ev[a] = e;
+                            sum += r[a] > 0.f ? r[a] : 0.f;
+                        }
+                    const float uni = 1.0f / static_cast<float>(na);
+                    const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+                    auto sigma = [&](int a) {
+                        if (frozen >= 0) return a == frozen ? 1.0f : 0.0f;
+                        return sum > 0.f ? (r[a] > 0.f ? r[a] : 0.f) * inv : uni;
+                    };
+                    float v = 0.f;
+#pragma unroll
+                    for (int a = 0; a < SS_MAX_ACTIONS; ++a)
+                        if (a < na) v += sigma(a) * ev[a];
+#pragma unroll
+                    for (int a = 0; a < SS_MAX_ACTIONS; ++a)
+                        if (a < na) {
+                            Rh[a * HS] = (r[a] + (ev[a] - v)) * d;
+                            Sh[a * HS] = sm[a] + w * sigma(a);
+                        }
+                    c.val[static_cast<size_t>(I0.w) * HS + h] = v * __int_as_float(I1.x);
+                }
+            }
+        } else if (act) {
+            for (int it = sa.y + slot; it < sa.z; it += slots) {
+                const int4 I = reach_items[it];   // first_edge, na, parent_row, frozen
+                const float *Rh = R + static_cast<size_t>(I.x) * HS;
+                float *out = reach + static_cast<size_t>(I.x) * HS;
+                const float pr = reach[static_cast<size_t>(I.z) * HS];
+                float r[SS_MAX_ACTIONS], sum = 0.f;
+#pragma unroll
+                for (int a = 0; a < SS_MAX_ACTIONS; ++a)
+                    if (a < I.y) {
+                        r[a] = Rh[a * HS];
+                        sum += r[a] > 0.f ? r[a] : 0.f;
+                    }
+                const float uni = 1.0f / static_cast<float>(I.y);
+                const bool pos = sum > 0.f;
+                const float inv = pos ? 1.0f / sum : 0.f;
+#pragma unroll
+                for (int a = 0; a < SS_MAX_ACTIONS; ++a)
+                    if (a < I.y) {
+                        float s = pos ? (r[a] > 0.f ? r[a] : 0.f) * inv : uni;
+                        if (I.w >= 0) s = (a == I.w) ? 1.0f : 0.0f;
+                        out[a * HS] = pr * s;
+                    }
+            }
+        }
+        // the stage's value and reach rows are read by other slots of the
+        // block in the next stages, and its partial sums are overwritten
+        __syncthreads();
+    }
 }
 
 // --------------------------------------------------------------------------
@@ -1117,9 +1282,9 @@ __global__ void __launch_bounds__(kTermThreads, sizeof(T) == 4 ? 5 : 2) k_term_c
 #include "ss_cr2_tc.cuh"
 
 template <class T>
-constexpr size_t cr1_gather_smem(int HS) {
-    return (static_cast<size_t>(HS) + 4) * sizeof(T) + static_cast<size_t>(HS) * 4 + 64 * 8 + 64 * 4 +
-           3 * kTermGroupMax * 4 + 2 * 16 + 8 * 16;
+__host__ __device__ constexpr size_t cr1_gather_smem(int HS) {
+    return ((static_cast<size_t>(HS) + 4) * sizeof(T) + static_cast<size_t>(HS) * 4 + 64 * 8 + 64 * 4 +
+            3 * kTermGroupMax * 4 + 2 * 16 + 8 * 16 + 15) / 16 * 16;
 }
 
 // One counted opponent over the dense deck, for ranges without a repeated
@@ -1129,12 +1294,11 @@ constexpr size_t cr1_gather_smem(int HS) {
 // compatible positive-reach opponent hands N - n(a) - n(b) + [f(h) > 0]
 // decides a value of exactly 0.  One block per group of terminals sharing the
 // opponent's reach row (the traverser's own continuation choices).
-template <class T>
-__global__ void __launch_bounds__(kTermThreads) k_term_cr1(DevCtx c0, const DevCtx *__restrict__ ctxs,
-                                                           const TermItem *__restrict__ items, int trav) {
-    wait_prior_grid();
-    extern __shared__ __align__(16) char smem[];
-    const TermItem *I0 = items + blockIdx.x;
+// The work of kTermThreads threads (tid) with their own barrier (sync).
+template <class T, class Sync>
+__device__ __forceinline__ void cr1_terminal(const DevCtx &c0, const DevCtx *__restrict__ ctxs,
+                                             const TermItem *__restrict__ I0, int trav, char *smem, int tid,
+                                             Sync sync) {
     if (I0->follow) return;   // written by the block of its group's first item
     if (retired(ctxs, I0->sg)) return;
     const int ng = I0->gextra + 1;
@@ -1142,7 +1306,7 @@ __global__ void __launch_bounds__(kTermThreads) k_term_cr1(DevCtx c0, const DevC
     const Cr2View<T> V = ctxs ? cr2_view<T>(ctxs[I0->sg], trav, o, o) : cr2_view<T>(c0, trav, o, o);
     const int HS = V.HS;
     if (HS > c0.HS || V.deck > 52) return;   // shared memory was provisioned for c0's row stride
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int lane = tid & 31;
     const int Dp = (V.deck + 3) & ~3;
     Carve cv{smem};
     T *r = cv.take<T>(HS + 4);                 // staged reach row, r[HS] = 0 for missing pairs
@@ -1174,7 +1338,7 @@ __global__ void __launch_bounds__(kTermThreads) k_term_cr1(DevCtx c0, const DevC
         }
     }
     cp_async_wait_all();
-    __syncthreads();
+    sync();
     // per card c: u(c) and the count of positive-reach hands holding c, four
     // lanes per card (a quarter of the table row each, shuffles in a fixed order)
     {
@@ -1199,7 +1363,7 @@ __global__ void __launch_bounds__(kTermThreads) k_term_cr1(DevCtx c0, const DevC
             nz[col] = n;
         }
     }
-    __syncthreads();
+    sync();
     double F;
     int N;
     {
@@ -1235,8 +1399,16 @@ __global__ void __launch_bounds__(kTermThreads) k_term_cr1(DevCtx c0, const DevC
 }
 
 template <class T>
+__global__ void __launch_bounds__(kTermThreads) k_term_cr1(DevCtx c0, const DevCtx *__restrict__ ctxs,
+                                                           const TermItem *__restrict__ items, int trav) {
+    wait_prior_grid();
+    extern __shared__ __align__(16) char smem[];
+    cr1_terminal<T>(c0, ctxs, items + blockIdx.x, trav, smem, threadIdx.x, [] { __syncthreads(); });
+}
+
+template <class T>
 constexpr size_t sd1_smem() {
-    return 1326 * sizeof(T) + 1327 * 8 + 52 * 53 * 8 + 52 * 4 + (kTermThreads / 32) * 8 + 52 * 8 + 64;
+    return 1326 * sizeof(T) + 1327 * 8 + 52 * 53 * 8 + 52 * 4 + 8 * 8 + 52 * 8 + 64;
 }
 
 // Showdown against one live opponent (street_solve.cu:886-903): with W, T, L
@@ -1250,55 +1422,64 @@ constexpr size_t sd1_smem() {
 //   S = P[end] - PC[c1][end] - PC[c2][end] + f(h)
 // A traverser hand with no compatible positive-reach opponent hand gets
 // exactly 0 (positive-reach masks per card, as in the two-opponent kernels).
+//
+// Latency-bound: a heads-up river launches tens of these blocks and waits for
+// one.  1024 threads: eight warps scan the rank positions while the other 24
+// take the cards' lists, and every table that no kernel writes is read before
+// the wait for the previous kernel where a register can hold it.
+constexpr int kSd1Threads = 1024;
+constexpr int kSd1Scan = 256;   // threads of the rank-order scan (fixes its summation order)
 template <class T>
-__global__ void __launch_bounds__(kTermThreads) k_term_sd1(DevCtx c0, const DevCtx *__restrict__ ctxs,
-                                                           const TermItem *__restrict__ items, int trav) {
-    wait_prior_grid();
-    extern __shared__ __align__(16) char smem[];
+__device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__restrict__ ctxs,
+                                             const TermItem *__restrict__ item, int trav, char *smem) {
     Carve cv{smem};
     T *Rr = cv.take<T>(1326);
     double *Pp = cv.take<double>(1327);
     double *PC = cv.take<double>(52 * 53);
     int *clen = cv.take<int>(52);
-    double *wsum = cv.take<double>(kTermThreads / 32);
+    double *wsum = cv.take<double>(kSd1Scan / 32);
     unsigned long long *B = cv.take<unsigned long long>(52);
-    int *npos = cv.take<int>(1);
-    const TermItem I = items[blockIdx.x];
-    if (retired(ctxs, I.sg)) return;
+    const TermItem I = *item;
     const DevCtx &c = ctxs ? ctxs[I.sg] : c0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nc = c.ncomb;
-    for (int i = tid; i < nc; i += blockDim.x) Rr[i] = T(0);
-    __syncthreads();
-    {
-        const int o = I.opp_player[0];
-        const T *r = reach_rows<T>(c) + static_cast<size_t>(I.opp_row[0]) * c.HS;
-        const int *pos = c.sd_pos + static_cast<size_t>(o) * c.HS;
-        const bool dup = c.dup[o] != 0;
-        for (int j = tid; j < c.H[o]; j += blockDim.x) {
-            const int q = pos[j];
-            if (q < 0) continue;
-            if (dup)
-                atomicAdd(&Rr[q], r[j]);
-            else
-                Rr[q] = r[j];
+    const int nc = c.ncomb, HS = c.HS, Ht = c.H[trav];
+    const int o = I.opp_player[0];
+    const bool dup = c.dup[o] != 0;
+    const int *ph = c.pos_hand + static_cast<size_t>(o) * nc;
+    const int *tpos = c.sd_pos + static_cast<size_t>(trav) * HS;
+    const int ph0 = tid < nc ? __ldg(ph + tid) : -1;
+    const int q0 = tid < Ht ? __ldg(tpos + tid) : -1;
+    wait_prior_grid();
+    if (retired(ctxs, I.sg)) return;
+    const T *r = reach_rows<T>(c) + static_cast<size_t>(I.opp_row[0]) * HS;
+    if (!dup) {
+        // the opponent's reach by rank position, gathered
+        for (int q = tid; q < nc; q += kSd1Threads) {
+            const int j = q == tid ? ph0 : __ldg(ph + q);
+            Rr[q] = j >= 0 ? r[j] : T(0);
         }
+    } else {
+        for (int i = tid; i < nc; i += kSd1Threads) Rr[i] = T(0);
+        __syncthreads();
+        const int *pos = c.sd_pos + static_cast<size_t>(o) * HS;
+        for (int j = tid; j < c.H[o]; j += kSd1Threads)
+            if (pos[j] >= 0) atomicAdd(&Rr[pos[j]], r[j]);
     }
     __syncthreads();
-    // exclusive prefix over rank positions: each thread scans a contiguous chunk
-    {
-        const int per = (nc + blockDim.x - 1) / blockDim.x;
+    if (warp < kSd1Scan / 32) {
+        // exclusive prefix over rank positions: each thread scans a contiguous chunk
+        const int per = (nc + kSd1Scan - 1) / kSd1Scan;
         const int b0 = tid * per, b1 = min(nc, b0 + per);
         double local = 0.0;
         for (int i = b0; i < b1; ++i) local += Rr[i];
         double incl = local;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+        for (int k = 1; k < 32; k <<= 1) {
+            const double y = __shfl_up_sync(0xffffffffu, incl, k);
+            if (lane >= k) incl += y;
         }
         if (lane == 31) wsum[warp] = incl;
-        __syncthreads();
+        asm volatile("bar.sync 1, %0;" ::"n"(kSd1Scan) : "memory");
         double base = 0.0;
         for (int w = 0; w < warp; ++w) base += wsum[w];
         double run = base + incl - local;
@@ -1306,62 +1487,56 @@ __global__ void __launch_bounds__(kTermThreads) k_term_sd1(DevCtx c0, const DevC
             Pp[i] = run;
             run += Rr[i];
         }
-        if (tid == blockDim.x - 1) {
+        if (tid == kSd1Scan - 1) {
             double tot = 0.0;
-            for (int w = 0; w < blockDim.x / 32; ++w) tot += wsum[w];
+            for (int w = 0; w < kSd1Scan / 32; ++w) tot += wsum[w];
             Pp[nc] = tot;
         }
-    }
-    // per card: exclusive prefix sums over its combos in rank order, and the
-    // mask of partner cards whose combo holds positive reach
-    for (int card = warp; card < 52; card += blockDim.x / 32) {
-        const short *L = c.sd_card_list + card * 52;
-        const short *Pt = c.sd_card_partner + card * 52;
-        const int i0 = 2 * lane, i1 = 2 * lane + 1;
-        const int q0 = i0 < 52 ? L[i0] : -1, q1 = i1 < 52 ? L[i1] : -1;
-        const T f0 = q0 >= 0 ? Rr[q0] : T(0), f1 = q1 >= 0 ? Rr[q1] : T(0);
-        const double v0 = f0, v1 = f1;
-        const double pair = v0 + v1;
-        double incl = pair;
+    } else {
+        // per card: exclusive prefix sums over its combos in rank order, and
+        // the mask of partner cards whose combo holds positive reach
+        for (int card = warp - kSd1Scan / 32; card < 52; card += (kSd1Threads - kSd1Scan) / 32) {
+            const short *L = c.sd_card_list + card * 52;
+            const short *Pt = c.sd_card_partner + card * 52;
+            const int i0 = 2 * lane, i1 = 2 * lane + 1;
+            const int q0c = i0 < 52 ? L[i0] : -1, q1c = i1 < 52 ? L[i1] : -1;
+            const T f0 = q0c >= 0 ? Rr[q0c] : T(0), f1 = q1c >= 0 ? Rr[q1c] : T(0);
+            const double v0 = f0, v1 = f1;
+            const double pair = v0 + v1;
+            double incl = pair;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const double ex = incl - pair;
-        const int len = __popc(__ballot_sync(0xffffffffu, q0 >= 0)) + __popc(__ballot_sync(0xffffffffu, q1 >= 0));
-        if (i0 <= len) PC[card * 53 + i0] = ex;
-        if (i1 <= len) PC[card * 53 + i1] = ex + v0;
-        unsigned long long m = 0ull;
-        if (f0 > T(0)) m |= 1ull << Pt[i0];
-        if (f1 > T(0)) m |= 1ull << Pt[i1];
-        const unsigned lo = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(m));
-        const unsigned hi = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(m >> 32));
-        if (lane == 0) {
-            clen[card] = len;
-            B[card] = static_cast<unsigned long long>(lo) | (static_cast<unsigned long long>(hi) << 32);
+            for (int k = 1; k < 32; k <<= 1) {
+                const double y = __shfl_up_sync(0xffffffffu, incl, k);
+                if (lane >= k) incl += y;
+            }
+            const double ex = incl - pair;
+            const int len =
+                __popc(__ballot_sync(0xffffffffu, q0c >= 0)) + __popc(__ballot_sync(0xffffffffu, q1c >= 0));
+            if (i0 <= len) PC[card * 53 + i0] = ex;
+            if (i1 <= len) PC[card * 53 + i1] = ex + v0;
+            unsigned long long m = 0ull;
+            if (f0 > T(0)) m |= 1ull << Pt[i0];
+            if (f1 > T(0)) m |= 1ull << Pt[i1];
+            const unsigned lo = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(m));
+            const unsigned hi = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(m >> 32));
+            if (lane == 0) {
+                clen[card] = len;
+                B[card] = static_cast<unsigned long long>(lo) | (static_cast<unsigned long long>(hi) << 32);
+            }
         }
     }
     __syncthreads();
-    if (warp == 0) {
-        int n = __popcll(B[lane]) + (lane + 32 < 52 ? __popcll(B[lane + 32]) : 0);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-        if (lane == 0) *npos = n / 2;
-    }
-    __syncthreads();
-    const int Ht = c.H[trav];
-    const int *tpos = c.sd_pos + static_cast<size_t>(trav) * c.HS;
-    T *out = val_rows<T>(c) + static_cast<size_t>(I.node) * c.HS;
+    // positive-reach hands of the opponent (every warp for itself)
+    const int np_ = (__reduce_add_sync(0xffffffffu, __popcll(B[lane]) + (lane + 32 < 52 ? __popcll(B[lane + 32]) : 0))) / 2;
+    T *out = val_rows<T>(c) + static_cast<size_t>(I.node) * HS;
     // payoff per class with the reference's float coefficients (win pot - bet,
     // tie pot * 0.5 - bet, loss -bet): a coefficient that is exactly 0 drops
     // its class exactly, as in the reference's sum
     const double cw = static_cast<double>(I.pot - I.bet), ct = static_cast<double>(I.pot * 0.5f - I.bet);
     const double cl = -static_cast<double>(I.bet);
-    const int np_ = *npos;
-    for (int h = tid; h < c.HS; h += blockDim.x) {
+    for (int h = tid; h < HS; h += kSd1Threads) {
         double v = 0.0;
-        const int q = h < Ht ? tpos[h] : -1;
+        const int q = h == tid ? q0 : h < Ht ? __ldg(tpos + h) : -1;
         if (q >= 0) {
             const SdCombo s = c.sd_combo[q];
             const unsigned long long B1 = B[s.c1], B2 = B[s.c2];
@@ -1377,6 +1552,52 @@ __global__ void __launch_bounds__(kTermThreads) k_term_sd1(DevCtx c0, const DevC
         }
         store_value(out, h, v);
     }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kSd1Threads, 2) k_term_sd1(DevCtx c0, const DevCtx *__restrict__ ctxs,
+                                                          const TermItem *__restrict__ items, int trav) {
+    extern __shared__ __align__(16) char smem[];
+    sd1_terminal<T>(c0, ctxs, items + blockIdx.x, trav, smem);
+}
+
+// Two-way showdowns, one-opponent folds and zero rows of a river in one
+// launch: one block per showdown, then one per four folds (256 threads each,
+// their own barriers), then one per four zero rows.  A river has tens of
+// each, so a launch of its own costs each kind more than its work: on side
+// streams of the captured iteration they also doubled the graph's build and
+// release time.
+constexpr int kLightGroups = kSd1Threads / kTermThreads;
+__global__ void __launch_bounds__(kSd1Threads, 2) k_term_light(DevCtx c0, const DevCtx *__restrict__ ctxs,
+                                                               const TermItem *__restrict__ sd1, int n_sd1,
+                                                               const TermItem *__restrict__ cr1, int n_cr1,
+                                                               const TermItem *__restrict__ zero, int n_zero,
+                                                               int trav) {
+    extern __shared__ __align__(16) char smem[];
+    int b = blockIdx.x;
+    if (b < n_sd1) {
+        sd1_terminal<float>(c0, ctxs, sd1 + b, trav, smem);
+        return;
+    }
+    wait_prior_grid();
+    b -= n_sd1;
+    const int group = threadIdx.x / kTermThreads, tid = threadIdx.x % kTermThreads;
+    const int cr1_blocks = (n_cr1 + kLightGroups - 1) / kLightGroups;
+    if (b < cr1_blocks) {
+        const int i = b * kLightGroups + group;
+        if (i < n_cr1)
+            cr1_terminal<float>(c0, ctxs, cr1 + i, trav, smem + group * cr1_gather_smem<float>(c0.HS), tid, [group] {
+                asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kTermThreads) : "memory");
+            });
+        return;
+    }
+    const int i = (b - cr1_blocks) * kLightGroups + group;
+    if (i >= n_zero) return;
+    const TermItem &I = zero[i];
+    if (retired(ctxs, I.sg)) return;
+    const DevCtx &c = ctxs ? ctxs[I.sg] : c0;
+    float *out = c.val + static_cast<size_t>(I.node) * c.HS;
+    for (int h = tid; h < c.HS; h += kTermThreads) out[h] = 0.f;
 }
 
 // ---------------------------------------------------------------------------
@@ -2641,8 +2862,10 @@ __global__ void __launch_bounds__(128) k_snapshot_many(const DevCtx *__restrict_
     }
 }
 
-__global__ void k_bump(int *iter) {
-    wait_prior_grid(); *iter += 1; }
+__global__ void k_bump(int *iter, int by) {
+    wait_prior_grid();
+    *iter += by;
+}
 
 // out[h] = sum over rows of val[row][h]
 __global__ void __launch_bounds__(kHandThreads) k_sum_rows(DevCtx c, const int *__restrict__ rows, int n,
@@ -2743,18 +2966,34 @@ cudaError_t launch_reach(const DevCtx &c, const ReachItem *items, int n, int H, 
 }
 
 cudaError_t launch_cfv(const DevCtx &c, const CfvItem *items, int n, int n_long, int H, cudaStream_t s,
-                       const DevCtx *ctxs, int trav) {
+                       const DevCtx *ctxs, int trav, int iter_add) {
     if (n <= 0 || H <= 0) return cudaSuccess;
     n_long = n_long < 0 ? 0 : n_long > n ? n : n_long;
     const int n_short = n - n_long;
     if (n_short > 0) {
         const int nc = (H + 2 * kCfvThreads - 1) / (2 * kCfvThreads);
-        SSB_LAUNCH(k_cfv<1>, n_short * nc, kCfvThreads, 0, s, c, ctxs, items, nc, H, trav);
+        SSB_LAUNCH(k_cfv<1>, n_short * nc, kCfvThreads, 0, s, c, ctxs, items, nc, H, trav, iter_add);
     }
     if (n_long > 0) {
         const int nc = (H + 63) / 64;
         static_assert(32 * kCfvSplit == kCfvThreads, "the split form fills one block of kCfvThreads");
-        SSB_LAUNCH(k_cfv<kCfvSplit>, n_long * nc, kCfvThreads, 0, s, c, ctxs, items + n_short, nc, H, trav);
+        SSB_LAUNCH(k_cfv<kCfvSplit>, n_long * nc, kCfvThreads, 0, s, c, ctxs, items + n_short, nc, H, trav, iter_add);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tree(const DevCtx &c, const TreeRef &t, int H, cudaStream_t s, int iter_add) {
+    if (t.n_stages <= 0 || H <= 0) return cudaSuccess;
+    const unsigned grid = static_cast<unsigned>((H + kTreeHands - 1) / kTreeHands);
+    size_t sm = static_cast<size_t>(t.max_chains) * kTreeHands * sizeof(float);
+    if (t.bytes <= kTreeResident) {
+        sm += static_cast<size_t>(t.bytes);
+        const cudaError_t e = cudaFuncSetAttribute(k_tree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   kTreeResident + kTreeChains * kTreeHands * 4);
+        if (e != cudaSuccess) return e;
+        SSB_LAUNCH(k_tree<true>, grid, t.threads, sm, s, c, t, H, iter_add);
+    } else {
+        SSB_LAUNCH(k_tree<false>, grid, t.threads, sm, s, c, t, H, iter_add);
     }
     return cudaGetLastError();
 }
@@ -2809,7 +3048,7 @@ cudaError_t launch_terms_t(const DevCtx &c, int kind, const TermItem *items, int
                 e = cudaFuncSetAttribute(k_term_sd1<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(sd1_smem<T>()));
             if (e != cudaSuccess) return e;
-            SSB_LAUNCH(k_term_sd1<T>, n, kTermThreads, sd1_smem<T>(), s, c, ctxs, items, trav);
+            SSB_LAUNCH(k_term_sd1<T>, n, kSd1Threads, sd1_smem<T>(), s, c, ctxs, items, trav);
             break;
         case TK_SD2: {
             // runs per block: about two waves of four blocks per SM at most
@@ -2855,6 +3094,21 @@ cudaError_t launch_terms_t(const DevCtx &c, int kind, const TermItem *items, int
 cudaError_t launch_terms(const DevCtx &c, int kind, const TermItem *items, int n, int trav,
                          cudaStream_t s, const DevCtx *ctxs, const int *heads, int n_heads) {
     return launch_terms_t<float>(c, kind, items, n, trav, s, ctxs, heads, n_heads);
+}
+
+cudaError_t launch_terms_light(const DevCtx &c, const TermItem *sd1, int n_sd1, const TermItem *cr1, int n_cr1,
+                               const TermItem *zero, int n_zero, int trav, cudaStream_t s, const DevCtx *ctxs) {
+    const int grid = n_sd1 + (n_cr1 + kLightGroups - 1) / kLightGroups + (n_zero + kLightGroups - 1) / kLightGroups;
+    if (grid <= 0) return cudaSuccess;
+    const size_t sm = std::max(sd1_smem<float>(), n_cr1 > 0 ? kLightGroups * cr1_gather_smem<float>(c.HS) : 0);
+    if (sm > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_term_light, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(std::max(sd1_smem<float>(), kLightGroups * cr1_gather_smem<float>(kMaxHS))));
+        if (e != cudaSuccess) return e;
+    }
+    SSB_LAUNCH(k_term_light, grid, kSd1Threads, sm, s, c, ctxs, sd1, n_sd1, cr1, n_cr1, zero, n_zero, trav);
+    return cudaGetLastError();
 }
 
 template <class T>
@@ -2909,8 +3163,8 @@ cudaError_t launch_br_root_many(const DevCtx *ctxs, const RootItem *items, int n
     return cudaGetLastError();
 }
 
-cudaError_t launch_bump(int *iter, cudaStream_t s) {
-    SSB_LAUNCH(k_bump, 1, 1, 0, s, iter);
+cudaError_t launch_bump(int *iter, int by, cudaStream_t s) {
+    SSB_LAUNCH(k_bump, 1, 1, 0, s, iter, by);
     return cudaGetLastError();
 }
 

@@ -78,8 +78,6 @@ constexpr int kHandThreads = 64;
 constexpr int kHandsPerBlock = kHandThreads * 4;
 // threads per block of the value/regret kernel (2 hands each)
 constexpr int kCfvThreads = 128;
-// warps that share one hand chunk of a value/regret item with a long frontier
-constexpr int kCfvSplit = 4;
 // threads per block of the per-terminal kernels
 constexpr int kTermThreads = 256;
 
@@ -90,14 +88,28 @@ constexpr int kTermThreads = 256;
 cudaError_t launch_reach(const DevCtx &c, const ReachItem *items, int n, int H, cudaStream_t s,
                          const DevCtx *ctxs = nullptr, int player = -1);
 // The last n_long items (long frontiers) run with kCfvSplit warps per hand chunk.
+// The iteration number is *c.iter + iter_add.
 cudaError_t launch_cfv(const DevCtx &c, const CfvItem *items, int n, int n_long, int H, cudaStream_t s,
-                       const DevCtx *ctxs = nullptr, int trav = -1);
+                       const DevCtx *ctxs = nullptr, int trav = -1, int iter_add = 0);
+// The device copy of a TreePass (its blob) and its launch sizes.
+struct TreeRef {
+    const char *blob;
+    int bytes, o_items, o_chains, o_reach, o_rows;
+    int n_stages, max_chains, threads;
+};
+// player's small levels in one launch, over its H hands
+cudaError_t launch_tree(const DevCtx &c, const TreeRef &t, int H, cudaStream_t s, int iter_add = 0);
 // heads (optional, TK_CR2): the n_heads items that start work (TermItem
 // groups and chains); the launch then has one block per head instead of one
 // per item (the tensor-core two-opponent form takes every item)
 cudaError_t launch_terms(const DevCtx &c, int kind, const TermItem *items, int n, int trav,
                          cudaStream_t s, const DevCtx *ctxs = nullptr, const int *heads = nullptr,
                          int n_heads = 0);
+// Two-way showdowns, one-opponent folds (k_term_cr1's kind) and zero rows of
+// one traverser in one launch.
+cudaError_t launch_terms_light(const DevCtx &c, const TermItem *sd1, int n_sd1, const TermItem *cr1, int n_cr1,
+                               const TermItem *zero, int n_zero, int trav, cudaStream_t s,
+                               const DevCtx *ctxs = nullptr);
 cudaError_t launch_terms_fp64(const DevCtx &c, int kind, const TermItem *items, int n, int trav,
                               cudaStream_t s, const DevCtx *ctxs = nullptr);
 // Three-way showdowns of many subgames (batches): block b sweeps run group
@@ -119,7 +131,7 @@ bool cr2_tensor_form(const DevCtx &c);
 // The device fault word (a bounded tensor-core wait that ran out, or a block
 // a kernel was not built for): copied into *code and cleared; synchronizes s.
 cudaError_t read_device_fault(unsigned *code, cudaStream_t s);
-cudaError_t launch_bump(int *iter, cudaStream_t s);
+cudaError_t launch_bump(int *iter, int by, cudaStream_t s);
 cudaError_t launch_bump_many(const DevCtx *ctxs, const int *sgs, int n, cudaStream_t s);
 cudaError_t launch_snapshot_many(const DevCtx *ctxs, const int *sgs, int n, cudaStream_t s);
 cudaError_t launch_br_reach(const DevCtx &c, const ReachItem *items, int n, int H, const float *avg,

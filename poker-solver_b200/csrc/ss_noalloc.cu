@@ -255,7 +255,7 @@ int solve_noalloc(const Problem &pb, int iterations, SSOutput *out) {
     };
     for (int p = 0; p < np; ++p) NA_CK(reach(p));
     for (int it = 1; it <= iterations; ++it) {
-        NA_CK(launch_bump(iter_ptr, s0));
+        NA_CK(launch_bump(iter_ptr, 1, s0));
         for (int t = 0; t < np; ++t) {
             if (it == iterations && t == np - 1)
                 NA_CK(launch_root_strategy(c, P.first_edge[0], P.root_na, frozen_root,

@@ -55,6 +55,7 @@ class Session {
     std::vector<std::pair<int, int>> reach_lv[SS_MAX_PLAYERS];
     const CfvItem *cfv_items[SS_MAX_PLAYERS] = {};
     std::vector<std::pair<int, int>> cfv_lv[SS_MAX_PLAYERS];
+    TreeRef tree[SS_MAX_PLAYERS] = {};
     const TermItem *term_items[SS_MAX_PLAYERS][TK_COUNT] = {};
     const int *term_heads[SS_MAX_PLAYERS][TK_COUNT] = {};   // null for kinds without P.term_heads
     const int *root_fr[SS_MAX_PLAYERS] = {};
@@ -125,8 +126,9 @@ class Session {
         return cudaEventRecordWithFlags(m.ev, stream, cudaEventRecordExternal);
     }
 
-    cudaError_t reach(int p) {
-        for (size_t l = 0; l < reach_lv[p].size(); ++l) {
+    // player p's reach levels from level `from` on
+    cudaError_t reach(int p, size_t from = 0) {
+        for (size_t l = from; l < reach_lv[p].size(); ++l) {
             cudaError_t e = mark(PC_REACH, reach_bytes[p][l], reach_lv[p][l].second);
             if (e == cudaSuccess)
                 e = launch_reach(c, reach_items[p] + reach_lv[p][l].first, reach_lv[p][l].second,
@@ -136,13 +138,24 @@ class Session {
         return cudaSuccess;
     }
 
+    // Where traverser t has two-way showdowns, its one-opponent folds and zero
+    // rows ride in their launch (rivers: tens of short blocks of each kind).
+    bool light(int t, int k) const {
+        return !P.term[t][TK_SD1].empty() && (k == TK_SD1 || k == TK_CR1 || k == TK_ZERO);
+    }
+
     // traverser t's terminals of kind k (grouped kinds: one block per head)
     cudaError_t terms(int t, int k, cudaStream_t s) {
+        if (light(t, k))
+            return launch_terms_light(c, term_items[t][TK_SD1], static_cast<int>(P.term[t][TK_SD1].size()),
+                                      term_items[t][TK_CR1], static_cast<int>(P.term[t][TK_CR1].size()),
+                                      term_items[t][TK_ZERO], static_cast<int>(P.term[t][TK_ZERO].size()), t, s);
         return launch_terms(c, k, term_items[t][k], static_cast<int>(P.term[t][k].size()), t, s, nullptr,
                             term_heads[t][k], static_cast<int>(P.term_heads[t][k].size()));
     }
 
-    cudaError_t pass(int t, bool snapshot_root) {
+    // traverser t's part of iteration *iter + iter_add
+    cudaError_t pass(int t, bool snapshot_root, int iter_add) {
         cudaError_t e = cudaSuccess;
         if (snapshot_root) {
             e = mark(PC_OTHER, 0);
@@ -151,18 +164,27 @@ class Session {
                                          P.H[P.root_player], dsmall, stream);
             if (e != cudaSuccess) return e;
         }
+        // the launches of this pass; the one with the most work stays on the
+        // session stream (relative block times of full-range rivers and turns)
         int kinds[TK_COUNT], nk = 0, main_k = -1;
+        double main_w = 0, by[TK_COUNT] = {};
         for (int k = 0; k < TK_COUNT; ++k) {
             const int n = static_cast<int>(P.term[t][k].size());
-            if (n == 0) continue;
+            const int lk = light(t, k) ? static_cast<int>(TK_SD1) : k;
+            by[lk] += term_bytes[t][k];
+            if (n == 0 || lk != k) continue;
             kinds[nk++] = k;
-            if (main_k < 0 || n > static_cast<int>(P.term[t][main_k].size())) main_k = k;
+            const double w = n * (k == TK_SD3 || k == TK_CR3 ? 64.0 : k == TK_SD2 || k == TK_ENUM ? 16.0 : 1.0);
+            if (main_k < 0 || w > main_w) {
+                main_k = k;
+                main_w = w;
+            }
         }
         if (marks || nk <= 1 || !ev_fork) {
             // one kind after the other (the profile times each class)
             for (int i = 0; i < nk; ++i) {
                 const int k = kinds[i];
-                e = mark(term_class(k), term_bytes[t][k], static_cast<int>(P.term[t][k].size()));
+                e = mark(term_class(k), by[k], static_cast<int>(P.term[t][k].size()));
                 if (e == cudaSuccess) e = terms(t, k, stream);
                 if (e != cudaSuccess) return e;
             }
@@ -180,20 +202,36 @@ class Session {
                 if (kinds[i] != main_k) e = cudaStreamWaitEvent(stream, ev_join[kinds[i]], 0);
             if (e != cudaSuccess) return e;
         }
+        // the large value/regret levels, then the small levels of values and
+        // reach in one launch, then the large reach levels
+        const TreePass &T = P.tree[t];
+        double tree_by = 0;
+        int items = 0;
         for (size_t l = 0; l < cfv_lv[t].size(); ++l) {
+            if (static_cast<int>(l) >= T.cfv_from) {
+                tree_by += cfv_bytes[t][l];
+                items += cfv_lv[t][l].second;
+                continue;
+            }
             e = mark(PC_CFV, cfv_bytes[t][l], cfv_lv[t][l].second);
             if (e == cudaSuccess)
                 e = launch_cfv(c, cfv_items[t] + cfv_lv[t][l].first, cfv_lv[t][l].second, P.cfv_nlong[t][l],
-                               P.H[t], stream);
+                               P.H[t], stream, nullptr, -1, iter_add);
             if (e != cudaSuccess) return e;
         }
-        return reach(t);
+        if (tree[t].n_stages > 0) {
+            for (int l = 0; l < T.reach_to; ++l) tree_by += reach_bytes[t][l];
+            e = mark(PC_CFV, tree_by, items);
+            if (e == cudaSuccess) e = launch_tree(c, tree[t], P.H[t], stream, iter_add);
+            if (e != cudaSuccess) return e;
+        }
+        return reach(t, static_cast<size_t>(T.reach_to));
     }
 
-    cudaError_t iteration(bool last) {
-        cudaError_t e = mark(PC_OTHER, 0);
-        if (e == cudaSuccess) e = launch_bump(diter, stream);
-        for (int t = 0; t < P.np && e == cudaSuccess; ++t) e = pass(t, last && t == P.np - 1);
+    // iteration *iter + iter_add
+    cudaError_t iteration(bool last, int iter_add) {
+        cudaError_t e = cudaSuccess;
+        for (int t = 0; t < P.np && e == cudaSuccess; ++t) e = pass(t, last && t == P.np - 1, iter_add);
         return e;
     }
 
@@ -202,7 +240,9 @@ class Session {
         cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
         cudaError_t body = cudaSuccess;
-        for (int i = 0; i < iters && body == cudaSuccess; ++i) body = iteration(last && i == iters - 1);
+        for (int i = 0; i < iters && body == cudaSuccess; ++i) body = iteration(last && i == iters - 1, i + 1);
+        if (body == cudaSuccess) body = mark(PC_OTHER, 0);
+        if (body == cudaSuccess) body = launch_bump(diter, iters, stream);
         e = cudaStreamEndCapture(stream, &g);
         if (body != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
