@@ -293,9 +293,10 @@ class Batch {
                 ctx[i] = subs[i]->c;
                 ctx[i].live = active[i];
                 // launch-time sizes (grids, dynamic shared memory) come from
-                // cmax: the largest row stride, rank table and sweep run of the batch
+                // cmax: the largest row stride, rank table, deck and sweep run of the batch
                 cmax.HS = std::max(cmax.HS, subs[i]->c.HS);
                 cmax.ncomb = std::max(cmax.ncomb, subs[i]->c.ncomb);
+                cmax.deck = std::max(cmax.deck, subs[i]->c.deck);
                 for (int lg = 0; lg < kSd2Merge; ++lg)
                     cmax.sd_span[lg] = std::max(cmax.sd_span[lg], subs[i]->c.sd_span[lg]);
             }

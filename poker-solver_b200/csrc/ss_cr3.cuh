@@ -1,5 +1,8 @@
-// ss_cr3.cuh -- card-removal mass of three counted opponents (folds and
-// leaves of 4+ player subgames), the block phases of k_term_cr3.
+// ss_cr3.cuh -- card-removal mass of three counted opponents by conditioning
+// on the third one's hand: the four-way showdowns (k_term_sd3), whose classes
+// of the third opponent's hands need the sum hand by hand.  Folds and leaves
+// contract it instead (ss_triple.cuh); the whole-range form here is what the
+// host checks compare with enumeration.
 //
 // The reference sums, per traverser hand h, the reach products of every
 // tuple of opponent hands (o1, o2, o3) that are pairwise disjoint and
@@ -181,26 +184,6 @@ SSB_CR3_HD void phase_vectors(int tid, int nt, const Opp3<T> &in, const Tables &
         t.d[c] = t.P[c * kS + c];
         t.id[c] = popc64(t.mA[c] & t.mB[c]);
     }
-}
-
-// the third opponent's compacted positive-reach list in hand order (the
-// kS item of phase_vectors, on its own)
-template <class T>
-SSB_CR3_HD void compact_third_list(const Opp3<T> &in, const Tables &t) {
-    long long n = 0;
-    double f3 = 0.0;
-    for (int h = 0; h < in.H3; ++h) {
-        const int code = in.code3[h];
-        if (code & 0x10000) continue;   // touches the board
-        const T r = in.r3[h];
-        if (!(r > T(0))) continue;
-        t.r3[n] = static_cast<double>(r);
-        f3 += t.r3[n];
-        t.xy[n] = static_cast<unsigned short>(((code >> 20) & 63) | (((code >> 26) & 63) << 8));
-        ++n;
-    }
-    t.isc[4] = n;
-    t.sc[4] = f3;
 }
 
 // phase 5 (one item): the scalars

@@ -18,6 +18,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include "ss_cr3.cuh"
+#include "ss_triple.cuh"
 
 namespace ssb {
 
@@ -2270,25 +2271,36 @@ __global__ void __launch_bounds__(32 * kEnumWarps) k_term_enum(DevCtx c0, const 
 }
 
 // Folds and leaves with three counted opponents (4+ player subgames): the
-// card-removal mass by conditioning on the third opponent (ss_cr3.cuh), in
-// FP64, one block per (group of terminals, chunk of kTermThreads traverser
-// hands), one thread per hand; the first two opponents' aggregates are
-// rebuilt by every chunk's block (O(deck^3), small beside the O(H3) walk of
-// each hand).  A hand whose mass is within rounding of 0 takes the exact
-// tuple count, and 0 when there is none (the reference adds only positive
-// products).  Terminals on the same opponent reach rows (the traverser's own
-// continuation choices) form a group: its first item's blocks write every
-// member's row, each with its own factor.
-constexpr size_t cr3_smem(int HS) {
-    return (4 * cr3::kS * cr3::kS + 4 * cr3::kS + 8) * sizeof(double) + 4 * cr3::kS * sizeof(int) +
-           2 * cr3::kS * sizeof(unsigned long long) + 8 * sizeof(long long) +
-           static_cast<size_t>(HS) * (sizeof(double) + sizeof(unsigned short)) + 16 * 16;
+// card-removal mass by contraction (ss_triple.cuh), in FP64: O(deck) per
+// traverser hand over tables of O(deck^2), where conditioning on the third
+// opponent's hand took O(hands) two-opponent evaluations.  One block per
+// (group of terminals on the same reach rows, share of the hands); its first
+// item's blocks write every member's row, each with its own factor.  Bound by
+// the FP64 pipe and shared memory: per hand and card 34 FP64 operations and
+// 23 shared-memory wavefronts per warp, beside two 48 x 48 products per block.
+// A hand whose mass is within rounding of 0 is looked at exactly, and 0 when
+// it has no tuple (the reference adds only positive products).
+//
+// 384 threads take the 1128 hands of a turn in three rounds of 98 %, and the
+// tables of a 48-card deck (105 KB) leave two blocks per SM (512 and 576
+// threads spill: 1.4x slower).  Measured on the 4-player turn (5,681 nodes,
+// 2,696 terminals): 8.4 ms per launch by conditioning, 0.5 ms in the first
+// iterations, 1.06 ms where play has become near pure and many hands need the
+// exact look.
+constexpr int kCr3Threads = 384;
+constexpr int kCr3Rounds = (kMaxHS + kCr3Threads - 1) / kCr3Threads;
+// blocks a launch is brought to by sharing a group's hands between blocks (each
+// builds the tables): two per SM
+constexpr int kCr3Blocks = 2 * 148;
+constexpr size_t cr3_smem(int deck) {
+    return static_cast<size_t>(tri::doubles(deck)) * sizeof(double) + 2 * tri::kVS * sizeof(unsigned long long) +
+           4 * tri::kVS * sizeof(int) + 4 * sizeof(long long) + 8 * 16;
 }
 
 template <class T>
-__global__ void __launch_bounds__(kTermThreads, 2) k_term_cr3(DevCtx c0, const DevCtx *__restrict__ ctxs,
-                                                             const TermItem *__restrict__ items, int nchunk,
-                                                             int trav) {
+__global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const DevCtx *__restrict__ ctxs,
+                                                            const TermItem *__restrict__ items, int nchunk,
+                                                            int trav) {
     wait_prior_grid();
     extern __shared__ __align__(16) char smem[];
     const int it = blockIdx.x / nchunk;
@@ -2297,65 +2309,93 @@ __global__ void __launch_bounds__(kTermThreads, 2) k_term_cr3(DevCtx c0, const D
     if (I0->follow) return;   // written by the blocks of its group's first item
     if (retired(ctxs, I0->sg)) return;
     const int ng = I0->gextra + 1;
-    const TermItem I = *I0;
-    const DevCtx &c = ctxs ? ctxs[I.sg] : c0;
-    const int HS = c.HS;
-    // shared memory was provisioned for c0's row stride (the largest of a batch)
-    if (HS > c0.HS || c.deck > cr3::kS - 1) return;
-    const int h0 = ch * kTermThreads;
-    if (h0 >= HS) return;
+    const DevCtx &c = ctxs ? ctxs[I0->sg] : c0;
+    const int HS = c.HS, Ht = c.H[trav], n = c.deck;
+    // shared memory was provisioned for c0's deck (the largest of a batch)
+    if (HS > kMaxHS || n > c0.deck || ch * kCr3Threads >= HS) return;
+    const int tid = threadIdx.x;
     Carve cv{smem};
-    cr3::Tables t;
-    t.A = cv.take<double>(cr3::kS * cr3::kS);
-    t.B = cv.take<double>(cr3::kS * cr3::kS);
-    t.P = cv.take<double>(cr3::kS * cr3::kS);
-    t.PT = cv.take<double>(cr3::kS * cr3::kS);
-    t.uA = cv.take<double>(cr3::kS);
-    t.uB = cv.take<double>(cr3::kS);
-    t.w = cv.take<double>(cr3::kS);
-    t.d = cv.take<double>(cr3::kS);
-    t.sc = cv.take<double>(8);
-    t.iuA = cv.take<int>(cr3::kS);
-    t.iuB = cv.take<int>(cr3::kS);
-    t.iw = cv.take<int>(cr3::kS);
-    t.id = cv.take<int>(cr3::kS);
-    t.mA = cv.take<unsigned long long>(cr3::kS);
-    t.mB = cv.take<unsigned long long>(cr3::kS);
-    t.isc = cv.take<long long>(8);
-    t.r3 = cv.take<double>(HS);
-    t.xy = cv.take<unsigned short>(HS);
+    const tri::Tables t = tri::tables(cv.take<double>(tri::doubles(n)), n);
+    tri::Counts k;
+    k.mA = cv.take<unsigned long long>(tri::kVS);
+    k.mB = cv.take<unsigned long long>(tri::kVS);
+    k.nA = cv.take<int>(tri::kVS);
+    k.nB = cv.take<int>(tri::kVS);
+    k.nW = cv.take<int>(tri::kVS);
+    k.nD = cv.take<int>(tri::kVS);
+    k.s = cv.take<long long>(4);
+    const int o1 = I0->opp_player[0], o2 = I0->opp_player[1], o3 = I0->opp_player[2];
     const T *reach = reach_rows<T>(c);
     const size_t hs = static_cast<size_t>(HS);
-    cr3::Opp3<T> in;
-    in.r1 = reach + static_cast<size_t>(I.opp_row[0]) * hs;
-    in.r2 = reach + static_cast<size_t>(I.opp_row[1]) * hs;
-    in.r3 = reach + static_cast<size_t>(I.opp_row[2]) * hs;
-    in.pair1 = c.pair_idx + static_cast<size_t>(I.opp_player[0]) * 52 * 52;
-    in.pair2 = c.pair_idx + static_cast<size_t>(I.opp_player[1]) * 52 * 52;
-    in.code3 = c.hand_code + static_cast<size_t>(I.opp_player[2]) * hs;
-    in.H3 = c.H[I.opp_player[2]];
-    in.HS = HS;
-    in.deck = c.deck;
-    const int tid = threadIdx.x;
-    static_assert(kTermThreads == 256, "the device build steps assume 256 threads");
-    cr3::gather_dev(tid, in, t, nullptr, 0, 0, nullptr, 0, 0);
+    const T *r1 = reach + static_cast<size_t>(I0->opp_row[0]) * hs;
+    const T *r2 = reach + static_cast<size_t>(I0->opp_row[1]) * hs;
+    const T *r3 = reach + static_cast<size_t>(I0->opp_row[2]) * hs;
+    const int *code3 = c.hand_code + static_cast<size_t>(o3) * hs;
+    const int H3 = c.H[o3];
+    const bool dup3 = c.dup[o3] != 0;
+    tri::phase_gather(tid, kCr3Threads, t, r1, r2, r3, c.pair_idx + static_cast<size_t>(o1) * 52 * 52,
+                      c.pair_idx + static_cast<size_t>(o2) * 52 * 52, c.pair_idx + static_cast<size_t>(o3) * 52 * 52,
+                      HS, !dup3);
     __syncthreads();
-    cr3::build_step1(tid, t);
-    if (tid == kTermThreads - 1) cr3::compact_third_list(in, t);
-    __syncthreads();
-    cr3::build_step2(tid, t);
-    __syncthreads();
-    const int h = h0 + tid;
-    if (h >= HS) return;
-    T *val = val_rows<T>(c);
-    if (h >= c.H[trav]) {
-        for (int g = 0; g < ng; ++g) val[static_cast<size_t>(I0[g].node) * hs + h] = T(0);
-        return;
+    if (dup3) {
+        tri::phase_gather_third(tid, kCr3Threads, t, r3, code3, H3);
+        __syncthreads();
     }
-    const double m = cr3::cr3_hand_value_mass(c.hand_code[static_cast<size_t>(trav) * hs + h], c.deck, t);
-    for (int g = 0; g < ng; ++g) {
-        const TermItem &Ig = I0[g];
-        val[static_cast<size_t>(Ig.node) * hs + h] = static_cast<T>(static_cast<double>(term_factor(c, Ig, h)) * m);
+    tri::phase_products(tid, kCr3Threads, t);
+    __syncthreads();
+    tri::phase_vectors(tid, kCr3Threads, t);
+    __syncthreads();
+    tri::phase_scalars(tid, kCr3Threads, t);
+    __syncthreads();
+    // an opponent without positive reach: every mass is 0
+    const bool none = t.sc[tri::FA] == 0.0 || t.sc[tri::FB] == 0.0 || t.sc[tri::FC] == 0.0;
+    const double zb = tri::zero_bound(t);
+    const int *code_t = c.hand_code + static_cast<size_t>(trav) * hs;
+    auto dense = [&](int hc, int shift) {
+        const int d = (hc >> shift) & 63;
+        return d < n ? d : n;
+    };
+    T *val = val_rows<T>(c);
+    auto write = [&](int h, double m) {
+        for (int g = 0; g < ng; ++g) {
+            const TermItem &Ig = I0[g];
+            val[static_cast<size_t>(Ig.node) * hs + h] =
+                h < Ht ? static_cast<T>(static_cast<double>(term_factor(c, Ig, h)) * m) : T(0);
+        }
+    };
+    unsigned near = 0;   // this thread's hands (by round) within rounding of 0
+#pragma unroll 1
+    for (int r = ch; r < kCr3Rounds; r += nchunk) {
+        const int h = r * kCr3Threads + tid;
+        if (h >= HS) break;
+        double m = 0.0;
+        if (h < Ht && !none) {
+            const int hc = __ldg(code_t + h);
+            m = tri::hand_mass(dense(hc, 20), dense(hc, 26), t);
+            if (fabs(m) <= zb) near |= 1u << r;
+        }
+        write(h, m);
+    }
+    if (!__syncthreads_or(near != 0)) return;
+    // a warp per hand within rounding of 0, 32 third-opponent hands at a time;
+    // the list of those hands takes C's space
+    int *n_near = reinterpret_cast<int *>(t.C);
+    unsigned short *list = reinterpret_cast<unsigned short *>(n_near + 4);
+    static_assert(kMaxHS * 2 + 16 <= 47 * 47 * 8, "the list fits C's space");
+    if (tid == 0) *n_near = 0;
+    tri::phase_masks(tid, kCr3Threads, t, k);
+    __syncthreads();
+    for (int r = ch; r < kCr3Rounds; r += nchunk)
+        if (near >> r & 1u) list[atomicAdd(n_near, 1)] = static_cast<unsigned short>(r * kCr3Threads + tid);
+    tri::phase_counts(tid, kCr3Threads, t, k);
+    __syncthreads();
+    const int lane = tid & 31;
+    for (int i = tid >> 5; i < *n_near; i += kCr3Threads / 32) {
+        const int h = list[i], hc = __ldg(code_t + h), a = dense(hc, 20), b = dense(hc, 26);
+        bool any = false;
+        for (int j = lane; !any && j - lane < H3; j += 32)
+            any = __any_sync(0xffffffffu, j < H3 && tri::tuple_with(a, b, k, r3[j], __ldg(code3 + j)));
+        if (!any && lane == 0) write(h, 0.0);
     }
 }
 
@@ -2377,7 +2417,10 @@ constexpr int kSd3MaxE = 64;
 // a table build in units of one D2 evaluation (the sparse steps' cost model)
 constexpr double kSd3BuildCost = 3000.0;
 constexpr size_t sd3_smem(int HS) {
-    return cr3_smem(HS) + static_cast<size_t>(HS) * sizeof(int) + 16 + 3 * kTermThreads +
+    return (4 * cr3::kS * cr3::kS + 4 * cr3::kS + 8) * sizeof(double) + 4 * cr3::kS * sizeof(int) +
+           2 * cr3::kS * sizeof(unsigned long long) + 8 * sizeof(long long) +
+           static_cast<size_t>(HS) * (sizeof(double) + sizeof(unsigned short)) + 16 * 16 +
+           static_cast<size_t>(HS) * sizeof(int) + 16 + 3 * kTermThreads +
            2 * kSd3Warps * (sizeof(double) + sizeof(long long)) + 64 + 2 * kSd3MaxE * sizeof(cr3::EHand) + 16 + 64;
 }
 
@@ -3077,12 +3120,13 @@ cudaError_t launch_terms_t(const DevCtx &c, int kind, const TermItem *items, int
             break;
         }
         case TK_CR3: {
-            if (c.HS > kMaxHS) return cudaErrorInvalidValue;
-            const int nc = (c.HS + kTermThreads - 1) / kTermThreads;
+            if (c.HS > kMaxHS || c.deck < 0 || c.deck > 52) return cudaErrorInvalidValue;
+            const int rounds = (c.HS + kCr3Threads - 1) / kCr3Threads;
+            const int nc = std::min(rounds, std::max(1, kCr3Blocks / n));
             e = cudaFuncSetAttribute(k_term_cr3<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(cr3_smem(kMaxHS)));
+                                     static_cast<int>(cr3_smem(52)));
             if (e != cudaSuccess) return e;
-            SSB_LAUNCH(k_term_cr3<T>, n * nc, kTermThreads, cr3_smem(c.HS), s, c, ctxs, items, nc, trav);
+            SSB_LAUNCH(k_term_cr3<T>, n * nc, kCr3Threads, cr3_smem(c.deck), s, c, ctxs, items, nc, trav);
             break;
         }
         default:

@@ -1,0 +1,322 @@
+// ss_triple.cuh -- card-removal mass of three counted opponents for every
+// traverser hand (folds and leaves of 4+ player subgames), by contraction.
+//
+// With symmetric combo matrices A, B, C (zero diagonal) of the three
+// opponents' reach over the dense deck, the mass of pairwise disjoint hands
+// (o1, o2, o3) is, by inclusion-exclusion over the cards that two of them
+// share (u = row sums, F = sum u / 2, Q_XY = u_X . u_Y, d_XY(x) =
+// sum_y X[x][y] Y[x][y], E_XY = sum d_XY / 2),
+//   F_A F_B F_C + F_C (E_AB - Q_AB) + F_B (E_AC - Q_AC) + F_A (E_BC - Q_BC)
+//   + 2 sum_x u_A u_B u_C + u_A C u_B + u_C B u_A + u_C A u_B
+//   - 2 sum_x (u_A d_BC + u_B d_AC + u_C d_AB)
+//   + 2 sum_xy A B C - tr(A B C).
+// For a traverser hand {a, b} it is the same expression on the matrices with
+// rows and columns a, b removed (primed).  F', Q', E', the elementwise sum
+// and the trace follow from tables of the full matrices in O(1); the sums
+// over x run over the deck with u'(x) = u(x) - X[x][a] - X[x][b],
+// (C' u_B')(x) = (C u_B)(x) - (C B)[x][a] - (C B)[x][b] - C[x][a] u_B'(a) -
+// C[x][b] u_B'(b), and the like: O(deck) per hand.  (Conditioning on the
+// third opponent's hand, ss_cr3.cuh, takes O(hands) evaluations of the
+// two-opponent form instead.)
+//
+// A board card of the traverser's hand maps to the dummy index n (the deck
+// size), whose rows, columns and vector entries are zero.  Rows are S = n + 1
+// rounded up to odd doubles, so rows and columns both read without bank
+// conflicts across consecutive cards.
+//
+// Each phase is a function of (thread index, thread count) whose work items
+// are independent within the phase; the kernel separates phases with block
+// barriers, and a host build runs them one after another.
+#pragma once
+
+#if defined(__CUDACC__)
+#define SSB_TRI_HD __host__ __device__ __forceinline__
+#else
+#define SSB_TRI_HD inline
+#endif
+
+namespace ssb {
+namespace tri {
+
+// per-card vectors, then the scalars (one array, fixed order)
+enum Vec : int { UA, UB, UC, DAB, DAC, DBC, AUB, BUA, AUC, CUA, BUC, CUB, HH, TABC, TCAB, TACB, N_VEC };
+enum Scal : int { FA, FB, FC, QAB, QAC, QBC, EAB, EAC, EBC, SH, TR, N_SCAL };
+constexpr int kVS = 56;   // stride of a per-card vector (n <= 52 plus the dummy)
+
+struct Tables {
+    double *A, *B, *C, *AB, *CB;   // [S][S]
+    double *v;                     // [N_VEC][kVS]
+    double *sc;                    // [N_SCAL]
+    int n, S;
+};
+
+SSB_TRI_HD constexpr int stride(int n) { return (n + 1) | 1; }
+SSB_TRI_HD constexpr int doubles(int n) { return 5 * stride(n) * stride(n) + N_VEC * kVS + N_SCAL + 1; }
+
+SSB_TRI_HD Tables tables(double *mem, int n) {
+    Tables t;
+    t.n = n;
+    t.S = stride(n);
+    const int m = t.S * t.S;
+    t.A = mem;
+    t.B = mem + m;
+    t.C = mem + 2 * m;
+    t.AB = mem + 3 * m;
+    t.CB = mem + 4 * m;
+    t.v = mem + 5 * m;
+    t.sc = t.v + N_VEC * kVS;
+    return t;
+}
+
+// phase 1: the matrices from the opponents' pair tables ([52][52] dense pair
+// -> range index, HS if none); the dummy row and column are zero.  With
+// code3 (a third range that repeats a combo) C is left to phase_gather_third.
+template <class T>
+SSB_TRI_HD void phase_gather(int tid, int nt, const Tables &t, const T *r1, const T *r2, const T *r3,
+                             const int *pair1, const int *pair2, const int *pair3, int HS, bool third) {
+    const int m = t.n + 1;
+    for (int i = tid; i < m * m; i += nt) {
+        const int x = i / m, y = i - x * m, at = x * t.S + y;
+        double a = 0.0, b = 0.0, c = 0.0;
+        if (x < t.n && y < t.n) {
+            const int j1 = pair1[x * 52 + y], j2 = pair2[x * 52 + y], j3 = third ? pair3[x * 52 + y] : HS;
+            if (j1 < HS) a = static_cast<double>(r1[j1]);
+            if (j2 < HS) b = static_cast<double>(r2[j2]);
+            if (j3 < HS && r3[j3] > T(0)) c = static_cast<double>(r3[j3]);
+        }
+        t.A[at] = a;
+        t.B[at] = b;
+        t.C[at] = c;
+    }
+}
+
+// phase 1 continued, for a third range that repeats a combo: its hands add up
+// in hand order, one item per row
+template <class T>
+SSB_TRI_HD void phase_gather_third(int tid, int nt, const Tables &t, const T *r3, const int *code3, int H3) {
+    for (int x = tid; x < t.n; x += nt)
+        for (int h = 0; h < H3; ++h) {
+            const int code = code3[h];
+            if ((code & 0x10000) || !(r3[h] > T(0))) continue;   // touches the board, or nothing to add
+            const int p = (code >> 20) & 63, q = (code >> 26) & 63;
+            if (p == x) t.C[x * t.S + q] += static_cast<double>(r3[h]);
+            if (q == x) t.C[x * t.S + p] += static_cast<double>(r3[h]);
+        }
+}
+
+// phase 2: row sums, and AB = A B, CB = C B in 3 x 3 cells per item (A and C
+// are symmetric: row k is column k), each cell summed over k in order
+SSB_TRI_HD void phase_products(int tid, int nt, const Tables &t) {
+    const int n = t.n, S = t.S, nt3 = (n + 2) / 3;
+    for (int i = tid; i < 3 * n; i += nt) {
+        const int c = i % n;
+        const double *M = (i < n ? t.A : i < 2 * n ? t.B : t.C) + c * S;
+        double u = 0.0;
+        for (int x = 0; x < n; ++x) u += M[x];
+        t.v[(i < n ? UA : i < 2 * n ? UB : UC) * kVS + c] = u;
+    }
+    for (int i = tid; i < N_VEC; i += nt) t.v[i * kVS + n] = 0.0;
+    for (int i = tid; i <= n; i += nt) t.AB[n * S + i] = t.AB[i * S + n] = t.CB[n * S + i] = t.CB[i * S + n] = 0.0;
+    for (int q = tid; q < 2 * nt3 * nt3; q += nt) {
+        const bool second = q >= nt3 * nt3;
+        const int r = second ? q - nt3 * nt3 : q;
+        const double *M = second ? t.C : t.A;
+        double *P = second ? t.CB : t.AB;
+        int ii[3], jj[3];
+        for (int i = 0; i < 3; ++i) {   // past the deck: the dummy's zeros
+            ii[i] = r / nt3 * 3 + i < n ? r / nt3 * 3 + i : n;
+            jj[i] = r % nt3 * 3 + i < n ? r % nt3 * 3 + i : n;
+        }
+        double acc[3][3] = {};
+        for (int k = 0; k < n; ++k) {
+            double x[3], y[3];
+            for (int i = 0; i < 3; ++i) {
+                x[i] = M[k * S + ii[i]];
+                y[i] = t.B[k * S + jj[i]];
+            }
+            for (int i = 0; i < 3; ++i)
+                for (int j = 0; j < 3; ++j) acc[i][j] += x[i] * y[j];
+        }
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j)
+                if (ii[i] < n && jj[j] < n) P[ii[i] * S + jj[j]] = acc[i][j];
+    }
+}
+
+// phase 3: the other per-card vectors, one item per (vector, card)
+SSB_TRI_HD void phase_vectors(int tid, int nt, const Tables &t) {
+    const int n = t.n, S = t.S;
+    for (int i = tid; i < 10 * n; i += nt) {
+        const int g = i / n, c = i - g * n;
+        if (g < 6) {
+            const double *M = (g == 0 || g == 2 ? t.A : g == 1 || g == 4 ? t.B : t.C) + c * S;
+            const double *u = t.v + (g == 0 || g == 5 ? UB : g == 1 || g == 3 ? UA : UC) * kVS;
+            double s = 0.0;
+            for (int x = 0; x < n; ++x) s += M[x] * u[x];
+            t.v[(AUB + g) * kVS + c] = s;
+        } else if (g == 6) {
+            double dac = 0.0, h = 0.0;
+            for (int x = 0; x < n; ++x) {
+                const double ac = t.A[c * S + x] * t.C[c * S + x];
+                dac += ac;
+                h += ac * t.B[c * S + x];
+            }
+            t.v[DAC * kVS + c] = dac;
+            t.v[HH * kVS + c] = h;
+            t.v[DAB * kVS + c] = t.AB[c * S + c];
+            t.v[DBC * kVS + c] = t.CB[c * S + c];
+        } else {
+            // (A B C), (C A B) and (A C B) at [c][c]
+            const double *M = (g == 9 ? t.A : t.C) + c * S;
+            const double *P = g == 9 ? t.CB : t.AB;
+            double s = 0.0;
+            for (int x = 0; x < n; ++x) s += M[x] * P[g == 7 ? c * S + x : x * S + c];
+            t.v[(g == 7 ? TABC : g == 8 ? TCAB : TACB) * kVS + c] = s;
+        }
+    }
+}
+
+// phase 4: the scalars, one item each
+SSB_TRI_HD void phase_scalars(int tid, int nt, const Tables &t) {
+    for (int k = tid; k < N_SCAL; k += nt) {
+        const int p = k == QAB || k == QAC ? UA : k == QBC ? UB : -1, q = k == QAB ? UB : UC;
+        const int one = k < 3 ? UA + k : k >= EAB && k <= EBC ? DAB + (k - EAB) : k == SH ? HH : TABC;
+        double s = 0.0;
+        for (int c = 0; c < t.n; ++c)
+            s += p >= 0 ? t.v[p * kVS + c] * t.v[q * kVS + c] : t.v[one * kVS + c];
+        t.sc[k] = k < 3 || (k >= EAB && k <= EBC) ? 0.5 * s : s;
+    }
+}
+
+// the mass of one traverser hand with dense cards (a, b)
+SSB_TRI_HD double hand_mass(int a, int b, const Tables &t) {
+    const int S = t.S;
+    const double *v = t.v, *sc = t.sc;
+    const double Aab = t.A[a * S + b], Bab = t.B[a * S + b], Cab = t.C[a * S + b];
+    const double Aa = v[UA * kVS + a] - Aab, Ab = v[UA * kVS + b] - Aab;
+    const double Ba = v[UB * kVS + a] - Bab, Bb = v[UB * kVS + b] - Bab;
+    const double Ca = v[UC * kVS + a] - Cab, Cb = v[UC * kVS + b] - Cab;
+    double acc = 0.0, ACab = 0.0, ACba = 0.0;   // AC = A C at [a][b] and [b][a]
+#pragma unroll 2
+    for (int x = 0; x < t.n; ++x) {
+        const double Xa = t.A[x * S + a], Xb = t.A[x * S + b];
+        const double Ya = t.B[x * S + a], Yb = t.B[x * S + b];
+        const double Za = t.C[x * S + a], Zb = t.C[x * S + b];
+        ACab += Xa * Zb;
+        ACba += Xb * Za;
+        const bool out = x == a || x == b;
+        const double al = out ? 0.0 : v[UA * kVS + x] - Xa - Xb;
+        const double be = out ? 0.0 : v[UB * kVS + x] - Ya - Yb;
+        const double ga = out ? 0.0 : v[UC * kVS + x] - Za - Zb;
+        // (C' u_B')(x), (B' u_A')(x) + (A' u_B')(x), and d'_BC, d'_AC, d'_AB at x
+        const double cb = v[CUB * kVS + x] - (t.CB[x * S + a] + t.CB[x * S + b]) - Za * Ba - Zb * Bb;
+        const double ba = (v[BUA * kVS + x] + v[AUB * kVS + x]) - (t.AB[a * S + x] + t.AB[b * S + x]) -
+                          (t.AB[x * S + a] + t.AB[x * S + b]) - Ya * Aa - Yb * Ab - Xa * Ba - Xb * Bb;
+        const double dbc = v[DBC * kVS + x] - Ya * Za - Yb * Zb;
+        const double dac = v[DAC * kVS + x] - Xa * Za - Xb * Zb;
+        const double dab = v[DAB * kVS + x] - Xa * Ya - Xb * Yb;
+        acc += al * (2.0 * (be * ga - dbc) + cb) + ga * (ba - 2.0 * dab) - 2.0 * (be * dac);
+    }
+    const double ABs = t.AB[a * S + b] + t.AB[b * S + a], CBab = t.CB[a * S + b], CBba = t.CB[b * S + a];
+    auto at2 = [&](int k) { return v[k * kVS + a] + v[k * kVS + b]; };
+    const double fa = sc[FA] - at2(UA) + Aab, fb = sc[FB] - at2(UB) + Bab, fc = sc[FC] - at2(UC) + Cab;
+    const double qab = sc[QAB] - (at2(AUB) + at2(BUA)) + (at2(DAB) + ABs) - (Aa * Ba + Ab * Bb);
+    const double qac = sc[QAC] - (at2(AUC) + at2(CUA)) + (at2(DAC) + (ACab + ACba)) - (Aa * Ca + Ab * Cb);
+    const double qbc = sc[QBC] - (at2(BUC) + at2(CUB)) + (at2(DBC) + (CBab + CBba)) - (Ba * Ca + Bb * Cb);
+    const double eab = sc[EAB] - at2(DAB) + Aab * Bab;
+    const double eac = sc[EAC] - at2(DAC) + Aab * Cab;
+    const double ebc = sc[EBC] - at2(DBC) + Bab * Cab;
+    const double h = sc[SH] - 2.0 * at2(HH) + 2.0 * (Aab * Bab * Cab);
+    const double tr = sc[TR] - at2(TABC) - at2(TCAB) + ABs * Cab - at2(TACB) + Aab * (CBab + CBba) + Bab * (ACab + ACba);
+    return fa * fb * fc + fc * (eab - qab) + fb * (eac - qac) + fa * (ebc - qbc) + acc + 2.0 * h - tr;
+}
+
+// A computed mass at or below this may be an empty set of tuples (every term
+// is at most a few F_A F_B F_C, its rounding far below the factor here)
+SSB_TRI_HD double zero_bound(const Tables &t) { return 1e-9 * t.sc[FA] * t.sc[FB] * t.sc[FC]; }
+
+// Whether a tuple of positive reach is disjoint and avoids {a, b} (exact):
+// tuple_with asks it for one hand of the third opponent, by the two-opponent
+// count on the positive cells of A and B (row masks mA, mB; row and vector
+// counts as in the mass).  Only hands near zero mass come here, and the first
+// third-opponent hand with a tuple ends it.
+struct Counts {
+    unsigned long long *mA, *mB;   // [kVS]
+    int *nA, *nB, *nW, *nD;        // [kVS]: row counts, (I_B n_A + I_A n_B), common cells
+    long long *s;                  // F_A, F_B, Q, E
+};
+SSB_TRI_HD int popc(unsigned long long x) {
+#if defined(__CUDA_ARCH__)
+    return __popcll(x);
+#else
+    return __builtin_popcountll(x);
+#endif
+}
+SSB_TRI_HD void phase_masks(int tid, int nt, const Tables &t, const Counts &k) {
+    for (int c = tid; c <= t.n; c += nt) {
+        unsigned long long a = 0ull, b = 0ull;
+        for (int x = 0; x < t.n; ++x) {
+            a |= static_cast<unsigned long long>(t.A[c * t.S + x] > 0.0) << x;
+            b |= static_cast<unsigned long long>(t.B[c * t.S + x] > 0.0) << x;
+        }
+        k.mA[c] = a;
+        k.mB[c] = b;
+        k.nA[c] = popc(a);
+        k.nB[c] = popc(b);
+        k.nD[c] = popc(a & b);
+    }
+}
+SSB_TRI_HD void phase_counts(int tid, int nt, const Tables &t, const Counts &k) {
+    for (int c = tid; c <= t.n; c += nt) {
+        int w = 0;
+        for (int x = 0; x < t.n; ++x)
+            w += ((k.mB[c] >> x) & 1ull ? k.nA[x] : 0) + ((k.mA[c] >> x) & 1ull ? k.nB[x] : 0);
+        k.nW[c] = w;
+    }
+    if (tid == nt - 1) {
+        long long fa = 0, fb = 0, q = 0, e = 0;
+        for (int c = 0; c < t.n; ++c) {
+            fa += k.nA[c];
+            fb += k.nB[c];
+            q += static_cast<long long>(k.nA[c]) * k.nB[c];
+            e += k.nD[c];
+        }
+        k.s[0] = fa / 2;
+        k.s[1] = fb / 2;
+        k.s[2] = q;
+        k.s[3] = e / 2;
+    }
+}
+template <class T>
+SSB_TRI_HD bool tuple_with(int a, int b, const Counts &k, T r, int code) {
+    if ((code & 0x10000) || !(r > T(0))) return false;
+    const int s[4] = {a, b, (code >> 20) & 63, (code >> 26) & 63};
+    if (s[2] == a || s[2] == b || s[3] == a || s[3] == b) return false;
+    // pairs of the first two opponents avoiding the four cards
+    long long fa = k.s[0], fb = k.s[1], q = k.s[2], e = k.s[3];
+    for (int i = 0; i < 4; ++i) {
+        const int c = s[i];
+        int na = k.nA[c], nb = k.nB[c];
+        fa -= na;
+        fb -= nb;
+        q -= k.nW[c];
+        e -= k.nD[c];
+        for (int j = 0; j < 4; ++j) {
+            const int f = s[j];
+            const int ab = static_cast<int>((k.mA[c] >> f) & 1ull), bb = static_cast<int>((k.mB[c] >> f) & 1ull);
+            na -= ab;
+            nb -= bb;
+            q += popc(k.mA[c] & k.mB[f]);
+            if (j > i) {
+                fa += ab;
+                fb += bb;
+                e += ab & bb;
+            }
+        }
+        q -= static_cast<long long>(na) * nb;
+    }
+    return fa * fb - q + e > 0;
+}
+
+}  // namespace tri
+}  // namespace ssb
