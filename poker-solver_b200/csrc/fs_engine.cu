@@ -14,12 +14,12 @@
 //     opponent's decisions and through chance nodes, whose average becomes a
 //     weight 1 / cards dealt folded into each frontier row when it is written
 //     (the items' `scale`), so k_cfv sums rows unchanged;
-//   * terminals: one block per terminal stages the opponent's reach row,
-//     cards and (showdowns) 7-card strengths for the node's board in shared
-//     memory; each thread sums its traverser hands over them (at most 200
-//     hands per player by the ABI: 40 K operations per terminal);
-//   * strengths: once per solve for every river board of the tree with the
-//     device ranker (ss_rank.cuh), instead of once per showdown node;
+//   * terminals: one warp per terminal over the opponent's reach row, with the
+//     ranges' tables or the river board's in the block's shared memory: sums
+//     per card and in strength order, then O(1) per traverser hand;
+//   * strengths and the tables by strength: once per solve for every river
+//     board of the tree on the device (k_fs_tables), instead of once per
+//     showdown node;
 //   * iterations are captured as CUDA graphs with the counter on the device.
 // fs_solve_gpu_extract_all reads the average strategy of every node and the
 // last traverser's values at every node (terminals, both players' decisions,
@@ -243,6 +243,14 @@ int build_plan(const FSTreeData &td, FsPlan *out) {
                 board_row[x] = static_cast<int>(std::lower_bound(uk.begin(), uk.end(), k) - uk.begin());
             }
     }
+    // each board's first showdown item
+    P.bstart.assign(P.sboards.size() / 5 + 1, 0);
+    int n_fold = 0;
+    for (int x = 0; x < N; ++x) {
+        n_fold += nd[x].type == FS_NODE_FOLD;
+        if (board_row[x] >= 0) ++P.bstart[board_row[x] + 1];
+    }
+    for (size_t b = 1; b < P.bstart.size(); ++b) P.bstart[b] += P.bstart[b - 1];
     for (int t = 0; t < 2; ++t) {
         // chance weights for traverser t again (the loop above kept t = 1's)
         for (int x : order) {
@@ -255,7 +263,10 @@ int build_plan(const FSTreeData &td, FsPlan *out) {
                    : nd[par].type == FS_NODE_CHANCE ? w[par] / nd[par].num_children
                                                     : w[par];
         }
-        P.term[t].clear();
+        // folds first, then showdowns by river board (one launch each)
+        P.term[t].resize(static_cast<size_t>(n_fold) + P.bstart.back());
+        int fold_at = 0;
+        std::vector<int> sd_at(P.bstart);
         for (int x = 0; x < N; ++x) {
             const FSNode &n = nd[x];
             if (n.type != FS_NODE_FOLD && n.type != FS_NODE_SHOWDOWN) continue;
@@ -274,12 +285,9 @@ int build_plan(const FSTreeData &td, FsPlan *out) {
             it.scale = static_cast<float>(w[x]);
             it.nb = n.num_board;
             for (int b = 0; b < n.num_board; ++b) it.board[b] = n.board_cards[b];
-            P.term[t].push_back(it);
+            P.term[t][n.type == FS_NODE_FOLD ? fold_at++ : n_fold + sd_at[board_row[x]]++] = it;
         }
-        // folds first, then showdowns (one launch each)
-        std::stable_partition(P.term[t].begin(), P.term[t].end(), [](const FsTermItem &i) { return i.kind == 0; });
-        P.nfold[t] = static_cast<int>(std::count_if(P.term[t].begin(), P.term[t].end(),
-                                                    [](const FsTermItem &i) { return i.kind == 0; }));
+        P.nfold[t] = n_fold;
     }
     // hands, and per player the hands holding each card (folds)
     const int HSi = P.HS;
@@ -301,75 +309,18 @@ int build_plan(const FSTreeData &td, FsPlan *out) {
         }
         P.f_coff[p * 53 + 52] = at;
     }
-    // showdown tables per river board (see fs_engine.h)
-    const int nsb = static_cast<int>(P.sboards.size() / 5);
-    P.sd_str.assign(static_cast<size_t>(nsb) * 2 * HSi, 0u);
-    P.sd_ord.assign(static_cast<size_t>(nsb) * 2 * HSi, -1);
-    P.sd_hpos.assign(static_cast<size_t>(nsb) * 2 * HSi * 4, 0);
-    P.sd_coff.assign(static_cast<size_t>(nsb) * 2 * 53, 0);
-    P.sd_clist.assign(static_cast<size_t>(nsb) * 2 * 2 * HSi, 0);
-    for (int bi = 0; bi < nsb; ++bi) {
-        const int *bd = &P.sboards[5 * bi];
-        std::vector<unsigned> srt[2];
-        for (int p = 0; p < 2; ++p) {
-            unsigned *str = &P.sd_str[(static_cast<size_t>(bi) * 2 + p) * HSi];
-            for (int h = 0; h < P.H[p]; ++h) str[h] = rank7_host(bd, td.hands[p][h][0], td.hands[p][h][1]);
-            int *ord = &P.sd_ord[(static_cast<size_t>(bi) * 2 + p) * HSi];
-            std::vector<int> idx(P.H[p]);
-            for (int h = 0; h < P.H[p]; ++h) idx[h] = h;
-            std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return str[x] < str[y]; });
-            std::vector<int> pos(P.H[p]);
-            for (int k = 0; k < P.H[p]; ++k) {
-                ord[k] = idx[k];
-                pos[idx[k]] = k;
-                srt[p].push_back(str[idx[k]]);
-            }
-            // card lists of this player as the opponent, by position
-            std::vector<std::vector<int>> byc(52);
-            for (int k = 0; k < P.H[p]; ++k) {
-                byc[td.hands[p][idx[k]][0]].push_back(k);
-                byc[td.hands[p][idx[k]][1]].push_back(k);
-            }
-            int *coff = &P.sd_coff[(static_cast<size_t>(bi) * 2 + p) * 53];
-            int *cl = &P.sd_clist[(static_cast<size_t>(bi) * 2 + p) * 2 * HSi];
-            int at = 0;
-            for (int c = 0; c < 52; ++c) {
-                coff[c] = at;
-                for (int k : byc[c]) cl[at++] = k;
-            }
-            coff[52] = at;
+    // each hand's combo in the opponent's range (where combos repeat, the last)
+    P.f_same.assign(2 * static_cast<size_t>(HSi), -1);
+    for (int p = 0; p < 2; ++p) {
+        std::vector<int> of(52 * 52, -1);
+        P.dup[p] = 0;
+        for (int h = 0; h < P.H[p]; ++h) {
+            const int a = td.hands[p][h][0], b = td.hands[p][h][1];
+            if (of[a * 52 + b] >= 0) P.dup[p] = 1;
+            of[a * 52 + b] = of[b * 52 + a] = h;
         }
-        for (int t = 0; t < 2; ++t) {
-            const int o = 1 - t;
-            const unsigned *st = &P.sd_str[(static_cast<size_t>(bi) * 2 + t) * HSi];
-            const unsigned *so = &P.sd_str[(static_cast<size_t>(bi) * 2 + o) * HSi];
-            const int *coff = &P.sd_coff[(static_cast<size_t>(bi) * 2 + o) * 53];
-            const int *cl = &P.sd_clist[(static_cast<size_t>(bi) * 2 + o) * 2 * HSi];
-            const int *ordo = &P.sd_ord[(static_cast<size_t>(bi) * 2 + o) * HSi];
-            for (int h = 0; h < P.H[t]; ++h) {
-                const unsigned s = st[h];
-                const int lo = static_cast<int>(std::lower_bound(srt[o].begin(), srt[o].end(), s) - srt[o].begin());
-                const int hi = static_cast<int>(std::upper_bound(srt[o].begin(), srt[o].end(), s) - srt[o].begin());
-                const int c1 = td.hands[t][h][0], c2 = td.hands[t][h][1];
-                int cnt[2][2];
-                const int cs[2] = {c1, c2};
-                for (int j = 0; j < 2; ++j) {
-                    int below = 0, upto = 0;
-                    for (int k = coff[cs[j]]; k < coff[cs[j] + 1]; ++k) {
-                        const unsigned x = so[ordo[cl[k]]];
-                        below += x < s;
-                        upto += x <= s;
-                    }
-                    cnt[j][0] = below;
-                    cnt[j][1] = upto;
-                }
-                int *hp = &P.sd_hpos[((static_cast<size_t>(bi) * 2 + t) * HSi + h) * 4];
-                hp[0] = lo | (hi << 16);
-                hp[1] = c1 | (c2 << 8);
-                hp[2] = cnt[0][0] | (cnt[0][1] << 16);
-                hp[3] = cnt[1][0] | (cnt[1][1] << 16);
-            }
-        }
+        for (int h = 0; h < P.H[1 - p]; ++h)
+            P.f_same[(1 - p) * HSi + h] = of[td.hands[1 - p][h][0] * 52 + td.hands[1 - p][h][1]];
     }
     // read-out levels: BFS depth, deepest first
     int maxd = 0;
@@ -392,98 +343,217 @@ namespace {
 
 constexpr int kFsThreads = 256;
 
-// Folds (flop_solve.cu:731-779): payoff x the opponent's reach over hands
-// sharing no card with the traverser's hand {a, b} or with the node's board.
-// One block per terminal: the opponent's hands the board leaves are staged
-// (reach in FP64, and whether it is positive); per card c their sums u(c),
-// and F in all; then per traverser hand
-//   mass = F - u(a) - u(b) + (the opponent's reach on the combo {a, b}),
-// the last term from the opponent's list of card a.  The same sums over 0/1
-// count the opponent hands with positive reach; none gives exactly 0, as the
-// reference's sum of zeros does.
 struct FsTables {
     const int *hand_cards;                    // [2][HS]
     const int *f_coff, *f_clist;              // [2][53], [2][2 HS]
+    const int *f_same;                        // [2][HS]: the opponent's hand of the same two cards, -1 if none
+    int dup[2];                               // the player's range repeats a combo
     const unsigned *sd_str;                   // [nsb][2][HS]
     const int *sd_ord, *sd_hpos, *sd_coff, *sd_clist;
     int HS, H0, H1;
 };
 
-__global__ void __launch_bounds__(kFsThreads) k_fs_fold(const FsTermItem *__restrict__ items, int trav,
+// The showdown tables of every river board (layouts in fs_engine.h), one block
+// per board, straight into device memory: 7-card strengths, then positions,
+// card lists and the traverser's bounds by counting over the at most 200 hands
+// of each player in shared memory (200 broadcast reads per entry).  On the
+// host the same tables (2,352 boards, 200 hands: 34 MB) took 300 ms of sorting
+// and the copy; here they are not worth a mention beside one iteration.
+struct FsTableOut {
+    unsigned *str;
+    int *ord, *hpos, *coff, *clist;
+};
+__global__ void __launch_bounds__(kFsThreads) k_fs_tables(const int *__restrict__ boards,
+                                                         const int *__restrict__ hand_cards, FsTableOut O, int HS,
+                                                         int H0, int H1) {
+    __shared__ unsigned st[2][FS_MAX_HANDS];
+    __shared__ int cd[2][FS_MAX_HANDS];
+    __shared__ short pos[2][FS_MAX_HANDS];
+    __shared__ int off[2][53];
+    const int tid = threadIdx.x;
+    const size_t row = static_cast<size_t>(blockIdx.x) * 2;
+    const size_t hs = static_cast<size_t>(HS);
+    const int H[2] = {H0, H1};
+    int bd[5];
+    for (int i = 0; i < 5; ++i) bd[i] = __ldg(boards + 5 * blockIdx.x + i);
+    static_assert(FS_MAX_HANDS <= kFsThreads, "one thread per hand");
+    for (int p = 0; p < 2; ++p)
+        if (tid < H[p]) {
+            const int code = __ldg(hand_cards + p * HS + tid);
+            const int c[7] = {bd[0], bd[1], bd[2], bd[3], bd[4], code & 0xff, (code >> 8) & 0xff};
+            bool repeat = false;
+            for (int i = 0; i < 7; ++i)
+                for (int j = i + 1; j < 7; ++j) repeat |= c[i] == c[j];
+            const unsigned v = repeat ? 0u : rank7(c);
+            st[p][tid] = v;
+            cd[p][tid] = code;
+            O.str[(row + p) * hs + tid] = v;
+        }
+    __syncthreads();
+    // positions by ascending strength, ties in hand order
+    for (int p = 0; p < 2; ++p)
+        if (tid < H[p]) {
+            const unsigned v = st[p][tid];
+            int k = 0;
+            for (int j = 0; j < H[p]; ++j) k += st[p][j] < v || (st[p][j] == v && j < tid);
+            pos[p][tid] = static_cast<short>(k);
+            O.ord[(row + p) * hs + k] = tid;
+        }
+    // hands per card
+    if (tid < 2 * 52) {
+        const int p = tid / 52, c = tid - p * 52;
+        int n = 0;
+        for (int j = 0; j < H[p]; ++j) n += (cd[p][j] & 0xff) == c || ((cd[p][j] >> 8) & 0xff) == c;
+        off[p][c + 1] = n;
+    }
+    __syncthreads();
+    if (tid < 2) {
+        off[tid][0] = 0;
+        for (int c = 0; c < 52; ++c) off[tid][c + 1] += off[tid][c];
+    }
+    __syncthreads();
+    if (tid < 2 * 53) O.coff[row * 53 + tid] = off[tid / 53][tid % 53];
+    for (int p = 0; p < 2; ++p)
+        if (tid < H[p]) {
+            // this hand's place in the lists of its two cards (as the opponent)
+            const int c1 = cd[p][tid] & 0xff, c2 = (cd[p][tid] >> 8) & 0xff, k = pos[p][tid];
+            int k1 = 0, k2 = 0;
+            for (int j = 0; j < H[p]; ++j) {
+                const int x = cd[p][j] & 0xff, y = (cd[p][j] >> 8) & 0xff;
+                const bool before = pos[p][j] < k;
+                k1 += before && (x == c1 || y == c1);
+                k2 += before && (x == c2 || y == c2);
+            }
+            O.clist[(row + p) * 2 * hs + off[p][c1] + k1] = k;
+            O.clist[(row + p) * 2 * hs + off[p][c2] + k2] = k;
+            // its bounds among the opponent's hands (as the traverser)
+            const int o = 1 - p;
+            const unsigned v = st[p][tid];
+            int lo = 0, hi = 0, l1 = 0, h1 = 0, l2 = 0, h2 = 0;
+            for (int j = 0; j < H[o]; ++j) {
+                const int x = cd[o][j] & 0xff, y = (cd[o][j] >> 8) & 0xff;
+                const bool w = st[o][j] < v, we = st[o][j] <= v;
+                const bool on1 = x == c1 || y == c1, on2 = x == c2 || y == c2;
+                lo += w;
+                hi += we;
+                l1 += w && on1;
+                h1 += we && on1;
+                l2 += w && on2;
+                h2 += we && on2;
+            }
+            reinterpret_cast<int4 *>(O.hpos)[(row + p) * hs + tid] =
+                make_int4(lo | (hi << 16), c1 | (c2 << 8), l1 | (h1 << 16), l2 | (h2 << 16));
+        }
+}
+
+// Terminals: one warp per terminal and no block barriers (a block per terminal
+// spent its time waiting at three of them: 764 us for 113,488 folds, 640 us
+// for 152,880 showdowns of 200 hands; now 182 and 374 us).  What the terminals of a block share
+// sits in shared memory: the ranges' tables (folds), one river board's tables
+// (showdowns).  Every sum keeps a fixed order: positions or hands in runs per
+// lane, lists in list order.
+constexpr int kFsWarps = kFsThreads / 32;
+constexpr int kFsRun = (FS_MAX_HANDS + 31) / 32;   // hands or positions per lane
+
+// Folds (flop_solve.cu:731-779): payoff x the opponent's reach over hands
+// sharing no card with the traverser's hand {a, b} or with the node's board.
+// Per terminal: the opponent's hands the board leaves; per card c their sums
+// u(c), and F in all; then per traverser hand
+//   mass = F - u(a) - u(b) + (the opponent's reach on the combo {a, b}),
+// the last term by the table of equal combos (or, in a range that repeats a
+// combo, from the opponent's list of card a).  The same sums over 0/1
+// count the opponent hands with positive reach; none gives exactly 0, as the
+// reference's sum of zeros does.
+__global__ void __launch_bounds__(kFsThreads) k_fs_fold(const FsTermItem *__restrict__ items, int n, int trav,
                                                        const float *__restrict__ reach, FsTables T,
                                                        float *__restrict__ out, int scaled) {
-    __shared__ double r_o[FS_MAX_HANDS];
-    __shared__ double u[52];
-    __shared__ int cu[52];
-    __shared__ double tot[kFsThreads / 32];
-    __shared__ int ctot[kFsThreads / 32];
-    const FsTermItem I = items[blockIdx.x];
+    __shared__ unsigned long long mask_o[FS_MAX_HANDS];
+    __shared__ short list[2 * FS_MAX_HANDS], off[53], same_t[FS_MAX_HANDS];
+    __shared__ unsigned char ca[FS_MAX_HANDS], cb[FS_MAX_HANDS];
+    __shared__ double r_w[kFsWarps][FS_MAX_HANDS];
+    __shared__ double u_w[kFsWarps][52];
+    __shared__ int cu_w[kFsWarps][52];
     const int opp = 1 - trav;
     const int Ho = opp == 0 ? T.H0 : T.H1, Ht = trav == 0 ? T.H0 : T.H1;
     const size_t hs = static_cast<size_t>(T.HS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double f = 0.0;
-    int cf = 0;
-    for (int o = tid; o < Ho; o += blockDim.x) {
-        const int code = T.hand_cards[opp * T.HS + o];
-        const int x = code & 0xff, y = (code >> 8) & 0xff;
-        bool blocked = false;
-        for (int k = 0; k < I.nb; ++k) blocked |= x == I.board[k] || y == I.board[k];
-        const double r = blocked ? 0.0 : static_cast<double>(reach[static_cast<size_t>(I.opp_row) * hs + o]);
-        r_o[o] = blocked ? -1.0 : r;   // -1: the board blocks the hand
-        f += r;
-        cf += (!blocked && r > 0.0) ? 1 : 0;
+    const bool dup = T.dup[opp] != 0;
+    if (tid < Ho) {
+        const int code = T.hand_cards[opp * T.HS + tid];
+        mask_o[tid] = (1ull << (code & 0xff)) | (1ull << ((code >> 8) & 0xff));
     }
-    for (int k = 16; k > 0; k >>= 1) {
-        f += __shfl_xor_sync(0xffffffffu, f, k);
-        cf += __shfl_xor_sync(0xffffffffu, cf, k);
+    if (tid < Ht) {
+        const int code = T.hand_cards[trav * T.HS + tid];
+        ca[tid] = static_cast<unsigned char>(code & 0xff);
+        cb[tid] = static_cast<unsigned char>((code >> 8) & 0xff);
+        same_t[tid] = static_cast<short>(T.f_same[trav * T.HS + tid]);
     }
-    if (lane == 0) {
-        tot[warp] = f;
-        ctot[warp] = cf;
-    }
+    if (tid < 53) off[tid] = static_cast<short>(T.f_coff[opp * 53 + tid]);
+    for (int k = tid; k < 2 * Ho; k += kFsThreads) list[k] = static_cast<short>(T.f_clist[opp * 2 * T.HS + k]);
     __syncthreads();
-    if (tid < 52) {
-        double s = 0.0;
-        int n = 0;
-        const int *cl = T.f_clist + opp * 2 * T.HS;
-        for (int k = T.f_coff[opp * 53 + tid]; k < T.f_coff[opp * 53 + tid + 1]; ++k) {
-            const double r = r_o[cl[k]];
-            if (r >= 0.0) {
+    double *r_o = r_w[warp], *u = u_w[warp];
+    int *cu = cu_w[warp];
+    for (int i = blockIdx.x * kFsWarps + warp; i < n; i += gridDim.x * kFsWarps) {
+        const FsTermItem I = items[i];
+        unsigned long long board = 0ull;
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            if (k < I.nb) board |= 1ull << I.board[k];
+        const float *row = reach + static_cast<size_t>(I.opp_row) * hs;
+        float x[kFsRun];
+#pragma unroll
+        for (int g = 0; g < kFsRun; ++g) x[g] = g * 32 + lane < Ho ? row[g * 32 + lane] : 0.f;
+        double F = 0.0;
+        int CF = 0;
+#pragma unroll
+        for (int g = 0; g < kFsRun; ++g) {
+            const int o = g * 32 + lane;
+            const bool on = o < Ho && !(mask_o[o] & board);
+            double f = on ? static_cast<double>(x[g]) : 0.0;
+            if (o < Ho) r_o[o] = f;
+            CF += __popc(__ballot_sync(0xffffffffu, f > 0.0));
+#pragma unroll
+            for (int k = 16; k > 0; k >>= 1) f += __shfl_xor_sync(0xffffffffu, f, k);
+            F += f;
+        }
+        __syncwarp();
+        for (int c = lane; c < 52; c += 32) {
+            double s = 0.0;
+            int m = 0;
+            for (int k = off[c]; k < off[c + 1]; ++k) {
+                const double r = r_o[list[k]];
                 s += r;
-                n += r > 0.0 ? 1 : 0;
+                m += r > 0.0 ? 1 : 0;
             }
+            u[c] = s;
+            cu[c] = m;
         }
-        u[tid] = s;
-        cu[tid] = n;
-    }
-    __syncthreads();
-    double F = 0.0;
-    int CF = 0;
-    for (int w = 0; w < kFsThreads / 32; ++w) {
-        F += tot[w];
-        CF += ctot[w];
-    }
-    const float sc = scaled ? I.scale : 1.0f;
-    const int *cl = T.f_clist + opp * 2 * T.HS;
-    for (int h = tid; h < Ht; h += blockDim.x) {
-        const int code = T.hand_cards[trav * T.HS + h];
-        const int a = code & 0xff, b = (code >> 8) & 0xff;
-        double same = 0.0;
-        int csame = 0;
-        for (int k = T.f_coff[opp * 53 + a]; k < T.f_coff[opp * 53 + a + 1]; ++k) {
-            const int o = cl[k];
-            const int oc = T.hand_cards[opp * T.HS + o];
-            if ((oc & 0xff) != b && ((oc >> 8) & 0xff) != b) continue;
-            const double r = r_o[o];
-            if (r >= 0.0) {
-                same += r;
-                csame += r > 0.0 ? 1 : 0;
+        __syncwarp();
+        const float sc = scaled ? I.scale : 1.0f;
+        float *dst = out + static_cast<size_t>(I.node) * hs;
+        for (int h = lane; h < Ht; h += 32) {
+            const int a = ca[h], b = cb[h];
+            double same = 0.0;
+            int csame = 0;
+            if (!dup) {
+                const int o = same_t[h];
+                if (o >= 0) {
+                    same = r_o[o];
+                    csame = same > 0.0 ? 1 : 0;
+                }
+            } else {
+                for (int k = off[a]; k < off[a + 1]; ++k) {
+                    const int o = list[k];
+                    if (!(mask_o[o] >> b & 1ull)) continue;
+                    same += r_o[o];
+                    csame += r_o[o] > 0.0 ? 1 : 0;
+                }
             }
+            const int cnt = CF - cu[a] - cu[b] + csame;
+            const double mass = cnt == 0 ? 0.0 : F - u[a] - u[b] + same;
+            dst[h] = static_cast<float>(mass) * I.payoff * sc;
         }
-        const int cnt = CF - cu[a] - cu[b] + csame;
-        const double mass = cnt == 0 ? 0.0 : F - u[a] - u[b] + same;
-        out[static_cast<size_t>(I.node) * hs + h] = static_cast<float>(mass) * I.payoff * sc;
+        __syncwarp();
     }
 }
 
@@ -494,102 +564,144 @@ __global__ void __launch_bounds__(kFsThreads) k_fs_fold(const FsTermItem *__rest
 // holding one of its two cards (their own prefix sums along each card's
 // list); value = (W - L) x half_pot, FP64 sums.  The same on 0/1 counts
 // gives exactly 0 where no positive-reach opponent hand wins or loses.
-__global__ void __launch_bounds__(kFsThreads) k_fs_showdown(const FsTermItem *__restrict__ items, int trav,
+// One block per river board: its terminals [bstart[b], bstart[b + 1]) are
+// consecutive items.
+//
+// Bound by shared-memory wavefronts, so the zero test keeps no counts beside
+// the sums: a W or L above 1e-9 of the opponent's whole reach cannot be the
+// rounding of an empty set (a few hundred roundings of 1e-16), an exact 0 is
+// the answer either way, and only what lies between is looked up exactly, as
+// 7 words of positive positions against the card masks of the board.
+struct FsSdWarp {
+    double P[FS_MAX_HANDS + 1];
+    double PC[2 * FS_MAX_HANDS + 52];
+    float x[FS_MAX_HANDS];
+};
+constexpr size_t fs_sd_smem() {
+    return FS_MAX_HANDS * sizeof(int4) + kFsWarps * sizeof(FsSdWarp) + 52 * kFsRun * sizeof(unsigned) +
+           (FS_MAX_HANDS + 2 * FS_MAX_HANDS + 64 + FS_MAX_HANDS) * sizeof(short) + 16;
+}
+__global__ void __launch_bounds__(kFsThreads) k_fs_showdown(const FsTermItem *__restrict__ items,
+                                                           const int *__restrict__ bstart, int trav,
                                                            const float *__restrict__ reach, FsTables T,
                                                            float *__restrict__ out, int scaled) {
-    __shared__ double P[FS_MAX_HANDS + 1];
-    __shared__ int Pc[FS_MAX_HANDS + 1];
-    __shared__ double PC[2 * FS_MAX_HANDS + 52];
-    __shared__ int PCc[2 * FS_MAX_HANDS + 52];
-    __shared__ double x_s[FS_MAX_HANDS];
-    const FsTermItem I = items[blockIdx.x];
+    extern __shared__ __align__(16) char smem[];
+    int4 *hpos = reinterpret_cast<int4 *>(smem);                               // [Ht]
+    FsSdWarp *all = reinterpret_cast<FsSdWarp *>(hpos + FS_MAX_HANDS);
+    unsigned *cmask = reinterpret_cast<unsigned *>(all + kFsWarps);             // [52][kFsRun] positions holding a card
+    short *ord = reinterpret_cast<short *>(cmask + 52 * kFsRun);                // [Ho], -1 where the board blocks it
+    short *list = ord + FS_MAX_HANDS, *off = list + 2 * FS_MAX_HANDS;           // [2 Ho], [53]
+    short *live = off + 64;                                                     // [Ht]
     const int opp = 1 - trav;
     const int Ho = opp == 0 ? T.H0 : T.H1, Ht = trav == 0 ? T.H0 : T.H1;
     const size_t hs = static_cast<size_t>(T.HS);
-    const int tid = threadIdx.x, lane = tid & 31;
-    const size_t bo = static_cast<size_t>(I.sboard) * 2 + opp, bt = static_cast<size_t>(I.sboard) * 2 + trav;
-    const int *ord = T.sd_ord + bo * hs;
-    const unsigned *so = T.sd_str + bo * hs;
-    // the opponent's reach by position (0 where the board blocks the hand)
-    for (int k = tid; k < Ho; k += blockDim.x) {
-        const int o = ord[k];
-        x_s[k] = so[o] == 0u ? 0.0 : static_cast<double>(reach[static_cast<size_t>(I.opp_row) * hs + o]);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const size_t bo = static_cast<size_t>(blockIdx.x) * 2 + opp, bt = static_cast<size_t>(blockIdx.x) * 2 + trav;
+    for (int i = tid; i < 52 * kFsRun; i += kFsThreads) cmask[i] = 0u;
+    if (tid < Ho) {
+        const int o = T.sd_ord[bo * hs + tid];
+        ord[tid] = static_cast<short>(T.sd_str[bo * hs + o] == 0u ? -1 : o);
     }
+    if (tid < Ht) {
+        hpos[tid] = reinterpret_cast<const int4 *>(T.sd_hpos)[bt * hs + tid];
+        live[tid] = T.sd_str[bt * hs + tid] != 0u;
+    }
+    if (tid < 53) off[tid] = static_cast<short>(T.sd_coff[bo * 53 + tid]);
+    for (int k = tid; k < 2 * Ho; k += kFsThreads) list[k] = static_cast<short>(T.sd_clist[bo * 2 * hs + k]);
     __syncthreads();
-    if (tid < 32) {
-        // prefix sums over positions: each lane a run of consecutive
-        // positions, lane totals scanned across the warp (fixed order)
-        constexpr int kRun = (FS_MAX_HANDS + 31) / 32;
-        const int k0 = lane * kRun;
+    // position k is bit k / kFsRun of word k % kFsRun (the warp's ballots below)
+    if (tid < 52)
+        for (int k = off[tid]; k < off[tid + 1]; ++k) cmask[tid * kFsRun + list[k] % kFsRun] |= 1u << (list[k] / kFsRun);
+    __syncthreads();
+    FsSdWarp &W = all[warp];
+    for (int i = bstart[blockIdx.x] + warp; i < bstart[blockIdx.x + 1]; i += kFsWarps) {
+        const FsTermItem &I = items[i];
+        const float *row = reach + static_cast<size_t>(I.opp_row) * hs;
+        // the opponent's reach by position (0 where the board blocks the
+        // hand): each lane a run of consecutive positions
+        const int k0 = lane * kFsRun;
+        float x[kFsRun];
+        unsigned live_k[kFsRun];
+#pragma unroll
+        for (int j = 0; j < kFsRun; ++j) {
+            const int o = k0 + j < Ho ? ord[k0 + j] : -1;
+            x[j] = o >= 0 ? row[o] : 0.f;
+        }
         double s = 0.0;
-        int n = 0;
-        for (int i = 0; i < kRun; ++i)
-            if (k0 + i < Ho) {
-                s += x_s[k0 + i];
-                n += x_s[k0 + i] > 0.0 ? 1 : 0;
+#pragma unroll
+        for (int j = 0; j < kFsRun; ++j) {
+            live_k[j] = __ballot_sync(0xffffffffu, x[j] > 0.f);
+            if (k0 + j < Ho) {
+                W.x[k0 + j] = x[j];
+                s += static_cast<double>(x[j]);
             }
+        }
+        // prefix sums over positions: lane totals scanned across the warp
+        // (fixed order), then along each lane's run
         double incl = s;
-        int nincl = n;
+#pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const double v = __shfl_up_sync(0xffffffffu, incl, d);
-            const int m = __shfl_up_sync(0xffffffffu, nincl, d);
-            if (lane >= d) {
-                incl += v;
-                nincl += m;
-            }
+            if (lane >= d) incl += v;
         }
         double run = incl - s;
-        int nrun = nincl - n;
-        for (int i = 0; i < kRun; ++i)
-            if (k0 + i < Ho) {
-                P[k0 + i] = run;
-                Pc[k0 + i] = nrun;
-                run += x_s[k0 + i];
-                nrun += x_s[k0 + i] > 0.0 ? 1 : 0;
+#pragma unroll
+        for (int j = 0; j < kFsRun; ++j)
+            if (k0 + j < Ho) {
+                W.P[k0 + j] = run;
+                run += static_cast<double>(x[j]);
             }
-        if (lane == 31) {
-            P[Ho] = incl;
-            Pc[Ho] = nincl;
-        }
-    } else if (tid >= 64 && tid < 64 + 52) {
+        const double total = __shfl_sync(0xffffffffu, incl, 31);
+        if (lane == 31) W.P[Ho] = incl;
+        __syncwarp();
         // per card: prefix sums along the opponent's hands holding it
-        const int c = tid - 64;
-        const int *coff = T.sd_coff + bo * 53;
-        const int *cl = T.sd_clist + bo * 2 * hs;
-        const int base = coff[c] + c;
-        double s = 0.0;
-        int n = 0;
-        PC[base] = 0.0;
-        PCc[base] = 0;
-        for (int k = coff[c]; k < coff[c + 1]; ++k) {
-            const double v = x_s[cl[k]];
-            s += v;
-            n += v > 0.0 ? 1 : 0;
-            PC[base + (k - coff[c]) + 1] = s;
-            PCc[base + (k - coff[c]) + 1] = n;
+        for (int c = lane; c < 52; c += 32) {
+            const int b0 = off[c], b1 = off[c + 1];
+            double q = 0.0;
+            W.PC[b0 + c] = 0.0;
+            for (int k = b0; k < b1; ++k) {
+                q += static_cast<double>(W.x[list[k]]);
+                W.PC[k + c + 1] = q;
+            }
         }
-    }
-    __syncthreads();
-    const float sc = scaled ? I.scale : 1.0f;
-    const unsigned *st = T.sd_str + bt * hs;
-    const int *coff = T.sd_coff + bo * 53;
-    for (int h = tid; h < Ht; h += blockDim.x) {
-        float v = 0.f;
-        if (st[h] != 0u) {
-            const int4 hp = reinterpret_cast<const int4 *>(T.sd_hpos)[bt * hs + h];
-            const int lo = hp.x & 0xffff, hi = hp.x >> 16;
-            const int c1 = hp.y & 0xff, c2 = (hp.y >> 8) & 0xff;
-            const int b1 = coff[c1] + c1, n1 = coff[c1 + 1] - coff[c1];
-            const int b2 = coff[c2] + c2, n2 = coff[c2 + 1] - coff[c2];
-            const int l1lo = hp.z & 0xffff, l1hi = hp.z >> 16, l2lo = hp.w & 0xffff, l2hi = hp.w >> 16;
-            const double W = P[lo] - PC[b1 + l1lo] - PC[b2 + l2lo];
-            const double L = (P[Ho] - P[hi]) - (PC[b1 + n1] - PC[b1 + l1hi]) - (PC[b2 + n2] - PC[b2 + l2hi]);
-            const int cw = Pc[lo] - PCc[b1 + l1lo] - PCc[b2 + l2lo];
-            const int closs = (Pc[Ho] - Pc[hi]) - (PCc[b1 + n1] - PCc[b1 + l1hi]) - (PCc[b2 + n2] - PCc[b2 + l2hi]);
-            const double w = cw == 0 ? 0.0 : W, l = closs == 0 ? 0.0 : L;
-            v = static_cast<float>((w - l) * static_cast<double>(I.half_pot));
+        __syncwarp();
+        // whether an opponent hand of positive reach at a position in
+        // [from, to) holds neither c1 nor c2
+        auto any_in = [&](int c1, int c2, int from, int to) {
+            unsigned hit = 0u;
+#pragma unroll
+            for (int j = 0; j < kFsRun; ++j) {
+                const int nf = max(0, (from - j + kFsRun - 1) / kFsRun), nt = max(0, (to - j + kFsRun - 1) / kFsRun);
+                const unsigned in = ((nt >= 32 ? 0u : 1u << nt) - 1u) & ~((nf >= 32 ? 0u : 1u << nf) - 1u);
+                hit |= live_k[j] & in & ~cmask[c1 * kFsRun + j] & ~cmask[c2 * kFsRun + j];
+            }
+            return hit != 0u;
+        };
+        bool odd = false;   // a negative or NaN reach voids the bound: look everything up
+#pragma unroll
+        for (int j = 0; j < kFsRun; ++j) odd |= !(x[j] >= 0.f);
+        const double zb = __any_sync(0xffffffffu, odd) ? __longlong_as_double(0x7ff0000000000000ll) : 1e-9 * total;
+        const float sc = scaled ? I.scale : 1.0f;
+        const double half_pot = static_cast<double>(I.half_pot);
+        float *dst = out + static_cast<size_t>(I.node) * hs;
+        for (int h = lane; h < Ht; h += 32) {
+            float v = 0.f;
+            if (live[h]) {
+                const int4 hp = hpos[h];
+                const int lo = hp.x & 0xffff, hi = hp.x >> 16;
+                const int c1 = hp.y & 0xff, c2 = (hp.y >> 8) & 0xff;
+                const int b1 = off[c1] + c1, e1 = off[c1 + 1] + c1;
+                const int b2 = off[c2] + c2, e2 = off[c2 + 1] + c2;
+                const int l1lo = hp.z & 0xffff, l1hi = hp.z >> 16, l2lo = hp.w & 0xffff, l2hi = hp.w >> 16;
+                double w = W.P[lo] - W.PC[b1 + l1lo] - W.PC[b2 + l2lo];
+                double l = (total - W.P[hi]) - (W.PC[e1] - W.PC[b1 + l1hi]) - (W.PC[e2] - W.PC[b2 + l2hi]);
+                if (w != 0.0 && !(fabs(w) > zb) && !any_in(c1, c2, 0, lo)) w = 0.0;
+                if (l != 0.0 && !(fabs(l) > zb) && !any_in(c1, c2, hi, Ho)) l = 0.0;
+                v = static_cast<float>((w - l) * half_pot);
+            }
+            dst[h] = v * sc;
         }
-        out[static_cast<size_t>(I.node) * hs + h] = v * sc;
+        __syncwarp();
     }
 }
 
@@ -665,7 +777,7 @@ class Solve {
   public:
     FsPlan P;
     cudaStream_t stream = nullptr;
-    char *dbase = nullptr;
+    char *dbase = nullptr, *dtab = nullptr;
     float *dstate = nullptr;
     int *diter = nullptr;
     float *dsnap = nullptr;
@@ -677,6 +789,7 @@ class Solve {
     const FsTermItem *term_items[2] = {};
     const int *hand_cards = nullptr, *edge_first = nullptr, *edge_na = nullptr, *depth_nodes = nullptr;
     FsTables tab{};
+    const int *bstart = nullptr;
     FSNode *dnodes = nullptr;
     int *dchildren = nullptr;
     const int *dfirst_edge = nullptr;
@@ -686,7 +799,7 @@ class Solve {
     ~Solve() {
         if (gblock) cudaGraphExecDestroy(gblock);
         if (stream) {
-            for (void *p : {static_cast<void *>(dbase), static_cast<void *>(dstate),
+            for (void *p : {static_cast<void *>(dbase), static_cast<void *>(dtab), static_cast<void *>(dstate),
                             static_cast<void *>(diter), static_cast<void *>(dsnap), static_cast<void *>(dsig),
                             static_cast<void *>(dval), static_cast<void *>(dnodes), static_cast<void *>(dchildren)})
                 if (p) cudaFreeAsync(p, stream);
@@ -730,9 +843,7 @@ class Solve {
         }
         const size_t o_fro = b.add(P.fr_off), o_fri = b.add(P.fr_items), o_hc = b.add(P.hand_cards),
                      o_ef = b.add(ef), o_ena = b.add(ena), o_dn = b.add(P.depth_nodes), o_fe = b.add(P.first_edge),
-                     o_fco = b.add(P.f_coff), o_fcl = b.add(P.f_clist), o_sst = b.add(P.sd_str),
-                     o_sor = b.add(P.sd_ord), o_shp = b.add(P.sd_hpos), o_sco = b.add(P.sd_coff),
-                     o_scl = b.add(P.sd_clist);
+                     o_fco = b.add(P.f_coff), o_fcl = b.add(P.f_clist), o_sbd = b.add(P.sboards), o_fsm = b.add(P.f_same), o_bst = b.add(P.bstart);
         FCK(cudaMallocAsync(reinterpret_cast<void **>(&dbase), std::max<size_t>(b.host.size(), 256), stream));
         FCK(cudaMemcpyAsync(dbase, b.host.data(), b.host.size(), cudaMemcpyHostToDevice, stream));
         for (int p = 0; p < 2; ++p) {
@@ -744,11 +855,37 @@ class Solve {
         tab.hand_cards = hand_cards;
         tab.f_coff = reinterpret_cast<const int *>(dbase + o_fco);
         tab.f_clist = reinterpret_cast<const int *>(dbase + o_fcl);
-        tab.sd_str = reinterpret_cast<const unsigned *>(dbase + o_sst);
-        tab.sd_ord = reinterpret_cast<const int *>(dbase + o_sor);
-        tab.sd_hpos = reinterpret_cast<const int *>(dbase + o_shp);
-        tab.sd_coff = reinterpret_cast<const int *>(dbase + o_sco);
-        tab.sd_clist = reinterpret_cast<const int *>(dbase + o_scl);
+        // the showdown tables: [boards][2 players][...], made on the device
+        const size_t rows = P.sboards.size() / 5 * 2;
+        if (rows > 0) {
+            FsTableOut O{};
+            size_t at = 0;
+            auto take = [&](size_t ints) {
+                const size_t off = at;
+                at += (ints * sizeof(int) + 255) / 256 * 256;
+                return off;
+            };
+            const size_t t_str = take(rows * HS), t_ord = take(rows * HS), t_hpos = take(rows * HS * 4),
+                         t_coff = take(rows * 53), t_clist = take(rows * 2 * HS);
+            FCK(cudaMallocAsync(reinterpret_cast<void **>(&dtab), at, stream));
+            O.str = reinterpret_cast<unsigned *>(dtab + t_str);
+            O.ord = reinterpret_cast<int *>(dtab + t_ord);
+            O.hpos = reinterpret_cast<int *>(dtab + t_hpos);
+            O.coff = reinterpret_cast<int *>(dtab + t_coff);
+            O.clist = reinterpret_cast<int *>(dtab + t_clist);
+            k_fs_tables<<<static_cast<unsigned>(rows / 2), kFsThreads, 0, stream>>>(
+                reinterpret_cast<const int *>(dbase + o_sbd), hand_cards, O, P.HS, P.H[0], P.H[1]);
+            FCK(cudaGetLastError());
+            tab.sd_str = O.str;
+            tab.sd_ord = O.ord;
+            tab.sd_hpos = O.hpos;
+            tab.sd_coff = O.coff;
+            tab.sd_clist = O.clist;
+        }
+        tab.f_same = reinterpret_cast<const int *>(dbase + o_fsm);
+        tab.dup[0] = P.dup[0];
+        tab.dup[1] = P.dup[1];
+        bstart = reinterpret_cast<const int *>(dbase + o_bst);
         tab.HS = P.HS;
         tab.H0 = P.H[0];
         tab.H1 = P.H[1];
@@ -795,9 +932,19 @@ class Solve {
     }
 
     cudaError_t terms(int t, float *out, int scaled) {
-        const int nf = P.nfold[t], ns = static_cast<int>(P.term[t].size()) - nf;
-        if (nf > 0) k_fs_fold<<<nf, kFsThreads, 0, stream>>>(term_items[t], t, c.reach, tab, out, scaled);
-        if (ns > 0) k_fs_showdown<<<ns, kFsThreads, 0, stream>>>(term_items[t] + nf, t, c.reach, tab, out, scaled);
+        const int nf = P.nfold[t], boards = static_cast<int>(P.bstart.size()) - 1;
+        if (nf > 0) {
+            // eight resident blocks per SM, each over many terminals
+            const int grid = std::min((nf + kFsWarps - 1) / kFsWarps, 8 * 148);
+            k_fs_fold<<<grid, kFsThreads, 0, stream>>>(term_items[t], nf, t, c.reach, tab, out, scaled);
+        }
+        if (boards > 0) {
+            cudaError_t e = cudaFuncSetAttribute(k_fs_showdown, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(fs_sd_smem()));
+            if (e != cudaSuccess) return e;
+            k_fs_showdown<<<boards, kFsThreads, fs_sd_smem(), stream>>>(term_items[t] + nf, bstart, t, c.reach, tab, out,
+                                                                       scaled);
+        }
         return cudaGetLastError();
     }
 
