@@ -123,13 +123,54 @@ __device__ __forceinline__ void regret_match4(const float *__restrict__ R, size_
 // subgame, so the test is block-uniform (ahead of any barrier).
 __device__ __forceinline__ bool retired(const DevCtx *ctxs, int sg) { return ctxs && !ctxs[sg].live; }
 
-__global__ void __launch_bounds__(kHandThreads) k_reach(DevCtx c0, const DevCtx *__restrict__ ctxs,
-                                                        const ReachItem *__restrict__ items, int nchunk, int H,
-                                                        int p) {
+// reach rows of 4 hands at an item of at most A actions (regret_match4's
+// strategy, formed action by action)
+template <int A>
+__device__ __forceinline__ void reach_item(const float *__restrict__ R, float *__restrict__ reach, size_t HS,
+                                           const ReachItem &I, int h0) {
+    float4 r[A];
+    const float4 pr = ld4(reach + static_cast<size_t>(I.parent_row) * HS + h0);
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+        if (a < I.na) r[a] = ld4(R + static_cast<size_t>(I.first_edge + a) * HS + h0);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+        if (a < I.na) {
+            sum.x += r[a].x > 0.f ? r[a].x : 0.f;
+            sum.y += r[a].y > 0.f ? r[a].y : 0.f;
+            sum.z += r[a].z > 0.f ? r[a].z : 0.f;
+            sum.w += r[a].w > 0.f ? r[a].w : 0.f;
+        }
+    const float uni = 1.0f / static_cast<float>(I.na);
+    const float4 inv = make_float4(sum.x > 0.f ? 1.0f / sum.x : 0.f, sum.y > 0.f ? 1.0f / sum.y : 0.f,
+                                   sum.z > 0.f ? 1.0f / sum.z : 0.f, sum.w > 0.f ? 1.0f / sum.w : 0.f);
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+        if (a < I.na) {
+            auto sigma = [&](float ra, float s, float i) {
+                if (I.frozen >= 0) return a == I.frozen ? 1.0f : 0.0f;
+                return s > 0.f ? (ra > 0.f ? ra : 0.f) * i : uni;
+            };
+            st4(reach + static_cast<size_t>(I.first_edge + a) * HS + h0,
+                make_float4(pr.x * sigma(r[a].x, sum.x, inv.x), pr.y * sigma(r[a].y, sum.y, inv.y),
+                            pr.z * sigma(r[a].z, sum.z, inv.z), pr.w * sigma(r[a].w, sum.w, inv.w)));
+        }
+}
+
+// Four (item, chunk) units of 64 threads per block: a block per unit was
+// bound by block launches on trees of many items (96,432 items of 200 hands,
+// 340 MB: 146 us so, 97 us now).
+constexpr int kReachUnits = 4;
+__global__ void __launch_bounds__(kHandThreads *kReachUnits, 5) k_reach(DevCtx c0, const DevCtx *__restrict__ ctxs,
+                                                                    const ReachItem *__restrict__ items, int units,
+                                                                    int nchunk, int H, int p) {
     wait_prior_grid();
-    const int it = blockIdx.x / nchunk;
-    const int ch = blockIdx.x - it * nchunk;
-    const int h0 = (ch * kHandThreads + threadIdx.x) * 4;
+    const int unit = blockIdx.x * kReachUnits + threadIdx.x / kHandThreads;
+    if (unit >= units) return;
+    const int it = unit / nchunk;
+    const int ch = unit - it * nchunk;
+    const int h0 = (ch * kHandThreads + threadIdx.x % kHandThreads) * 4;
     const ReachItem I = items[it];
     if (retired(ctxs, I.sg)) return;
     // context fields in registers (a reference to either the parameter or a
@@ -144,28 +185,17 @@ __global__ void __launch_bounds__(kHandThreads) k_reach(DevCtx c0, const DevCtx 
     }
     if (h0 >= Hp) return;
     const size_t HS = static_cast<size_t>(HSi);
-    float r[SS_MAX_ACTIONS][4], sig[SS_MAX_ACTIONS][4];
-    regret_match4(R, HS, I.first_edge, I.na, I.frozen, h0, r, sig);
-    const float4 pr = ld4(reach + static_cast<size_t>(I.parent_row) * HS + h0);
-#pragma unroll
-    for (int a = 0; a < SS_MAX_ACTIONS; ++a) {
-        if (a < I.na) {
-            float4 o;
-            o.x = pr.x * sig[a][0];
-            o.y = pr.y * sig[a][1];
-            o.z = pr.z * sig[a][2];
-            o.w = pr.w * sig[a][3];
-            st4(reach + static_cast<size_t>(I.first_edge + a) * HS + h0, o);
-        }
-    }
+    if (I.na <= 4)
+        reach_item<4>(R, reach, HS, I, h0);
+    else
+        reach_item<SS_MAX_ACTIONS>(R, reach, HS, I, h0);
 }
 
 // --------------------------------------------------------------------------
 // cfv: value, regret and strategy-sum update at traverser nodes
 // (street_solve.cu:1155-1175): v = sum_a sigma_a ev_a; r_a = (r_a + (ev_a - v))
 // * t/(t+1); s_a += t * sigma_a; ev_a = sum of val over frontier(edge a).
-// Each lane owns 2 hands, each warp 64 consecutive hands.  S == 1: the four
-// warps of a block take four hand chunks and walk whole frontiers, eight row
+// Each thread owns 2 hands.  S == 1: it walks whole frontiers, eight row
 // loads in flight.  S > 1 (items with long frontiers, which are few): the S
 // warps of a block share one hand chunk and each sums every S-th frontier
 // row; warp 0 adds the S partial sums in a fixed order and updates.
@@ -209,22 +239,108 @@ __device__ __forceinline__ CfvHead cfv_head(const CfvItem *p) {
     return CfvHead{a.x, a.y, a.z, a.w, b.x, __int_as_float(b.y), b.z, b.w};
 }
 
+__device__ __forceinline__ void cfv_short(const CfvView &V, const CfvHead &I, const CfvItem *item,
+                                          const float *__restrict__ val, int h0, int iter_add) {
+    constexpr int kA = 4;
+    const size_t HS = static_cast<size_t>(V.HS);
+    const int4 *fp = reinterpret_cast<const int4 *>(item) + 2;
+    const int4 f0 = __ldg(fp), f1 = __ldg(fp + 1);
+    float *Rh = V.R + static_cast<size_t>(I.first_edge) * HS + h0, *Sh = V.S + static_cast<size_t>(I.first_edge) * HS + h0;
+    float2 r[kA], sm[kA], x[kCfvInline];
+#pragma unroll
+    for (int a = 0; a < kA; ++a)
+        if (a < I.na) {
+            r[a] = ld2(Rh + a * HS);
+            sm[a] = ld2(Sh + a * HS);
+        }
+    const int rows[kCfvInline] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+#pragma unroll
+    for (int i = 0; i < kCfvInline; ++i)
+        x[i] = i < I.nfr ? ld2(val + static_cast<size_t>(rows[i]) * HS) : make_float2(0.f, 0.f);
+    const int t = *V.iter + iter_add;
+    const float d = static_cast<float>(t) / (static_cast<float>(t) + 1.0f);
+    const float w = static_cast<float>(t);
+    float2 ev[kA];
+#pragma unroll
+    for (int a = 0; a < kA; ++a) ev[a] = make_float2(0.f, 0.f);
+    const unsigned bnd = static_cast<unsigned>(I.fr_bnd);
+#pragma unroll
+    for (int i = 0; i < kCfvInline; ++i)
+        if (i < I.nfr) {
+            int e = 0;   // the edge of row i: the edges whose last row (nibble) is before it
+#pragma unroll
+            for (int a = 0; a < kA - 1; ++a) e += i > static_cast<int>((bnd >> (4 * a)) & 15u) ? 1 : 0;
+#pragma unroll
+            for (int a = 0; a < kA; ++a)
+                if (e == a) add2(ev[a], x[i]);
+        }
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int a = 0; a < kA; ++a)
+        if (a < I.na) {
+            s0 += r[a].x > 0.f ? r[a].x : 0.f;
+            s1 += r[a].y > 0.f ? r[a].y : 0.f;
+        }
+    const float uni = 1.0f / static_cast<float>(I.na);
+    const float inv0 = s0 > 0.f ? 1.0f / s0 : 0.f, inv1 = s1 > 0.f ? 1.0f / s1 : 0.f;
+    auto sigma = [&](int a, float ra, float sum, float inv) {
+        if (I.frozen >= 0) return a == I.frozen ? 1.0f : 0.0f;
+        return sum > 0.f ? (ra > 0.f ? ra : 0.f) * inv : uni;
+    };
+    float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+    for (int a = 0; a < kA; ++a)
+        if (a < I.na) {
+            v0 += sigma(a, r[a].x, s0, inv0) * ev[a].x;
+            v1 += sigma(a, r[a].y, s1, inv1) * ev[a].y;
+        }
+#pragma unroll
+    for (int a = 0; a < kA; ++a)
+        if (a < I.na) {
+            float2 nr, ns;
+            nr.x = (r[a].x + (ev[a].x - v0)) * d;
+            nr.y = (r[a].y + (ev[a].y - v1)) * d;
+            ns.x = sm[a].x + w * sigma(a, r[a].x, s0, inv0);
+            ns.y = sm[a].y + w * sigma(a, r[a].y, s1, inv1);
+            st2(Rh + a * HS, nr);
+            st2(Sh + a * HS, ns);
+        }
+    st2(V.val + static_cast<size_t>(I.node) * HS + h0, make_float2(v0 * I.scale, v1 * I.scale));
+}
+
+// A S == 1 item of at most kCfvShort actions whose frontier is held in it
+// (the bulk of a tree: its lowest level) loads all it needs at once -- value,
+// regret and strategy-sum rows -- and keeps them in registers (the general
+// form reads the regrets three times through L1): 96,432 items of 200 hands
+// 345 -> 245 us with the back-to-back hand pairs.
+constexpr int kCfvShort = 4;
 template <int S>
 __global__ void __launch_bounds__(kCfvThreads, 8) k_cfv(DevCtx c0, const DevCtx *__restrict__ ctxs,
-                                                     const CfvItem *__restrict__ items, int nchunk, int Hl,
+                                                     const CfvItem *__restrict__ items, int n, int nchunk, int Hl,
                                                      int trav, int iter_add) {
     wait_prior_grid();
-    const int it = blockIdx.x / nchunk;
-    const int ch = blockIdx.x - it * nchunk;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // S == 1: nchunk hand pairs per item, one per thread, items back to back
+    // (64-hand chunks per warp left a quarter of the lanes idle at 200 hands);
+    // S > 1: a block per (item, 64 hands)
+    const int unit = S == 1 ? blockIdx.x * kCfvThreads + threadIdx.x : blockIdx.x;
+    const int it = unit / nchunk;
+    const int ch = unit - it * nchunk;
+    if (S == 1 && it >= n) return;
     const CfvHead I = cfv_head(items + it);
     if (retired(ctxs, I.sg)) return;
     const CfvView V = ctxs ? cfv_view(ctxs[I.sg], ctxs[I.sg].H[trav]) : cfv_view(c0, Hl);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = (S == 1 ? ch * (kCfvThreads / 32) + warp : ch) * 64 + lane * 2;
+    const int h0 = S == 1 ? ch * 2 : ch * 64 + lane * 2;
     const bool act = h0 < V.H;
     if (S == 1 && !act) return;
     const size_t HS = static_cast<size_t>(V.HS);
     const float *val = V.val + h0;
+    if constexpr (S == 1) {
+        if (I.nfr > 0 && I.na <= kCfvShort) {
+            cfv_short(V, I, items + it, val, h0, iter_add);
+            return;
+        }
+    }
     const int *__restrict__ fr = V.fr_items;
     // the regret and strategy-sum rows are needed after the frontier sums:
     // start bringing them into L1 now (no registers held)
@@ -3003,8 +3119,9 @@ cudaError_t read_device_fault(unsigned *code, cudaStream_t s) {
 cudaError_t launch_reach(const DevCtx &c, const ReachItem *items, int n, int H, cudaStream_t s,
                          const DevCtx *ctxs, int player) {
     if (n <= 0 || H <= 0) return cudaSuccess;
-    const int nc = chunks(H);
-    SSB_LAUNCH(k_reach, n * nc, kHandThreads, 0, s, c, ctxs, items, nc, H, player);
+    const int nc = chunks(H), units = n * nc;
+    SSB_LAUNCH(k_reach, (units + kReachUnits - 1) / kReachUnits, kHandThreads * kReachUnits, 0, s, c, ctxs, items, units,
+               nc, H, player);
     return cudaGetLastError();
 }
 
@@ -3014,13 +3131,16 @@ cudaError_t launch_cfv(const DevCtx &c, const CfvItem *items, int n, int n_long,
     n_long = n_long < 0 ? 0 : n_long > n ? n : n_long;
     const int n_short = n - n_long;
     if (n_short > 0) {
-        const int nc = (H + 2 * kCfvThreads - 1) / (2 * kCfvThreads);
-        SSB_LAUNCH(k_cfv<1>, n_short * nc, kCfvThreads, 0, s, c, ctxs, items, nc, H, trav, iter_add);
+        const int pairs = (H + 1) / 2;
+        const long long threads = static_cast<long long>(n_short) * pairs;
+        SSB_LAUNCH(k_cfv<1>, static_cast<unsigned>((threads + kCfvThreads - 1) / kCfvThreads), kCfvThreads, 0, s, c, ctxs,
+                   items, n_short, pairs, H, trav, iter_add);
     }
     if (n_long > 0) {
         const int nc = (H + 63) / 64;
         static_assert(32 * kCfvSplit == kCfvThreads, "the split form fills one block of kCfvThreads");
-        SSB_LAUNCH(k_cfv<kCfvSplit>, n_long * nc, kCfvThreads, 0, s, c, ctxs, items + n_short, nc, H, trav, iter_add);
+        SSB_LAUNCH(k_cfv<kCfvSplit>, n_long * nc, kCfvThreads, 0, s, c, ctxs, items + n_short, n_long, nc, H, trav,
+                   iter_add);
     }
     return cudaGetLastError();
 }
