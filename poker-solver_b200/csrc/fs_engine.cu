@@ -28,6 +28,7 @@
 #include "fs_engine.h"
 #include "ss_kernels.h"
 #include "ss_rank.cuh"
+#include "ss_stage.h"
 
 #include <cuda_runtime.h>
 
@@ -845,7 +846,7 @@ class Solve {
                      o_ef = b.add(ef), o_ena = b.add(ena), o_dn = b.add(P.depth_nodes), o_fe = b.add(P.first_edge),
                      o_fco = b.add(P.f_coff), o_fcl = b.add(P.f_clist), o_sbd = b.add(P.sboards), o_fsm = b.add(P.f_same), o_bst = b.add(P.bstart);
         FCK(cudaMallocAsync(reinterpret_cast<void **>(&dbase), std::max<size_t>(b.host.size(), 256), stream));
-        FCK(cudaMemcpyAsync(dbase, b.host.data(), b.host.size(), cudaMemcpyHostToDevice, stream));
+        FCK(stage_upload(dbase, b.host.data(), b.host.size(), stream));
         for (int p = 0; p < 2; ++p) {
             reach_items[p] = reinterpret_cast<const ReachItem *>(dbase + o_reach[p]);
             cfv_items[p] = reinterpret_cast<const CfvItem *>(dbase + o_cfv[p]);

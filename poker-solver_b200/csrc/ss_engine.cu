@@ -16,6 +16,7 @@
 //   * plan, tables and state stay resident in a Session, so a solve can be
 //     extended, reset or read without re-uploading.
 #include "ss_session.h"
+#include "ss_stage.h"
 
 #include <cuda_runtime.h>
 
@@ -47,6 +48,11 @@ struct Blob {
     }
 };
 
+const char *kClassName[SS_PROFILE_CLASSES] = {"reach", "cfv", "term_fill", "term_cr1",
+                                             "term_cr2", "term_sd", "term_enum", "other"};
+
+}  // namespace
+
 void keep_pool_warm(int device) {
     static std::mutex mu;
     static bool done[64] = {};
@@ -59,11 +65,6 @@ void keep_pool_warm(int device) {
     }
     done[device] = true;
 }
-
-const char *kClassName[SS_PROFILE_CLASSES] = {"reach", "cfv", "term_fill", "term_cr1",
-                                             "term_cr2", "term_sd", "term_enum", "other"};
-
-}  // namespace
 
 void set_error(const std::string &msg) { g_err = msg; }
 const char *last_error() { return g_err.c_str(); }
@@ -259,7 +260,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     dec_na_host = dna;
     dec_player_host = dpl;
     CK(cudaMallocAsync(reinterpret_cast<void **>(&dbase), std::max<size_t>(b.host.size(), 256), stream));
-    CK(cudaMemcpyAsync(dbase, b.host.data(), b.host.size(), cudaMemcpyHostToDevice, stream));
+    CK(stage_upload(dbase, b.host.data(), b.host.size(), stream));
     for (int p = 0; p < np; ++p) {
         reach_items[p] = reinterpret_cast<const ReachItem *>(dbase + o_reach[p]);
         cfv_items[p] = reinterpret_cast<const CfvItem *>(dbase + o_cfv[p]);
@@ -301,7 +302,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     if (pb.leaf_values && pb.num_leaves > 0) {
         const size_t n = static_cast<size_t>(pb.num_leaves) * np * P.max_h;
         CK(cudaMallocAsync(reinterpret_cast<void **>(&dleaf), n * sizeof(float), stream));
-        CK(cudaMemcpyAsync(dleaf, pb.leaf_values, n * sizeof(float), cudaMemcpyHostToDevice, stream));
+        CK(stage_upload(dleaf, pb.leaf_values, n * sizeof(float), stream));
     }
     n_rs = static_cast<size_t>(P.root_na) * P.H[P.root_player];
     CK(cudaMallocAsync(reinterpret_cast<void **>(&dsmall), (n_rs + HS) * sizeof(float), stream));
@@ -567,7 +568,7 @@ int Session::exploitability(const float *host_avg, double *pct, double *nash, do
     const int np = P.np;
     const size_t n_avg = static_cast<size_t>(P.num_dec) * SS_MAX_ACTIONS * P.max_h;
     if (host_avg)
-        CK(cudaMemcpyAsync(davg_br, host_avg, n_avg * sizeof(float), cudaMemcpyHostToDevice, stream));
+        CK(stage_upload(davg_br, host_avg, n_avg * sizeof(float), stream));
     else
         CK(launch_avg_strategy(c, dec_fe, dec_na, dec_pl, P.num_dec, P.max_h, davg_br, stream));
     for (int p = 0; p < np; ++p)

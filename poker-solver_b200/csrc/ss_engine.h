@@ -34,6 +34,10 @@ const char *last_error();
 void *host_block_take(size_t bytes);
 bool host_block_give(void *p);
 
+// the device's stream-ordered memory pool keeps freed blocks (up to 8 GiB)
+// for the next call (ss_engine.cu)
+void keep_pool_warm(int device);
+
 // ---------------------------------------------------------------------------
 // tree builder (ss_tree.cpp)
 // ---------------------------------------------------------------------------

@@ -19,6 +19,7 @@
 #include "ss_engine.h"
 #include "ss_leaf.cuh"
 #include "ss_leaf.h"
+#include "ss_stage.h"
 
 #include <cuda_runtime.h>
 
@@ -121,13 +122,15 @@ int leaf_values_gpu(const SSLeafValueInput *in, float *out) {
 
     unsigned char *base = nullptr;
     cudaStream_t stream = nullptr;
-    cudaError_t e = cudaMalloc(&base, top);
+    keep_pool_warm(dev);
+    cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&base), top, stream);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
+        if (stream) cudaStreamDestroy(stream);
         set_error("ss_leaf_values_gpu: device allocation of " + std::to_string(top) + " bytes failed");
         return SS_ERR_NOMEM;
     }
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         for (const Part *p : {&p_nh, &p_cards, &p_board, &p_off, &p_owner, &p_thand, &p_pot, &p_set})
             if (e == cudaSuccess && p->bytes > 0)
@@ -166,17 +169,15 @@ int leaf_values_gpu(const SSLeafValueInput *in, float *out) {
             k_leaf_value<<<blocks_for(n, sms), kThreads, 0, stream>>>(c, static_cast<long>(row0), n);
             e = cudaGetLastError();
             if (e == cudaSuccess)
-                e = cudaMemcpyAsync(out + row0 * per_row, c.values, nrows * per_row * sizeof(float),
-                                    cudaMemcpyDeviceToHost, stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+                e = stage_download(out + row0 * per_row, c.values, nrows * per_row * sizeof(float), stream);
         }
     }
+    if (base) cudaFreeAsync(base, stream);
     if (stream) {
         const cudaError_t s = cudaStreamSynchronize(stream);
         if (e == cudaSuccess) e = s;
         cudaStreamDestroy(stream);
     }
-    if (base) cudaFree(base);
     if (e != cudaSuccess) {
         set_error(std::string("ss_leaf_values_gpu: CUDA: ") + cudaGetErrorString(e));
         return SS_ERR_CUDA;

@@ -183,8 +183,8 @@ def _produce(board, runouts, leaf_infos, max_hands, player_hands):
         raise ValueError(f"a range holds {int(nh.max())} hands, more than max_hands = {max_hands}")
     cards = np.zeros((N, max(max_hands, 1), 2), dtype=np.int32)
     for p, hands in enumerate(player_hands):
-        for h, hand in enumerate(hands):
-            cards[p, h, 0], cards[p, h, 1] = int(hand[0]), int(hand[1])
+        if len(hands):
+            cards[p, :len(hands)] = [(int(hand[0]), int(hand[1])) for hand in hands]
     board_a = np.ascontiguousarray([int(c) for c in board], dtype=np.int32)
     extra = 5 - len(board_a)
     run_a = np.ascontiguousarray(np.array(runouts, dtype=np.int32).reshape(-1, extra))
