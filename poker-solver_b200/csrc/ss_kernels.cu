@@ -2401,10 +2401,11 @@ __global__ void __launch_bounds__(32 * kEnumWarps) k_term_enum(DevCtx c0, const 
 // tables of a 48-card deck (105 KB) leave two blocks per SM (512 and 576
 // threads spill: 1.4x slower).  Measured on the 4-player turn (5,681 nodes,
 // 2,696 terminals): 8.4 ms per launch by conditioning, 0.5 ms in the first
-// iterations, 1.06 ms where play has become near pure and many hands need the
-// exact look.
+// iterations, 0.9 ms where play has become near pure and many hands need the
+// exact look; at 32 hands, where the tables are the work, 0.18 ms by
+// conditioning and 0.146 ms (0.22 before sparse products and split hands).
 constexpr int kCr3Threads = 384;
-constexpr int kCr3Rounds = (kMaxHS + kCr3Threads - 1) / kCr3Threads;
+static_assert(kMaxHS <= 14 * (kCr3Threads / 4), "a thread's rounds fit a mask");
 // blocks a launch is brought to by sharing a group's hands between blocks (each
 // builds the tables): two per SM
 constexpr int kCr3Blocks = 2 * 148;
@@ -2428,7 +2429,7 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
     const DevCtx &c = ctxs ? ctxs[I0->sg] : c0;
     const int HS = c.HS, Ht = c.H[trav], n = c.deck;
     // shared memory was provisioned for c0's deck (the largest of a batch)
-    if (HS > kMaxHS || n > c0.deck || ch * kCr3Threads >= HS) return;
+    if (HS > kMaxHS || n > c0.deck || (ch > 0 && ch * kCr3Threads >= HS)) return;
     const int tid = threadIdx.x;
     Carve cv{smem};
     const tri::Tables t = tri::tables(cv.take<double>(tri::doubles(n)), n);
@@ -2479,17 +2480,28 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
                 h < Ht ? static_cast<T>(static_cast<double>(term_factor(c, Ig, h)) * m) : T(0);
         }
     };
+    // lanes per hand: a range too small for the block's threads splits each
+    // hand's sum over the deck
+    const int lanes = Ht * 4 <= kCr3Threads ? 4 : Ht * 2 <= kCr3Threads ? 2 : 1;
+    const int per = kCr3Threads / lanes, mine = tid / lanes, part = tid % lanes;   // hands per round
+    const int first = ch * per, step = nchunk * per;
     unsigned near = 0;   // this thread's hands (by round) within rounding of 0
+    int round = 0;
 #pragma unroll 1
-    for (int r = ch; r < kCr3Rounds; r += nchunk) {
-        const int h = r * kCr3Threads + tid;
-        if (h >= HS) break;
-        double m = 0.0;
-        if (h < Ht && !none) {
-            const int hc = __ldg(code_t + h);
-            m = tri::hand_mass(dense(hc, 20), dense(hc, 26), t);
-            if (fabs(m) <= zb) near |= 1u << r;
+    for (int h0 = first; h0 < HS; h0 += step, ++round) {
+        const int h = h0 + mine;
+        const bool live = h < Ht && !none;
+        const int hc = live ? __ldg(code_t + h) : 0, a = dense(hc, 20), b = dense(hc, 26);
+        tri::Part p{0.0, 0.0, 0.0};
+        if (live) p = tri::hand_part(a, b, t, part, lanes);
+        for (int k = 1; k < lanes; k <<= 1) {
+            p.acc += __shfl_xor_sync(0xffffffffu, p.acc, k);
+            p.ACab += __shfl_xor_sync(0xffffffffu, p.ACab, k);
+            p.ACba += __shfl_xor_sync(0xffffffffu, p.ACba, k);
         }
+        if (part != 0 || h >= HS) continue;
+        const double m = live ? tri::hand_finish(a, b, t, p) : 0.0;
+        if (live && fabs(m) <= zb) near |= 1u << round;
         write(h, m);
     }
     if (!__syncthreads_or(near != 0)) return;
@@ -2501,8 +2513,8 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
     if (tid == 0) *n_near = 0;
     tri::phase_masks(tid, kCr3Threads, t, k);
     __syncthreads();
-    for (int r = ch; r < kCr3Rounds; r += nchunk)
-        if (near >> r & 1u) list[atomicAdd(n_near, 1)] = static_cast<unsigned short>(r * kCr3Threads + tid);
+    for (int r = 0; near >> r; ++r)
+        if (near >> r & 1u) list[atomicAdd(n_near, 1)] = static_cast<unsigned short>(first + r * step + mine);
     tri::phase_counts(tid, kCr3Threads, t, k);
     __syncthreads();
     const int lane = tid & 31;

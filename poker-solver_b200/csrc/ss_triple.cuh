@@ -47,11 +47,12 @@ struct Tables {
     double *A, *B, *C, *AB, *CB;   // [S][S]
     double *v;                     // [N_VEC][kVS]
     double *sc;                    // [N_SCAL]
+    unsigned long long *m;         // [3][kVS]: nonzero cells of each row of A, B, C
     int n, S;
 };
 
 SSB_TRI_HD constexpr int stride(int n) { return (n + 1) | 1; }
-SSB_TRI_HD constexpr int doubles(int n) { return 5 * stride(n) * stride(n) + N_VEC * kVS + N_SCAL + 1; }
+SSB_TRI_HD constexpr int doubles(int n) { return 5 * stride(n) * stride(n) + N_VEC * kVS + N_SCAL + 1 + 3 * kVS; }
 
 SSB_TRI_HD Tables tables(double *mem, int n) {
     Tables t;
@@ -65,29 +66,59 @@ SSB_TRI_HD Tables tables(double *mem, int n) {
     t.CB = mem + 4 * m;
     t.v = mem + 5 * m;
     t.sc = t.v + N_VEC * kVS;
+    t.m = reinterpret_cast<unsigned long long *>(t.sc + N_SCAL + 1);
     return t;
 }
 
 // phase 1: the matrices from the opponents' pair tables ([52][52] dense pair
-// -> range index, HS if none); the dummy row and column are zero.  With
-// code3 (a third range that repeats a combo) C is left to phase_gather_third.
+// -> range index, HS if none); the dummy row and column are zero.  Without
+// `third` (a third range that repeats a combo) C is left to
+// phase_gather_third.  On the device a warp fills whole rows and takes the
+// row's nonzero cells from ballots; on the host one item is a row.
+template <class T>
+SSB_TRI_HD void cell(const Tables &t, int x, int y, const T *r1, const T *r2, const T *r3, const int *pair1,
+                     const int *pair2, const int *pair3, int HS, bool third, double v[3]) {
+    v[0] = v[1] = v[2] = 0.0;
+    if (x < t.n && y < t.n) {
+        const int j1 = pair1[x * 52 + y], j2 = pair2[x * 52 + y], j3 = third ? pair3[x * 52 + y] : HS;
+        if (j1 < HS) v[0] = static_cast<double>(r1[j1]);
+        if (j2 < HS) v[1] = static_cast<double>(r2[j2]);
+        if (j3 < HS && r3[j3] > T(0)) v[2] = static_cast<double>(r3[j3]);
+    }
+    if (y <= t.n) {
+        t.A[x * t.S + y] = v[0];
+        t.B[x * t.S + y] = v[1];
+        t.C[x * t.S + y] = v[2];
+    }
+}
 template <class T>
 SSB_TRI_HD void phase_gather(int tid, int nt, const Tables &t, const T *r1, const T *r2, const T *r3,
                              const int *pair1, const int *pair2, const int *pair3, int HS, bool third) {
-    const int m = t.n + 1;
-    for (int i = tid; i < m * m; i += nt) {
-        const int x = i / m, y = i - x * m, at = x * t.S + y;
-        double a = 0.0, b = 0.0, c = 0.0;
-        if (x < t.n && y < t.n) {
-            const int j1 = pair1[x * 52 + y], j2 = pair2[x * 52 + y], j3 = third ? pair3[x * 52 + y] : HS;
-            if (j1 < HS) a = static_cast<double>(r1[j1]);
-            if (j2 < HS) b = static_cast<double>(r2[j2]);
-            if (j3 < HS && r3[j3] > T(0)) c = static_cast<double>(r3[j3]);
+#if defined(__CUDA_ARCH__)
+    const int lane = tid & 31;
+#pragma unroll 2
+    for (int x = tid >> 5; x <= t.n; x += nt >> 5) {
+        unsigned long long m[3] = {0ull, 0ull, 0ull};
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            double v[3];
+            cell(t, x, half * 32 + lane, r1, r2, r3, pair1, pair2, pair3, HS, third, v);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                m[i] |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, v[i] != 0.0)) << (32 * half);
         }
-        t.A[at] = a;
-        t.B[at] = b;
-        t.C[at] = c;
+        if (lane < 3) t.m[lane * kVS + x] = lane == 0 ? m[0] : lane == 1 ? m[1] : m[2];
     }
+#else
+    for (int x = tid; x <= t.n; x += nt) {
+        for (int i = 0; i < 3; ++i) t.m[i * kVS + x] = 0ull;
+        for (int y = 0; y <= t.n; ++y) {
+            double v[3];
+            cell(t, x, y, r1, r2, r3, pair1, pair2, pair3, HS, third, v);
+            for (int i = 0; i < 3; ++i) t.m[i * kVS + x] |= static_cast<unsigned long long>(v[i] != 0.0) << y;
+        }
+    }
+#endif
 }
 
 // phase 1 continued, for a third range that repeats a combo: its hands add up
@@ -99,48 +130,80 @@ SSB_TRI_HD void phase_gather_third(int tid, int nt, const Tables &t, const T *r3
             const int code = code3[h];
             if ((code & 0x10000) || !(r3[h] > T(0))) continue;   // touches the board, or nothing to add
             const int p = (code >> 20) & 63, q = (code >> 26) & 63;
-            if (p == x) t.C[x * t.S + q] += static_cast<double>(r3[h]);
-            if (q == x) t.C[x * t.S + p] += static_cast<double>(r3[h]);
+            if (p != x && q != x) continue;
+            const int o = p == x ? q : p;
+            t.C[x * t.S + o] += static_cast<double>(r3[h]);
+            t.m[2 * kVS + x] |= 1ull << o;
         }
 }
 
-// phase 2: row sums, and AB = A B, CB = C B in 3 x 3 cells per item (A and C
-// are symmetric: row k is column k), each cell summed over k in order
-SSB_TRI_HD void phase_products(int tid, int nt, const Tables &t) {
-    const int n = t.n, S = t.S, nt3 = (n + 2) / 3;
-    for (int i = tid; i < 3 * n; i += nt) {
-        const int c = i % n;
-        const double *M = (i < n ? t.A : i < 2 * n ? t.B : t.C) + c * S;
-        double u = 0.0;
-        for (int x = 0; x < n; ++x) u += M[x];
-        t.v[(i < n ? UA : i < 2 * n ? UB : UC) * kVS + c] = u;
+// sum of f(0) .. f(n - 1) in four interleaved partial sums (a chain of n
+// dependent FP64 additions is the latency of a phase)
+template <class F>
+SSB_TRI_HD double sum4(int n, F f) {
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    int x = 0;
+#pragma unroll 2
+    for (; x + 3 < n; x += 4) {
+        s0 += f(x);
+        s1 += f(x + 1);
+        s2 += f(x + 2);
+        s3 += f(x + 3);
     }
-    for (int i = tid; i < N_VEC; i += nt) t.v[i * kVS + n] = 0.0;
-    for (int i = tid; i <= n; i += nt) t.AB[n * S + i] = t.AB[i * S + n] = t.CB[n * S + i] = t.CB[i * S + n] = 0.0;
-    for (int q = tid; q < 2 * nt3 * nt3; q += nt) {
-        const bool second = q >= nt3 * nt3;
-        const int r = second ? q - nt3 * nt3 : q;
+    for (; x < n; ++x) s0 += f(x);
+    return (s0 + s1) + (s2 + s3);
+}
+
+SSB_TRI_HD int low_bit(unsigned long long m) {
+#if defined(__CUDA_ARCH__)
+    return __ffsll(static_cast<long long>(m)) - 1;
+#else
+    return __builtin_ctzll(m);
+#endif
+}
+
+// phase 2: row sums, and AB = A B, CB = C B in 4 x 4 cells per item (A and C
+// are symmetric: row k is column k), each cell summed over k in order, without
+// the k whose cells are all zero in one operand's tile (sparse ranges)
+SSB_TRI_HD void phase_products(int tid, int nt, const Tables &t) {
+    const int n = t.n, S = t.S, nt4 = (n + 3) / 4;
+    for (int q = tid; q < 2 * nt4 * nt4; q += nt) {
+        const bool second = q >= nt4 * nt4;
+        const int r = second ? q - nt4 * nt4 : q;
         const double *M = second ? t.C : t.A;
+        const unsigned long long *mM = t.m + (second ? 2 : 0) * kVS, *mB = t.m + kVS;
         double *P = second ? t.CB : t.AB;
-        int ii[3], jj[3];
-        for (int i = 0; i < 3; ++i) {   // past the deck: the dummy's zeros
-            ii[i] = r / nt3 * 3 + i < n ? r / nt3 * 3 + i : n;
-            jj[i] = r % nt3 * 3 + i < n ? r % nt3 * 3 + i : n;
+        int ii[4], jj[4];
+        unsigned long long rows = 0ull, cols = 0ull;
+        for (int i = 0; i < 4; ++i) {   // past the deck: the dummy's zeros
+            ii[i] = r / nt4 * 4 + i < n ? r / nt4 * 4 + i : n;
+            jj[i] = r % nt4 * 4 + i < n ? r % nt4 * 4 + i : n;
+            rows |= mM[ii[i]];
+            cols |= mB[jj[i]];
         }
-        double acc[3][3] = {};
-        for (int k = 0; k < n; ++k) {
-            double x[3], y[3];
-            for (int i = 0; i < 3; ++i) {
+        double acc[4][4] = {};
+        for (unsigned long long m = rows & cols; m; m &= m - 1) {
+            const int k = low_bit(m);
+            double x[4], y[4];
+            for (int i = 0; i < 4; ++i) {
                 x[i] = M[k * S + ii[i]];
                 y[i] = t.B[k * S + jj[i]];
             }
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) acc[i][j] += x[i] * y[j];
+            for (int i = 0; i < 4; ++i)
+                for (int j = 0; j < 4; ++j) acc[i][j] += x[i] * y[j];
         }
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j)
+        for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j)
                 if (ii[i] < n && jj[j] < n) P[ii[i] * S + jj[j]] = acc[i][j];
     }
+    // the row sums, on the threads that had the fewest tiles
+    for (int i = nt - 1 - tid; i < 3 * n; i += nt) {
+        const int c = i % n;
+        const double *M = (i < n ? t.A : i < 2 * n ? t.B : t.C) + c * S;
+        t.v[(i < n ? UA : i < 2 * n ? UB : UC) * kVS + c] = sum4(n, [&](int x) { return M[x]; });
+    }
+    for (int i = tid; i < N_VEC; i += nt) t.v[i * kVS + n] = 0.0;
+    for (int i = tid; i <= n; i += nt) t.AB[n * S + i] = t.AB[i * S + n] = t.CB[n * S + i] = t.CB[i * S + n] = 0.0;
 }
 
 // phase 3: the other per-card vectors, one item per (vector, card)
@@ -151,27 +214,20 @@ SSB_TRI_HD void phase_vectors(int tid, int nt, const Tables &t) {
         if (g < 6) {
             const double *M = (g == 0 || g == 2 ? t.A : g == 1 || g == 4 ? t.B : t.C) + c * S;
             const double *u = t.v + (g == 0 || g == 5 ? UB : g == 1 || g == 3 ? UA : UC) * kVS;
-            double s = 0.0;
-            for (int x = 0; x < n; ++x) s += M[x] * u[x];
-            t.v[(AUB + g) * kVS + c] = s;
+            t.v[(AUB + g) * kVS + c] = sum4(n, [&](int x) { return M[x] * u[x]; });
         } else if (g == 6) {
-            double dac = 0.0, h = 0.0;
-            for (int x = 0; x < n; ++x) {
-                const double ac = t.A[c * S + x] * t.C[c * S + x];
-                dac += ac;
-                h += ac * t.B[c * S + x];
-            }
-            t.v[DAC * kVS + c] = dac;
-            t.v[HH * kVS + c] = h;
+            const double *a = t.A + c * S, *b = t.B + c * S, *d = t.C + c * S;
+            t.v[DAC * kVS + c] = sum4(n, [&](int x) { return a[x] * d[x]; });
+            t.v[HH * kVS + c] = sum4(n, [&](int x) { return a[x] * b[x] * d[x]; });
             t.v[DAB * kVS + c] = t.AB[c * S + c];
             t.v[DBC * kVS + c] = t.CB[c * S + c];
         } else {
             // (A B C), (C A B) and (A C B) at [c][c]
             const double *M = (g == 9 ? t.A : t.C) + c * S;
             const double *P = g == 9 ? t.CB : t.AB;
-            double s = 0.0;
-            for (int x = 0; x < n; ++x) s += M[x] * P[g == 7 ? c * S + x : x * S + c];
-            t.v[(g == 7 ? TABC : g == 8 ? TCAB : TACB) * kVS + c] = s;
+            const int at = g == 7 ? c * S : c, step = g == 7 ? 1 : S;
+            t.v[(g == 7 ? TABC : g == 8 ? TCAB : TACB) * kVS + c] =
+                sum4(n, [&](int x) { return M[x] * P[at + x * step]; });
         }
     }
 }
@@ -181,24 +237,27 @@ SSB_TRI_HD void phase_scalars(int tid, int nt, const Tables &t) {
     for (int k = tid; k < N_SCAL; k += nt) {
         const int p = k == QAB || k == QAC ? UA : k == QBC ? UB : -1, q = k == QAB ? UB : UC;
         const int one = k < 3 ? UA + k : k >= EAB && k <= EBC ? DAB + (k - EAB) : k == SH ? HH : TABC;
-        double s = 0.0;
-        for (int c = 0; c < t.n; ++c)
-            s += p >= 0 ? t.v[p * kVS + c] * t.v[q * kVS + c] : t.v[one * kVS + c];
+        const double s = p >= 0 ? sum4(t.n, [&](int c) { return t.v[p * kVS + c] * t.v[q * kVS + c]; })
+                                : sum4(t.n, [&](int c) { return t.v[one * kVS + c]; });
         t.sc[k] = k < 3 || (k >= EAB && k <= EBC) ? 0.5 * s : s;
     }
 }
 
-// the mass of one traverser hand with dense cards (a, b)
-SSB_TRI_HD double hand_mass(int a, int b, const Tables &t) {
+// The mass of one traverser hand with dense cards (a, b): the sums over the
+// deck's cards x0, x0 + step, ... (few hands: several lanes per hand), then the
+// rest from their totals.
+struct Part {
+    double acc, ACab, ACba;   // AC = A C at [a][b] and [b][a]
+};
+SSB_TRI_HD Part hand_part(int a, int b, const Tables &t, int x0, int step) {
     const int S = t.S;
-    const double *v = t.v, *sc = t.sc;
-    const double Aab = t.A[a * S + b], Bab = t.B[a * S + b], Cab = t.C[a * S + b];
+    const double *v = t.v;
+    const double Aab = t.A[a * S + b], Bab = t.B[a * S + b];
     const double Aa = v[UA * kVS + a] - Aab, Ab = v[UA * kVS + b] - Aab;
     const double Ba = v[UB * kVS + a] - Bab, Bb = v[UB * kVS + b] - Bab;
-    const double Ca = v[UC * kVS + a] - Cab, Cb = v[UC * kVS + b] - Cab;
-    double acc = 0.0, ACab = 0.0, ACba = 0.0;   // AC = A C at [a][b] and [b][a]
+    double acc = 0.0, ACab = 0.0, ACba = 0.0;
 #pragma unroll 2
-    for (int x = 0; x < t.n; ++x) {
+    for (int x = x0; x < t.n; x += step) {
         const double Xa = t.A[x * S + a], Xb = t.A[x * S + b];
         const double Ya = t.B[x * S + a], Yb = t.B[x * S + b];
         const double Za = t.C[x * S + a], Zb = t.C[x * S + b];
@@ -217,6 +276,16 @@ SSB_TRI_HD double hand_mass(int a, int b, const Tables &t) {
         const double dab = v[DAB * kVS + x] - Xa * Ya - Xb * Yb;
         acc += al * (2.0 * (be * ga - dbc) + cb) + ga * (ba - 2.0 * dab) - 2.0 * (be * dac);
     }
+    return Part{acc, ACab, ACba};
+}
+SSB_TRI_HD double hand_finish(int a, int b, const Tables &t, const Part &part) {
+    const int S = t.S;
+    const double *v = t.v, *sc = t.sc;
+    const double acc = part.acc, ACab = part.ACab, ACba = part.ACba;
+    const double Aab = t.A[a * S + b], Bab = t.B[a * S + b], Cab = t.C[a * S + b];
+    const double Aa = v[UA * kVS + a] - Aab, Ab = v[UA * kVS + b] - Aab;
+    const double Ba = v[UB * kVS + a] - Bab, Bb = v[UB * kVS + b] - Bab;
+    const double Ca = v[UC * kVS + a] - Cab, Cb = v[UC * kVS + b] - Cab;
     const double ABs = t.AB[a * S + b] + t.AB[b * S + a], CBab = t.CB[a * S + b], CBba = t.CB[b * S + a];
     auto at2 = [&](int k) { return v[k * kVS + a] + v[k * kVS + b]; };
     const double fa = sc[FA] - at2(UA) + Aab, fb = sc[FB] - at2(UB) + Bab, fc = sc[FC] - at2(UC) + Cab;
@@ -230,6 +299,8 @@ SSB_TRI_HD double hand_mass(int a, int b, const Tables &t) {
     const double tr = sc[TR] - at2(TABC) - at2(TCAB) + ABs * Cab - at2(TACB) + Aab * (CBab + CBba) + Bab * (ACab + ACba);
     return fa * fb * fc + fc * (eab - qab) + fb * (eac - qac) + fa * (ebc - qbc) + acc + 2.0 * h - tr;
 }
+
+SSB_TRI_HD double hand_mass(int a, int b, const Tables &t) { return hand_finish(a, b, t, hand_part(a, b, t, 0, 1)); }
 
 // A computed mass at or below this may be an empty set of tuples (every term
 // is at most a few F_A F_B F_C, its rounding far below the factor here)
