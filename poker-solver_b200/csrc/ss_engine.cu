@@ -198,7 +198,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     Blob b;
     size_t o_heads[SS_MAX_PLAYERS][TK_COUNT] = {};
     size_t o_reach[SS_MAX_PLAYERS], o_cfv[SS_MAX_PLAYERS], o_term[SS_MAX_PLAYERS][TK_COUNT],
-        o_rootfr[SS_MAX_PLAYERS], o_tree[SS_MAX_PLAYERS];
+        o_rootfr[SS_MAX_PLAYERS], o_tree[SS_MAX_PLAYERS], o_whole[2] = {};
     for (int p = 0; p < np; ++p) {
         std::vector<ReachItem> all;
         for (auto &lv : P.reach_levels[p]) {
@@ -235,6 +235,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
         }
         o_rootfr[p] = b.add(P.root_fr[p]);
         o_tree[p] = b.add(P.tree[p].blob);
+        if (p < 2) o_whole[p] = b.add(P.whole[p].blob);
     }
     const size_t o_fr_off = b.add(P.fr_off);
     const size_t o_fr_items = b.add(P.fr_items);
@@ -273,6 +274,19 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
         const TreePass &T = P.tree[p];
         tree[p] = TreeRef{dbase + o_tree[p], static_cast<int>(T.blob.size()), T.o_items, T.o_chains, T.o_reach,
                           T.o_rows, static_cast<int>(T.stages.size()), T.max_chains, T.threads};
+        if (p < 2) {
+            const WholePass &W = P.whole[p];
+            small.tree[p] = WholeRef{dbase + o_whole[p], static_cast<int>(W.blob.size()), W.o_reach, W.o_end, W.o_edge,
+                                     W.o_rows, W.o_voff, W.o_roff, static_cast<int>(W.edge_row.size()),
+                                     static_cast<int>(W.rows.size()), static_cast<int>(W.value_off.size()) - 1,
+                                     static_cast<int>(W.reach_off.size()) - 1};
+            small.sd1[p] = term_items[p][TK_SD1];
+            small.cr1[p] = term_items[p][TK_CR1];
+            small.zero[p] = term_items[p][TK_ZERO];
+            small.n_sd1[p] = static_cast<int>(P.term[p][TK_SD1].size());
+            small.n_cr1[p] = static_cast<int>(P.term[p][TK_CR1].size());
+            small.n_zero[p] = static_cast<int>(P.term[p][TK_ZERO].size());
+        }
     }
     dec_fe = reinterpret_cast<const int *>(dbase + o_dfe);
     dec_na = reinterpret_cast<const int *>(dbase + o_dna);
@@ -288,7 +302,8 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     nVal = N * HS;
     CK(cudaMallocAsync(reinterpret_cast<void **>(&dstate), (2 * nR + nReach + nVal) * sizeof(float), stream));
     CK(cudaMemsetAsync(dstate, 0, (2 * nR + nReach + nVal) * sizeof(float), stream));
-    CK(cudaMallocAsync(reinterpret_cast<void **>(&diter), sizeof(int), stream));
+    CK(cudaMallocAsync(reinterpret_cast<void **>(&diter), 2 * sizeof(int), stream));   // iteration, grid barrier
+    small.barrier = reinterpret_cast<unsigned *>(diter + 1);
     float *R = dstate, *S = R + nR, *reach = S + nR, *val = reach + nReach;
     {
         std::vector<float> w(static_cast<size_t>(np) * HS, 0.f);
@@ -343,6 +358,8 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     c.root_na = P.root_na;
     c.root_frozen = frozen_root;
     c.root_player = P.root_player;
+    if (!cfg.batch_member && !P.whole[0].items.empty() && !P.whole[1].items.empty())
+        small_blocks = small_solve_blocks(c, &small);
     return reset();
 }
 
@@ -357,6 +374,10 @@ int Session::reset() {
     return SS_OK;
 }
 
+// iterations per cooperative launch of a small subgame: a launch holds its SMs
+// until it ends (a few milliseconds), so other streams get their turn between
+constexpr int kSmallIters = 128;
+
 int Session::run(int iters) {
     if (iters < 0) {
         set_error("iterations must be >= 0");
@@ -369,6 +390,15 @@ int Session::run(int iters) {
         return SS_ERR_UNSUPPORTED;
     }
     CK(cudaSetDevice(device));
+    if (small_blocks > 0) {
+        for (int done = 0; done < iters;) {
+            const int n = std::min(kSmallIters, iters - done);
+            done += n;
+            CK(launch_small_solve(c, small, small_blocks, n, done == iters, stream));
+        }
+        iterations += iters;
+        return SS_OK;
+    }
     const int rest = iters - 1;
     const int qA = rest / graph_iters, rC = rest % graph_iters;
     if (qA > 0 && !gA) CK(capture(graph_iters, false, &gA));
@@ -427,7 +457,7 @@ int Session::output(SSOutput *out) {
             set_error(std::string("CUDA: ") + cudaGetErrorString(e));
         else
             set_error("a kernel recorded a device fault (code " + std::to_string(fault) +
-                      "): the tensor-core product's completion wait ran out or it got a subgame it does not serve");
+                      "): a bounded wait in it ran out or it got a subgame it does not serve");
         return SS_ERR_CUDA;
     }
     for (int i = 0; i < P.num_dec; ++i) h_ids[i] = P.dec_nodes[i];

@@ -181,6 +181,40 @@ void build_tree_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const 
                      const std::vector<std::vector<ReachItem>> &reach_levels, const std::vector<int> &fr_off,
                      const std::vector<int> &fr_items, TreePass *out);
 
+// One player's whole tree for k_small_solve, whose blocks keep 8 hands' regret,
+// strategy-sum, reach and value rows in shared memory: the player's edges are
+// numbered locally (edge0 + action), and the frontier rows of all its edges
+// form one list, item by item and edge by edge; an edge's rows end at
+// edge_end.  A row is the node of a terminal, or -1 where it is one of the
+// player's own decisions (WholeItem.row of that decision).
+struct alignas(16) WholeItem {
+    int first_edge;   // the node's first edge in the subgame
+    int node;
+    short edge0, na, frozen, split;   // split: chains per edge (1 or kCfvSplit), as TreeItem
+    short row0, row;  // its first frontier row; where its own value goes (-1: the top)
+    float scale;
+    float uniform;    // 1 / na
+};
+struct alignas(16) WholeReach {
+    short edge0, na, parent, frozen;   // parent: local edge, -1: the range weights
+    float uniform;
+    int first_edge;
+};
+struct WholePass {
+    std::vector<WholeItem> items;      // by value level, bottom-up
+    std::vector<WholeReach> reach;     // by reach level, top-down
+    std::vector<short> edge_end;       // [edges]
+    std::vector<int> edge_row;         // [edges] the edge's row in the subgame (first_edge + action of its node)
+    std::vector<int> rows;
+    std::vector<int> value_off, reach_off;   // level boundaries
+    std::vector<char> blob;
+    int o_reach = 0, o_end = 0, o_edge = 0, o_rows = 0, o_voff = 0, o_roff = 0;
+};
+// Empty when the tree's numbers do not fit the tables' 16 bits.
+void build_whole_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const std::vector<int> &cfv_nlong,
+                      const std::vector<std::vector<ReachItem>> &reach_levels, const std::vector<int> &fr_off,
+                      const std::vector<int> &fr_items, int num_edges, WholePass *out);
+
 // A three-way showdown's rank-order sweep is cut into at most this many runs
 // of tie groups, each swept by its own block from a directly computed state.
 constexpr int kSd2Chunks = 16;
@@ -293,6 +327,7 @@ struct Plan {
     std::vector<std::vector<CfvItem>> cfv_levels[SS_MAX_PLAYERS];
     std::vector<int> cfv_nlong[SS_MAX_PLAYERS];
     TreePass tree[SS_MAX_PLAYERS];     // the small levels of both, in one launch per traverser
+    WholePass whole[2];                // small heads-up subgames (k_small_solve); no items otherwise
     // two-opponent terminals (TK_CR2): the items that start work (group leaders
     // that no chain head computes); the launch gets one block each.  (One block
     // per item, as for every other kind, keeps the one-opponent launches

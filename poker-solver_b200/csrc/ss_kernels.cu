@@ -114,6 +114,19 @@ __device__ __forceinline__ void regret_match4(const float *__restrict__ R, size_
     }
 }
 
+// regret-matched (and frozen) strategy of one node, out[na][H]
+// (street_solve.cu:1564-1573), by nt threads
+__device__ __forceinline__ void root_strategy(const float *__restrict__ R, size_t HS, int fe, int na, int frozen, int H,
+                                              float *out, int tid, int nt) {
+    for (int h0 = tid * 4; h0 < H; h0 += nt * 4) {
+        float r[SS_MAX_ACTIONS][4], sig[SS_MAX_ACTIONS][4];
+        regret_match4(R, HS, fe, na, frozen, h0, r, sig);
+        for (int a = 0; a < na; ++a)
+            for (int i = 0; i < 4; ++i)
+                if (h0 + i < H) out[static_cast<size_t>(a) * H + h0 + i] = sig[a][i];
+    }
+}
+
 // --------------------------------------------------------------------------
 // reach: reach[first_edge + a] = reach[parent_row] * sigma_a
 // (street_solve.cu:650-683, stored per sequence instead of per node)
@@ -524,19 +537,11 @@ __global__ void __launch_bounds__(kCfvThreads, 8) k_cfv(DevCtx c0, const DevCtx 
 // --------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-template <bool kResident>
-__global__ void __launch_bounds__(kTreeThreads, 1) k_tree(DevCtx c, TreeRef T, int H, int iter_add) {
-    extern __shared__ __align__(16) char smem[];
-    float *part = reinterpret_cast<float *>(smem);   // [chain of the tile][kTreeHands]
-    const char *tab = T.blob;
-    if constexpr (kResident) {
-        int4 *dst = reinterpret_cast<int4 *>(smem + static_cast<size_t>(T.max_chains) * kTreeHands * sizeof(float));
-        const int4 *src = reinterpret_cast<const int4 *>(T.blob);
-        for (int i = threadIdx.x; i < T.bytes / 16; i += blockDim.x) dst[i] = __ldg(src + i);
-        tab = reinterpret_cast<const char *>(dst);
-    }
-    wait_prior_grid();
-    if constexpr (kResident) __syncthreads();
+// The stages of one pass for hands [first, first + kTreeHands); tab: its blob
+// (shared or global memory), part: the tile's partial sums in shared memory.
+// Iteration t.  Every thread of the block takes part.
+__device__ __forceinline__ void tree_pass(const DevCtx &c, const TreeRef &T, const char *tab, float *part, int first,
+                                          int H, int t) {
     const TreeStage *stages = reinterpret_cast<const TreeStage *>(tab);
     const TreeItem *items = reinterpret_cast<const TreeItem *>(tab + T.o_items);
     const int2 *chains = reinterpret_cast<const int2 *>(tab + T.o_chains);
@@ -544,12 +549,11 @@ __global__ void __launch_bounds__(kTreeThreads, 1) k_tree(DevCtx c, TreeRef T, i
     const int *rows = reinterpret_cast<const int *>(tab + T.o_rows);
     const int hand = threadIdx.x & (kTreeHands - 1), slot = threadIdx.x / kTreeHands;
     const int slots = blockDim.x / kTreeHands;
-    const int h = blockIdx.x * kTreeHands + hand;
+    const int h = first + hand;
     const bool act = h < H;
     const size_t HS = static_cast<size_t>(c.HS);
     const float *val = c.val + h;
     float *R = c.R + h, *S = c.S + h, *reach = c.reach + h;
-    const int t = *c.iter + iter_add;
     const float d = static_cast<float>(t) / (static_cast<float>(t) + 1.0f);
     const float w = static_cast<float>(t);
     for (int si = 0; si < T.n_stages; ++si) {
@@ -671,6 +675,21 @@ __global__ void __launch_bounds__(kTreeThreads, 1) k_tree(DevCtx c, TreeRef T, i
         // block in the next stages, and its partial sums are overwritten
         __syncthreads();
     }
+}
+
+template <bool kResident>
+__global__ void __launch_bounds__(kTreeThreads, 1) k_tree(DevCtx c, TreeRef T, int H, int iter_add) {
+    extern __shared__ __align__(16) char smem[];
+    const char *tab = T.blob;
+    if constexpr (kResident) {
+        int4 *dst = reinterpret_cast<int4 *>(smem + static_cast<size_t>(T.max_chains) * kTreeHands * sizeof(float));
+        const int4 *src = reinterpret_cast<const int4 *>(T.blob);
+        for (int i = threadIdx.x; i < T.bytes / 16; i += blockDim.x) dst[i] = __ldg(src + i);
+        tab = reinterpret_cast<const char *>(dst);
+    }
+    wait_prior_grid();
+    if constexpr (kResident) __syncthreads();
+    tree_pass(c, T, tab, reinterpret_cast<float *>(smem), blockIdx.x * kTreeHands, H, *c.iter + iter_add);
 }
 
 // --------------------------------------------------------------------------
@@ -1715,6 +1734,630 @@ __global__ void __launch_bounds__(kSd1Threads, 2) k_term_light(DevCtx c0, const 
     const DevCtx &c = ctxs ? ctxs[I.sg] : c0;
     float *out = c.val + static_cast<size_t>(I.node) * c.HS;
     for (int h = tid; h < c.HS; h += kTermThreads) out[h] = 0.f;
+}
+
+// --------------------------------------------------------------------------
+// Many iterations of a small heads-up subgame in one cooperative launch: the
+// terminals of a traverser spread over the blocks, a grid barrier, the
+// traverser's tree (8 hands per block), a grid barrier, and so on.
+//
+// Such an iteration is bound by the latency of its chain of dependent steps.
+// As launches it was four kernels of 7-8 us, and in this form with the tree in
+// global memory still 8 us a phase: each level's values and regrets made a
+// round trip through L2 (4,000 cycles a level).  So a block keeps what only
+// its own hands touch in shared memory for the whole launch -- regrets,
+// strategy sums, the pass's values and reach -- beside the tables that no
+// kernel writes; what crosses the blocks is the reach rows (to the other
+// player's terminals) and the terminal rows, one L2 round trip each per phase.
+// Summation orders and expressions are those of the separate kernels.
+// Per iteration: heads-up river of 51 nodes and 1081 hands 34.4 us as launches,
+// 19.2 so (terminals 4.5 us, tree 3.3 us, two barriers 1.5 us each, twice); 141
+// nodes and 90 hands 35.8 -> 20.3; turn of 1,081 nodes and 1128 hands 58.6 ->
+// 42.5.
+// --------------------------------------------------------------------------
+constexpr unsigned kFaultGridWait = 4u;   // k_small_solve: a grid barrier's wait ran out
+constexpr unsigned kGridPolls = 4u << 20; // polls of the barrier (seconds) before a block gives up
+constexpr int kSmallThreads = kSd1Threads;
+
+// All blocks of the (cooperative) grid; count starts at 0 and grows by
+// gridDim.x per barrier.  False when the wait ran out: the caller returns.
+__device__ bool grid_barrier(unsigned *count) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned before;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(count) : "memory");
+        const unsigned target = (before / gridDim.x + 1u) * gridDim.x;
+        unsigned now = before + 1u, polls = 0;
+        while (static_cast<int>(now - target) < 0 && ++polls < kGridPolls)
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(count) : "memory");
+        ok = static_cast<int>(now - target) >= 0;
+        if (!ok) atomicOr(&g_ss_fault, kFaultGridWait);
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// Tables of one traverser's terminals in shared memory.
+struct SmallHand {         // a traverser hand at showdowns and folds
+    unsigned a, b, c;      // a: rank position | lo << 11; b: hi | c1 << 11 | c2 << 17 | unranked << 31;
+};                         // c: l1lo | l1hi << 6 | l2lo << 12 | l2hi << 18
+// (beside them: the player's hand at each rank position as short, -1 if none;
+// per card the rank positions of its combos as short, -1 past them, and their
+// number; per traverser hand dense a | dense b << 6 | its index
+// in the opponent's range << 12; the player's hand of each dense-card pair as
+// short, HS if none)
+
+__host__ __device__ constexpr size_t small_fold_space(int HS) { return (static_cast<size_t>(HS) + 4) * sizeof(float) + 64 * 12 + 64; }
+
+SmallLayout small_layout(const SmallRef &s, int HS, int ncomb, const int *H) {
+    SmallLayout L{};
+    unsigned at = 0;
+    auto take = [&](size_t bytes) {
+        const unsigned off = at;
+        at += static_cast<unsigned>((bytes + 15) / 16 * 16);
+        return off;
+    };
+    const bool river = s.n_sd1[0] + s.n_sd1[1] > 0, folds = s.n_cr1[0] + s.n_cr1[1] > 0;
+    const size_t row = kTreeHands * sizeof(float);
+    for (int p = 0; p < 2; ++p) L.tab[p] = take(s.tree[p].bytes);
+    for (int p = 0; p < 2; ++p) L.sd[p] = take(river ? H[p] * sizeof(SmallHand) : 0);
+    for (int p = 0; p < 2; ++p) L.pos_hand[p] = take(river ? ncomb * sizeof(short) : 0);
+    L.list = take(river ? 52 * 52 * sizeof(short) : 0);
+    L.clen = take(river ? 52 * sizeof(int) : 0);
+    for (int p = 0; p < 2; ++p) L.fold[p] = take(folds ? H[p] * sizeof(unsigned) : 0);
+    for (int p = 0; p < 2; ++p) L.pair[p] = take(folds ? 52 * 52 * sizeof(short) : 0);
+    for (int p = 0; p < 2; ++p) L.R[p] = take(s.tree[p].n_edges * row);
+    for (int p = 0; p < 2; ++p) L.S[p] = take(s.tree[p].n_edges * row);
+    // the phases' own space: a showdown, four folds, or a pass's rows and reach
+    size_t work = 0;
+    if (river) work = std::max(work, sd1_smem<float>());
+    if (folds) work = std::max(work, kLightGroups * small_fold_space(HS));
+    for (int p = 0; p < 2; ++p)
+        work = std::max(work, (static_cast<size_t>(s.tree[p].n_rows) + s.tree[p].n_edges) * row);
+    L.phase = take(work);
+    L.total = at;
+    return L;
+}
+
+// One two-way showdown (sd1_terminal on the tables in shared memory).
+__device__ __forceinline__ void small_sd1(const DevCtx &c, const SmallHand *hands, const short *pos_hand,
+                                          const short *card_list, const int *clen, const TermItem &I, int trav,
+                                          char *smem) {
+    Carve cv{smem};
+    float *Rr = cv.take<float>(1326);
+    double *Pp = cv.take<double>(1327);
+    double *PC = cv.take<double>(52 * 53);
+    double *wsum = cv.take<double>(kSd1Scan / 32);
+    int *wpos = cv.take<int>(kSmallThreads / 32);   // positions of positive reach, per warp
+    int *npos = cv.take<int>(52);                   // and per card
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int kRounds = (kMaxHS + kSmallThreads - 1) / kSmallThreads;   // positions, hands per thread
+    const int nc = c.ncomb, HS = c.HS, Ht = c.H[trav], opp = 1 - trav;
+    const float *r = c.reach + static_cast<size_t>(I.opp_row[0]) * HS;
+    if (!c.dup[opp]) {
+        float x[kRounds];
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+            const int q = tid + k * kSmallThreads, j = q < nc ? pos_hand[q] : -1;
+            x[k] = j >= 0 ? r[j] : 0.f;
+        }
+        int pos = 0;
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+            pos += __popc(__ballot_sync(0xffffffffu, x[k] > 0.f));
+            if (tid + k * kSmallThreads < nc) Rr[tid + k * kSmallThreads] = x[k];
+        }
+        if (lane == 0) wpos[warp] = pos;
+    } else {
+        for (int i = tid; i < nc; i += kSmallThreads) Rr[i] = 0.f;
+        __syncthreads();
+        const int *pos = c.sd_pos + static_cast<size_t>(opp) * HS;
+        for (int j = tid; j < c.H[opp]; j += kSmallThreads)
+            if (pos[j] >= 0) atomicAdd(&Rr[pos[j]], r[j]);
+        __syncthreads();
+        int n = 0;
+        for (int q = warp * 32; q < nc; q += kSmallThreads)
+            n += __popc(__ballot_sync(0xffffffffu, q + lane < nc && Rr[q + lane] > 0.f));
+        if (lane == 0) wpos[warp] = n;
+    }
+    __syncthreads();
+    if (warp < kSd1Scan / 32) {
+        // each thread's run of at most kRun positions in registers
+        constexpr int kRun = (1326 + kSd1Scan - 1) / kSd1Scan;
+        const int per = (nc + kSd1Scan - 1) / kSd1Scan, b0 = tid * per;
+        double x[kRun], local = 0.0;
+#pragma unroll
+        for (int i = 0; i < kRun; ++i) x[i] = i < per && b0 + i < nc ? static_cast<double>(Rr[b0 + i]) : 0.0;
+        local = x[0];
+#pragma unroll
+        for (int i = 1; i < kRun; ++i)
+            if (i < per) local += x[i];
+        double incl = local;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const double y = __shfl_up_sync(0xffffffffu, incl, k);
+            if (lane >= k) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        asm volatile("bar.sync 1, %0;" ::"n"(kSd1Scan) : "memory");
+        double ws[kSd1Scan / 32], base = 0.0, tot = 0.0;
+#pragma unroll
+        for (int w = 0; w < kSd1Scan / 32; ++w) ws[w] = wsum[w];
+#pragma unroll
+        for (int w = 0; w < kSd1Scan / 32; ++w) {
+            if (w == warp) base = tot;
+            tot += ws[w];
+        }
+        double run = base + incl - local;
+#pragma unroll
+        for (int i = 0; i < kRun; ++i) {
+            if (i < per) {
+                if (b0 + i < nc) Pp[b0 + i] = run;
+                run += x[i];
+            }
+        }
+        if (tid == kSd1Scan - 1) Pp[nc] = tot;
+    } else {
+        // this warp's cards side by side (one at a time is a chain of
+        // shuffles and FP64 additions per card)
+        constexpr int kCardWarps = (kSmallThreads - kSd1Scan) / 32, kCards = (52 + kCardWarps - 1) / kCardWarps;
+        const int i0 = 2 * lane, i1 = 2 * lane + 1, c0 = warp - kSd1Scan / 32;
+        double v0[kCards], pair[kCards], incl[kCards];
+#pragma unroll
+        for (int k = 0; k < kCards; ++k) {
+            const int card = c0 + k * kCardWarps;
+            const bool on = card < 52 && i0 < 52;   // i1 = i0 + 1 < 52 as well
+            const short2 q = on ? *reinterpret_cast<const short2 *>(card_list + card * 52 + i0) : make_short2(-1, -1);
+            const float f0 = q.x >= 0 ? Rr[q.x] : 0.f, f1 = q.y >= 0 ? Rr[q.y] : 0.f;
+            v0[k] = f0;
+            pair[k] = incl[k] = static_cast<double>(f0) + static_cast<double>(f1);
+            const int n = __popc(__ballot_sync(0xffffffffu, f0 > 0.f)) + __popc(__ballot_sync(0xffffffffu, f1 > 0.f));
+            if (lane == 0 && card < 52) npos[card] = n;
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            double y[kCards];
+#pragma unroll
+            for (int k = 0; k < kCards; ++k) y[k] = __shfl_up_sync(0xffffffffu, incl[k], d);
+#pragma unroll
+            for (int k = 0; k < kCards; ++k)
+                if (lane >= d) incl[k] += y[k];
+        }
+#pragma unroll
+        for (int k = 0; k < kCards; ++k) {
+            const int card = c0 + k * kCardWarps;
+            if (card >= 52) continue;
+            const int len = clen[card];
+            const double ex = incl[k] - pair[k];
+            if (i0 <= len) PC[card * 53 + i0] = ex;
+            if (i1 <= len) PC[card * 53 + i1] = ex + v0[k];
+        }
+    }
+    __syncthreads();
+    const int N = __reduce_add_sync(0xffffffffu, wpos[lane]);
+    const double total = Pp[nc];
+    float *out = c.val + static_cast<size_t>(I.node) * HS;
+    const double cw = static_cast<double>(I.pot - I.bet), ct = static_cast<double>(I.pot * 0.5f - I.bet);
+    const double cl = -static_cast<double>(I.bet);
+    double v[kRounds];
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k) {
+        const int h = tid + k * kSmallThreads;
+        v[k] = 0.0;
+        const SmallHand e = h < Ht ? hands[h] : SmallHand{0u, 1u << 31, 0u};
+        if (!(e.b >> 31)) {
+            const int q = e.a & 2047, lo = e.a >> 11, hi = e.b & 2047;
+            const int c1 = e.b >> 11 & 63, c2 = e.b >> 17 & 63;
+            const int l1lo = e.c & 63, l1hi = e.c >> 6 & 63, l2lo = e.c >> 12 & 63, l2hi = e.c >> 18 & 63;
+            const double *p1 = PC + c1 * 53, *p2 = PC + c2 * 53;
+            const float self = Rr[q];
+            const double W = Pp[lo] - p1[l1lo] - p2[l2lo];
+            const double Tt = (Pp[hi] - Pp[lo]) - (p1[l1hi] - p1[l1lo]) - (p2[l2hi] - p2[l2lo]) + static_cast<double>(self);
+            const double L = (total - Pp[hi]) - (p1[clen[c1]] - p1[l1hi]) - (p2[clen[c2]] - p2[l2hi]);
+            const double x = cw * W + ct * Tt + cl * L;
+            // a hand without a compatible hand of positive reach gets exactly 0
+            if (N - npos[c1] - npos[c2] + (self > 0.f ? 1 : 0) > 0) v[k] = x;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k)
+        if (tid + k * kSmallThreads < HS) store_value(out, tid + k * kSmallThreads, v[k]);
+}
+
+// One group of one-opponent folds or leaves (cr1_terminal on the tables in
+// shared memory) by kTermThreads threads with barrier `bar`.
+__device__ __forceinline__ void small_cr1(const DevCtx &c, const unsigned *hands, const short *pair,
+                                          const TermItem *__restrict__ I0, int trav, char *smem, int tid, int bar) {
+    if (I0->follow) return;
+    constexpr int kRounds = (kMaxHS + kTermThreads - 1) / kTermThreads;
+    auto sync = [bar] { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kTermThreads) : "memory"); };
+    const int ng = I0->gextra + 1, lane = tid & 31;
+    const int HS = c.HS, Ht = c.H[trav], Dp = (c.deck + 3) & ~3;
+    Carve cv{smem};
+    float *r = cv.take<float>(HS + 4);
+    double *u = cv.take<double>(64);
+    int *nz = cv.take<int>(64);
+    const float *src = c.reach + static_cast<size_t>(I0->opp_row[0]) * HS;
+    for (int q = tid * 4; q < HS; q += kTermThreads * 4) cp_async16(r + q, src + q);
+    // an item's factors of this thread's hands, loaded well before their use
+    auto factors = [&](const TermItem &I, float f[kRounds]) {
+        const int lo = __ldg(&I.leaf_off);
+        const float pay = __ldg(&I.payoff);
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+            const int h = tid + k * kTermThreads;
+            f[k] = h >= Ht ? 0.f : lo >= 0 ? __ldg(c.leaf_values + lo + h) : pay;
+        }
+    };
+    float f[kRounds];
+    factors(*I0, f);
+    if (tid == 0) r[HS] = 0.f;
+    if (tid < 64) {
+        u[tid] = 0.0;
+        nz[tid] = 0;
+    }
+    cp_async_wait_all();
+    sync();
+    {
+        const int col = tid >> 2, part = tid & 3, q = Dp >> 2;
+        double s = 0.0;
+        int n = 0;
+        if (col < Dp) {
+            const short *row = pair + col * 52 + part * q;
+            for (int b = 0; b < q; ++b) {
+                const float x = r[row[b]];
+                s += static_cast<double>(x);
+                n += x > 0.f ? 1 : 0;
+            }
+        }
+#pragma unroll
+        for (int k = 1; k < 4; k <<= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, k);
+            n += __shfl_xor_sync(0xffffffffu, n, k);
+        }
+        if (part == 0 && col < Dp) {
+            u[col] = s;
+            nz[col] = n;
+        }
+    }
+    sync();
+    double F;
+    int N;
+    {
+        double s = (lane < Dp ? u[lane] : 0.0) + (lane + 32 < Dp ? u[lane + 32] : 0.0);
+        int n = (lane < Dp ? nz[lane] : 0) + (lane + 32 < Dp ? nz[lane + 32] : 0);
+        s = warp_sum(s);
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) n += __shfl_xor_sync(0xffffffffu, n, k);
+        F = 0.5 * s;
+        N = n / 2;
+    }
+    double v[kRounds];
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k) {
+        const int h = tid + k * kTermThreads;
+        v[k] = 0.0;
+        if (h < Ht) {
+            const unsigned e = hands[h];
+            const int a = e & 63, b = e >> 6 & 63;
+            const float x = r[e >> 12];
+            const int live = N - nz[a] - nz[b] + (x > 0.f ? 1 : 0);
+            if (live > 0) v[k] = F - u[a] - u[b] + static_cast<double>(x);
+        }
+    }
+    for (int g = 0; g < ng; ++g) {
+        float *out = c.val + static_cast<size_t>(__ldg(&I0[g].node)) * HS;
+        float fn[kRounds];
+        if (g + 1 < ng)
+            factors(I0[g + 1], fn);
+        else
+            for (int k = 0; k < kRounds; ++k) fn[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+            const int h = tid + k * kTermThreads;
+            if (h < HS) out[h] = static_cast<float>(static_cast<double>(f[k]) * v[k]);
+            f[k] = fn[k];
+        }
+    }
+}
+
+// One player's values and regrets bottom-up, then its reach top-down, for hand
+// h of the block's 8 (act: a hand of the range): rv holds the frontier rows,
+// rs the reach of the local edges, weight the hand's range weight.  Iteration
+// t; node values also go to global memory with `keep`.
+//
+// A warp per item, a lane per (action, hand): one thread walking an item's
+// actions was a chain of some 300 dependent instructions, 6,000 cycles a
+// level.  The sums over actions run in action order on shuffled operands, the
+// same in every lane of a hand.
+__device__ __forceinline__ void whole_pass(const DevCtx &c, const WholeRef &T, const char *tab, float *R, float *S,
+                                           float *rv, float *rs, int h, bool act, float weight, int t, bool keep) {
+    const WholeItem *items = reinterpret_cast<const WholeItem *>(tab);
+    const WholeReach *reach = reinterpret_cast<const WholeReach *>(tab + T.o_reach);
+    const short *edge_end = reinterpret_cast<const short *>(tab + T.o_end);
+    const int *rows = reinterpret_cast<const int *>(tab + T.o_rows);
+    const int *voff = reinterpret_cast<const int *>(tab + T.o_voff), *roff = reinterpret_cast<const int *>(tab + T.o_roff);
+    const int hand = threadIdx.x & (kTreeHands - 1), warp = threadIdx.x >> 5;
+    const int a4 = (threadIdx.x & 31) / kTreeHands;   // this lane's actions: a4 and a4 + 4
+    constexpr int kWarps = kSmallThreads / 32, kSlots = kSmallThreads / kTreeHands;
+    static_assert(kTreeHands == 8 && SS_MAX_ACTIONS == 8, "a warp covers four actions of eight hands, twice");
+    const size_t HS = static_cast<size_t>(c.HS);
+    const float d = static_cast<float>(t) / (static_cast<float>(t) + 1.0f);
+    const float w = static_cast<float>(t);
+    if (act) {
+        const float *val = c.val + h;
+        constexpr int kAhead = 8;   // rows in flight per thread
+        for (int i0 = threadIdx.x / kTreeHands; i0 < T.n_rows; i0 += kAhead * kSlots) {
+            int row[kAhead];
+            float x[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) row[k] = i0 + k * kSlots < T.n_rows ? rows[i0 + k * kSlots] : -1;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) x[k] = row[k] >= 0 ? val[static_cast<size_t>(row[k]) * HS] : 0.f;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+                if (row[k] >= 0) rv[(i0 + k * kSlots) * kTreeHands + hand] = x[k];
+        }
+    }
+    __syncthreads();
+    // the strategy of this lane's actions from their regrets
+    auto strategy = [&](const float r[2], int na, int frozen, float uniform, float sig[2]) {
+        float rp[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) rp[j] = a4 + 4 * j < na && r[j] > 0.f ? r[j] : 0.f;
+        // past the node's actions rp is +0, which changes no sum
+        float x[4], sum = 0.f;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) x[a] = __shfl_sync(0xffffffffu, rp[0], a * kTreeHands + hand);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) sum += x[a];
+        if (na > 4) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) x[a] = __shfl_sync(0xffffffffu, rp[1], a * kTreeHands + hand);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) sum += x[a];
+        }
+        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            sig[j] = sum > 0.f ? rp[j] * inv : uniform;
+            if (frozen >= 0) sig[j] = a4 + 4 * j == frozen ? 1.0f : 0.0f;
+        }
+    };
+    for (int l = 0; l < T.value_levels; ++l) {
+        for (int it = voff[l] + warp; it < voff[l + 1]; it += kWarps) {
+            const WholeItem I = items[it];
+            const int na = I.na;
+            float r[2] = {0.f, 0.f}, ev[2] = {0.f, 0.f}, sig[2], sm[2] = {0.f, 0.f};
+            float *Rh = R + (I.edge0 + a4) * kTreeHands + hand, *Sh = S + (I.edge0 + a4) * kTreeHands + hand;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (j == 1 && na <= 4) break;
+                const int a = a4 + 4 * j;
+                if (a >= na) continue;
+                r[j] = Rh[4 * j * kTreeHands];
+                sm[j] = Sh[4 * j * kTreeHands];
+                int k = a ? edge_end[I.edge0 + a - 1] : I.row0;
+                const int end = edge_end[I.edge0 + a];
+                const float *x = rv + hand;
+                if (I.split == 1) {
+                    float e = 0.f;
+                    for (; k + 3 < end; k += 4) {
+                        const float x0 = x[k * kTreeHands], x1 = x[(k + 1) * kTreeHands];
+                        const float x2 = x[(k + 2) * kTreeHands], x3 = x[(k + 3) * kTreeHands];
+                        e += x0;
+                        e += x1;
+                        e += x2;
+                        e += x3;
+                    }
+                    for (; k < end; ++k) e += x[k * kTreeHands];
+                    ev[j] = e;
+                } else {
+                    // four interleaved chains, added in order
+                    static_assert(kCfvSplit == 4, "four chains");
+                    float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
+                    for (; k < end; k += 4) {
+                        q0 += x[k * kTreeHands];
+                        if (k + 1 < end) q1 += x[(k + 1) * kTreeHands];
+                        if (k + 2 < end) q2 += x[(k + 2) * kTreeHands];
+                        if (k + 3 < end) q3 += x[(k + 3) * kTreeHands];
+                    }
+                    ev[j] = q0 + q1 + q2 + q3;
+                }
+            }
+            strategy(r, na, I.frozen, I.uniform, sig);
+            // past the node's actions ev is +0, whose products add nothing
+            float v = 0.f;
+            auto add4 = [&](float sj, float ej) {
+                float sa[4], ea[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    sa[a] = __shfl_sync(0xffffffffu, sj, a * kTreeHands + hand);
+                    ea[a] = __shfl_sync(0xffffffffu, ej, a * kTreeHands + hand);
+                }
+#pragma unroll
+                for (int a = 0; a < 4; ++a) v += sa[a] * ea[a];
+            };
+            add4(sig[0], ev[0]);
+            if (na > 4) add4(sig[1], ev[1]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if ((j == 0 || na > 4) && a4 + 4 * j < na) {
+                    Rh[4 * j * kTreeHands] = (r[j] + (ev[j] - v)) * d;
+                    Sh[4 * j * kTreeHands] = sm[j] + w * sig[j];
+                }
+            v *= I.scale;
+            if (a4 == 0) {
+                if (I.row >= 0) rv[I.row * kTreeHands + hand] = v;
+                if (keep && act) c.val[static_cast<size_t>(I.node) * HS + h] = v;
+            }
+        }
+        __syncthreads();
+    }
+    for (int l = 0; l < T.reach_levels; ++l) {
+        for (int it = roff[l] + warp; it < roff[l + 1]; it += kWarps) {
+            const WholeReach I = reach[it];
+            const int na = I.na;
+            const float pr = I.parent >= 0 ? rs[I.parent * kTreeHands + hand] : weight;
+            float r[2] = {0.f, 0.f}, sig[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if ((j == 0 || na > 4) && a4 + 4 * j < na) r[j] = R[(I.edge0 + a4 + 4 * j) * kTreeHands + hand];
+            strategy(r, na, I.frozen, I.uniform, sig);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int a = a4 + 4 * j;
+                if ((j == 1 && na <= 4) || a >= na) continue;
+                const float x = pr * sig[j];
+                rs[(I.edge0 + a) * kTreeHands + hand] = x;
+                if (act) c.reach[static_cast<size_t>(I.first_edge + a) * HS + h] = x;
+            }
+        }
+        if (l + 1 < T.reach_levels) __syncthreads();   // a grid barrier follows the last
+    }
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_constant__ DevCtx c,
+                                                                const __grid_constant__ SmallRef s, int iters,
+                                                                int snapshot) {
+    extern __shared__ __align__(16) char smem[];
+    const size_t HS = static_cast<size_t>(c.HS);
+    const bool river = s.n_sd1[0] + s.n_sd1[1] > 0, folds = s.n_cr1[0] + s.n_cr1[1] > 0;
+    const int hand = threadIdx.x & (kTreeHands - 1), h = blockIdx.x * kTreeHands + hand;
+    float weight0 = 0.f, weight1 = 0.f;
+    // tables and the block's rows
+    for (int p = 0; p < 2; ++p) {
+        const int4 *src = reinterpret_cast<const int4 *>(s.tree[p].blob);
+        for (int i = threadIdx.x; i < s.tree[p].bytes / 16; i += kSmallThreads)
+            reinterpret_cast<int4 *>(smem + s.at.tab[p])[i] = __ldg(src + i);
+        if (river) {
+            for (int q = threadIdx.x; q < c.ncomb; q += kSmallThreads)
+                reinterpret_cast<short *>(smem + s.at.pos_hand[p])[q] = static_cast<short>(__ldg(c.pos_hand + static_cast<size_t>(p) * c.ncomb + q));
+            for (int i = threadIdx.x; i < c.H[p]; i += kSmallThreads) {
+                const int q = __ldg(c.sd_pos + p * HS + i);
+                SmallHand e{0u, 1u << 31, 0u};
+                if (q >= 0) {
+                    const SdCombo &k = c.sd_combo[q];
+                    e.a = static_cast<unsigned>(q) | static_cast<unsigned>(k.lo) << 11;
+                    e.b = static_cast<unsigned>(k.hi) | static_cast<unsigned>(k.c1) << 11 | static_cast<unsigned>(k.c2) << 17;
+                    e.c = static_cast<unsigned>(k.l1lo) | static_cast<unsigned>(k.l1hi) << 6 |
+                          static_cast<unsigned>(k.l2lo) << 12 | static_cast<unsigned>(k.l2hi) << 18;
+                }
+                reinterpret_cast<SmallHand *>(smem + s.at.sd[p])[i] = e;
+            }
+        }
+        if (folds) {
+            for (int i = threadIdx.x; i < 52 * 52; i += kSmallThreads)
+                reinterpret_cast<short *>(smem + s.at.pair[p])[i] = static_cast<short>(__ldg(c.pair_idx + p * 52 * 52 + i));
+            for (int i = threadIdx.x; i < c.H[p]; i += kSmallThreads) {
+                const int hc = __ldg(c.hand_code + p * HS + i);
+                const unsigned a = min((hc >> 20) & 63, kCr2Off), b = min((hc >> 26) & 63, kCr2Off);
+                const unsigned x = __ldg(c.cross_idx + (static_cast<size_t>(p) * c.np + (1 - p)) * HS + i);
+                reinterpret_cast<unsigned *>(smem + s.at.fold[p])[i] = a | b << 6 | x << 12;
+            }
+        }
+    }
+    {
+        const float *own = c.reach + static_cast<size_t>(s.tree[0].n_edges + s.tree[1].n_edges) * HS + h;
+        if (h < c.H[0]) weight0 = own[0];
+        if (h < c.H[1]) weight1 = own[HS];
+    }
+    if (river)
+        for (int i = threadIdx.x; i < 52 * 52; i += kSmallThreads)
+            reinterpret_cast<short *>(smem + s.at.list)[i] = __ldg(c.sd_card_list + i);
+    if (river && threadIdx.x < 52) {
+        int n = 0;
+        while (n < 52 && __ldg(c.sd_card_list + threadIdx.x * 52 + n) >= 0) ++n;
+        reinterpret_cast<int *>(smem + s.at.clen)[threadIdx.x] = n;
+    }
+    __syncthreads();
+    // the block's regrets and strategy sums, in and (at the end) out
+    auto rows = [&](bool out) {
+        for (int p = 0; p < 2; ++p) {
+            const int *edge_row = reinterpret_cast<const int *>(smem + s.at.tab[p] + s.tree[p].o_edge);
+            float *R = reinterpret_cast<float *>(smem + s.at.R[p]), *S = reinterpret_cast<float *>(smem + s.at.S[p]);
+            if (h < c.H[p])
+                for (int e = threadIdx.x / kTreeHands; e < s.tree[p].n_edges; e += kSmallThreads / kTreeHands) {
+                    const size_t g = static_cast<size_t>(edge_row[e]) * HS + h;
+                    if (out) {
+                        c.R[g] = R[e * kTreeHands + hand];
+                        c.S[g] = S[e * kTreeHands + hand];
+                    } else {
+                        R[e * kTreeHands + hand] = c.R[g];
+                        S[e * kTreeHands + hand] = c.S[g];
+                    }
+                }
+        }
+    };
+    rows(false);
+    __shared__ TermItem first_sd1[2];
+    if (threadIdx.x < 2 && static_cast<int>(blockIdx.x) < s.n_sd1[threadIdx.x])
+        first_sd1[threadIdx.x] = s.sd1[threadIdx.x][blockIdx.x];
+    const int base = *c.iter;
+    const int group = threadIdx.x / kTermThreads, tid = threadIdx.x % kTermThreads;
+    char *work = smem + s.at.phase;
+    __syncthreads();
+    for (int it = 1; it <= iters; ++it) {
+        for (int t = 0; t < 2; ++t) {
+            const int n_sd1 = s.n_sd1[t], n_cr1 = s.n_cr1[t], n_zero = s.n_zero[t];
+            const int cr1_jobs = (n_cr1 + kLightGroups - 1) / kLightGroups;
+            const int jobs = n_sd1 + cr1_jobs + (n_zero + kLightGroups - 1) / kLightGroups;
+            for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
+                if (job < n_sd1) {
+                    // the block's first showdown is the same every iteration
+                    small_sd1(c, reinterpret_cast<const SmallHand *>(smem + s.at.sd[t]),
+                              reinterpret_cast<const short *>(smem + s.at.pos_hand[1 - t]),
+                              reinterpret_cast<const short *>(smem + s.at.list),
+                              reinterpret_cast<const int *>(smem + s.at.clen), job == static_cast<int>(blockIdx.x) ? first_sd1[t] : s.sd1[t][job], t, work);
+                } else if (job < n_sd1 + cr1_jobs) {
+                    const int i = (job - n_sd1) * kLightGroups + group;
+                    if (i < n_cr1)
+                        small_cr1(c, reinterpret_cast<const unsigned *>(smem + s.at.fold[t]),
+                                  reinterpret_cast<const short *>(smem + s.at.pair[1 - t]), s.cr1[t] + i, t,
+                                  work + group * small_fold_space(c.HS), tid, group + 1);
+                } else {
+                    const int i = (job - n_sd1 - cr1_jobs) * kLightGroups + group;
+                    if (i < n_zero) {
+                        float *out = c.val + static_cast<size_t>(s.zero[t][i].node) * HS;
+                        for (int k = tid; k < c.HS; k += kTermThreads) out[k] = 0.f;
+                    }
+                }
+                if (job + static_cast<int>(gridDim.x) < jobs) __syncthreads();   // the next job's space
+            }
+            if (!grid_barrier(s.barrier)) return;
+            float *R = reinterpret_cast<float *>(smem + s.at.R[t]), *S = reinterpret_cast<float *>(smem + s.at.S[t]);
+            // the root strategy before the last traverser's pass
+            if (snapshot && it == iters && t == 1) {
+                const int p = c.root_player;
+                const int *edge_row = reinterpret_cast<const int *>(smem + s.at.tab[p] + s.tree[p].o_edge);
+                const float *Rp = reinterpret_cast<const float *>(smem + s.at.R[p]);
+                int e = 0;   // the root's first local edge
+                while (e < s.tree[p].n_edges && edge_row[e] != c.root_fe) ++e;
+                if (threadIdx.x < kTreeHands && h < c.H[p]) {
+                    float sum = 0.f;
+                    for (int a = 0; a < c.root_na; ++a) {
+                        const float r = Rp[(e + a) * kTreeHands + hand];
+                        sum += r > 0.f ? r : 0.f;
+                    }
+                    const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+                    for (int a = 0; a < c.root_na; ++a) {
+                        const float r = Rp[(e + a) * kTreeHands + hand];
+                        float x = sum > 0.f ? (r > 0.f ? r : 0.f) * inv : 1.0f / static_cast<float>(c.root_na);
+                        if (c.root_frozen >= 0) x = a == c.root_frozen ? 1.0f : 0.0f;
+                        c.snap[static_cast<size_t>(a) * c.H[p] + h] = x;
+                    }
+                }
+                __syncthreads();
+            }
+            float *rv = reinterpret_cast<float *>(work);
+            whole_pass(c, s.tree[t], smem + s.at.tab[t], R, S, rv, rv + s.tree[t].n_rows * kTreeHands, h, h < c.H[t],
+                       t ? weight1 : weight0, base + it, it == iters);
+            if (!grid_barrier(s.barrier)) return;
+        }
+    }
+    rows(true);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *const_cast<int *>(c.iter) = base + iters;
 }
 
 // ---------------------------------------------------------------------------
@@ -3023,14 +3666,8 @@ __global__ void __launch_bounds__(128) k_snapshot_many(const DevCtx *__restrict_
     wait_prior_grid();
     const DevCtx &c = ctxs[sgs[blockIdx.x]];
     if (!c.live) return;
-    const int H = c.H[c.root_player];
-    for (int h0 = threadIdx.x * 4; h0 < H; h0 += blockDim.x * 4) {
-        float r[SS_MAX_ACTIONS][4], sig[SS_MAX_ACTIONS][4];
-        regret_match4(c.R, static_cast<size_t>(c.HS), c.root_fe, c.root_na, c.root_frozen, h0, r, sig);
-        for (int a = 0; a < c.root_na; ++a)
-            for (int i = 0; i < 4; ++i)
-                if (h0 + i < H) c.snap[static_cast<size_t>(a) * H + h0 + i] = sig[a][i];
-    }
+    root_strategy(c.R, static_cast<size_t>(c.HS), c.root_fe, c.root_na, c.root_frozen, c.H[c.root_player], c.snap,
+                  threadIdx.x, blockDim.x);
 }
 
 __global__ void k_bump(int *iter, int by) {
@@ -3049,17 +3686,11 @@ __global__ void __launch_bounds__(kHandThreads) k_sum_rows(DevCtx c, const int *
     out[h] = s;
 }
 
-// regret-matched (and frozen) strategy of one node, [na][H] (street_solve.cu:1564-1573)
 __global__ void __launch_bounds__(kHandThreads) k_root_strategy(DevCtx c, int fe, int na, int frozen,
                                                                 int H, float *out) {
     wait_prior_grid();
-    const int h0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (h0 >= H) return;
-    float r[SS_MAX_ACTIONS][4], sig[SS_MAX_ACTIONS][4];
-    regret_match4(c.R, static_cast<size_t>(c.HS), fe, na, frozen, h0, r, sig);
-    for (int a = 0; a < na; ++a)
-        for (int i = 0; i < 4; ++i)
-            if (h0 + i < H) out[static_cast<size_t>(a) * H + h0 + i] = sig[a][i];
+    root_strategy(c.R, static_cast<size_t>(c.HS), fe, na, frozen, H, out, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
 }
 
 // normalised strategy sums of every decision node in the output layout
@@ -3171,6 +3802,47 @@ cudaError_t launch_tree(const DevCtx &c, const TreeRef &t, int H, cudaStream_t s
         SSB_LAUNCH(k_tree<false>, grid, t.threads, sm, s, c, t, H, iter_add);
     }
     return cudaGetLastError();
+}
+
+// The grid: a block per 8 hands and per terminal job, at most one per SM.
+int small_solve_blocks(const DevCtx &c, SmallRef *ref) {
+    SmallRef &s = *ref;
+    int dev = 0, coop = 0, sms = 0, optin = 0, per_sm = 0;
+    s.at = small_layout(s, c.HS, c.ncomb, c.H);
+    const size_t sm = s.at.total;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        sm > static_cast<size_t>(optin - 1024) ||
+        cudaFuncSetAttribute(k_small_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small_solve, kSmallThreads, sm) != cudaSuccess ||
+        per_sm < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    int widest = 1;
+    for (int t = 0; t < 2; ++t) {
+        const int jobs = s.n_sd1[t] + (s.n_cr1[t] + kLightGroups - 1) / kLightGroups +
+                         (s.n_zero[t] + kLightGroups - 1) / kLightGroups;
+        const int chunks = (c.H[t] + kTreeHands - 1) / kTreeHands;
+        if (chunks > sms) return 0;   // a block owns 8 hands for the whole launch
+        widest = std::max({widest, jobs, chunks});
+    }
+    return std::min(widest, sms);
+}
+
+cudaError_t launch_small_solve(const DevCtx &c, const SmallRef &s, int blocks, int iters, bool snapshot,
+                               cudaStream_t st) {
+    // the barrier counts from 0 in every launch (after a fault, too)
+    const cudaError_t e = cudaMemsetAsync(s.barrier, 0, sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    DevCtx ctx = c;
+    SmallRef ref = s;
+    int n = iters, snap = snapshot ? 1 : 0;
+    void *args[] = {&ctx, &ref, &n, &snap};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_small_solve), dim3(blocks), dim3(kSmallThreads),
+                                       args, s.at.total, st);
 }
 
 template <class T>

@@ -99,6 +99,32 @@ struct TreeRef {
 };
 // player's small levels in one launch, over its H hands
 cudaError_t launch_tree(const DevCtx &c, const TreeRef &t, int H, cudaStream_t s, int iter_add = 0);
+// A small heads-up subgame for k_small_solve: per player its tree (device copy
+// of a WholePass) and its terminals as the traverser (all two-way showdowns,
+// one-opponent folds or leaves, and zero rows).
+struct WholeRef {
+    const char *blob;
+    int bytes, o_reach, o_end, o_edge, o_rows, o_voff, o_roff;
+    int n_edges, n_rows, value_levels, reach_levels;
+};
+// Offsets of k_small_solve's shared memory (small_layout).
+struct SmallLayout {
+    unsigned tab[2], sd[2], pos_hand[2], list, clen, fold[2], pair[2], R[2], S[2], phase, total;
+};
+struct SmallRef {
+    WholeRef tree[2];
+    SmallLayout at;
+    const TermItem *sd1[2], *cr1[2], *zero[2];
+    int n_sd1[2], n_cr1[2], n_zero[2];
+    unsigned *barrier;   // grid barrier count
+};
+// Lays out s.at and returns the blocks of the cooperative grid; 0 where the
+// device or the shared memory cannot run it.
+int small_solve_blocks(const DevCtx &c, SmallRef *s);
+// `iters` iterations from *c.iter on (which advances); the root strategy of the
+// last one with snapshot
+cudaError_t launch_small_solve(const DevCtx &c, const SmallRef &s, int blocks, int iters, bool snapshot,
+                               cudaStream_t st);
 // heads (optional, TK_CR2): the n_heads items that start work (TermItem
 // groups and chains); the launch then has one block per head instead of one
 // per item (the tensor-core two-opponent form takes every item)

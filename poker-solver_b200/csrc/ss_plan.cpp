@@ -122,7 +122,7 @@ void inline_frontier(CfvItem &it, const std::vector<int> &fr_off, const std::vec
 // this bound: 3-player turn (21,436 nodes, 1128 hands) 917 without the pass,
 // 868 at 64, 856 at 128, 865 at 256, 1262 with every level in the pass;
 // heads-up turn (1,081 nodes) 81, 60, 59, 64.
-constexpr size_t kTreeLevelItems = 128;
+constexpr int kTreeLevelItems = 128;
 
 void build_tree_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const std::vector<int> &cfv_nlong,
                      const std::vector<std::vector<ReachItem>> &reach_levels, const std::vector<int> &fr_off,
@@ -130,8 +130,8 @@ void build_tree_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const 
     TreePass &T = *out;
     T = TreePass{};
     for (size_t l = 0; l < cfv_levels.size(); ++l)
-        if (cfv_levels[l].size() > kTreeLevelItems) T.cfv_from = static_cast<int>(l) + 1;
-    while (T.reach_to < static_cast<int>(reach_levels.size()) && reach_levels[T.reach_to].size() <= kTreeLevelItems)
+        if (static_cast<int>(cfv_levels[l].size()) > kTreeLevelItems) T.cfv_from = static_cast<int>(l) + 1;
+    while (T.reach_to < static_cast<int>(reach_levels.size()) && static_cast<int>(reach_levels[T.reach_to].size()) <= kTreeLevelItems)
         ++T.reach_to;
     int widest = 1;
     for (size_t l = static_cast<size_t>(T.cfv_from); l < cfv_levels.size(); ++l) {
@@ -185,6 +185,79 @@ void build_tree_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const 
     T.o_rows = put(T.rows.data(), T.rows.size() * sizeof(int));
     const int threads = (widest * kTreeHands + 31) / 32 * 32;
     T.threads = std::min(kTreeThreads, std::max(64, threads));
+}
+
+// largest heads-up tree for k_small_solve (its shared memory decides in the end)
+constexpr int kSmallNodes = 4096;
+
+void build_whole_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const std::vector<int> &cfv_nlong,
+                      const std::vector<std::vector<ReachItem>> &reach_levels, const std::vector<int> &fr_off,
+                      const std::vector<int> &fr_items, int num_edges, WholePass *out) {
+    WholePass &W = *out;
+    W = WholePass{};
+    std::vector<int> local(num_edges, -1);   // subgame edge -> local edge
+    std::vector<std::pair<int, int>> own;    // (node, item)
+    for (size_t l = 0; l < cfv_levels.size(); ++l) {
+        W.value_off.push_back(static_cast<int>(W.items.size()));
+        const size_t n_short = cfv_levels[l].size() - static_cast<size_t>(cfv_nlong[l]);
+        for (size_t j = 0; j < cfv_levels[l].size(); ++j) {
+            const CfvItem &it = cfv_levels[l][j];
+            WholeItem w{};
+            w.first_edge = it.first_edge;
+            w.node = it.node;
+            w.edge0 = static_cast<short>(W.edge_row.size());
+            w.na = static_cast<short>(it.na);
+            w.frozen = static_cast<short>(it.frozen);
+            w.split = j < n_short ? 1 : kCfvSplit;
+            w.row0 = static_cast<short>(W.rows.size());
+            w.row = -1;
+            w.scale = it.scale;
+            w.uniform = 1.0f / static_cast<float>(it.na);
+            for (int a = 0; a < it.na; ++a) {
+                local[it.first_edge + a] = static_cast<int>(W.edge_row.size());
+                W.edge_row.push_back(it.first_edge + a);
+                W.rows.insert(W.rows.end(), fr_items.begin() + fr_off[it.first_edge + a],
+                              fr_items.begin() + fr_off[it.first_edge + a + 1]);
+                W.edge_end.push_back(static_cast<short>(W.rows.size()));
+            }
+            if (W.rows.size() > 32000 || W.edge_row.size() > 32000) {
+                W = WholePass{};
+                return;
+            }
+            own.push_back({it.node, static_cast<int>(W.items.size())});
+            W.items.push_back(w);
+        }
+    }
+    W.value_off.push_back(static_cast<int>(W.items.size()));
+    std::sort(own.begin(), own.end());
+    for (size_t r = 0; r < W.rows.size(); ++r) {
+        const auto at = std::lower_bound(own.begin(), own.end(), std::make_pair(W.rows[r], -1));
+        if (at == own.end() || at->first != W.rows[r]) continue;
+        W.items[at->second].row = static_cast<short>(r);
+        W.rows[r] = -1;
+    }
+    for (const auto &lv : reach_levels) {
+        W.reach_off.push_back(static_cast<int>(W.reach.size()));
+        for (const ReachItem &it : lv)
+            W.reach.push_back(WholeReach{static_cast<short>(local[it.first_edge]), static_cast<short>(it.na),
+                                         static_cast<short>(it.parent_row < num_edges ? local[it.parent_row] : -1),
+                                         static_cast<short>(it.frozen), 1.0f / static_cast<float>(it.na),
+                                         it.first_edge});
+    }
+    W.reach_off.push_back(static_cast<int>(W.reach.size()));
+    auto put = [&](const void *src, size_t bytes) {
+        const size_t off = (W.blob.size() + 15) / 16 * 16;
+        W.blob.resize((off + bytes + 15) / 16 * 16);
+        if (bytes) std::memcpy(W.blob.data() + off, src, bytes);
+        return static_cast<int>(off);
+    };
+    put(W.items.data(), W.items.size() * sizeof(WholeItem));
+    W.o_reach = put(W.reach.data(), W.reach.size() * sizeof(WholeReach));
+    W.o_end = put(W.edge_end.data(), W.edge_end.size() * sizeof(short));
+    W.o_edge = put(W.edge_row.data(), W.edge_row.size() * sizeof(int));
+    W.o_rows = put(W.rows.data(), W.rows.size() * sizeof(int));
+    W.o_voff = put(W.value_off.data(), W.value_off.size() * sizeof(int));
+    W.o_roff = put(W.reach_off.data(), W.reach_off.size() * sizeof(int));
 }
 
 int build_plan(const Problem &pb, Plan *out) {
@@ -656,6 +729,18 @@ int build_plan(const Problem &pb, Plan *out) {
                 P.cross_idx[(static_cast<size_t>(t) * np + o) * HS + h] =
                     P.pair_idx[(static_cast<size_t>(o) * 52 + a) * 52 + b];
             }
+
+    // a small heads-up subgame runs whole iterations in one kernel: terminals
+    // of the kinds it serves, and both players' passes within its shared memory
+    if (np == 2 && N <= kSmallNodes) {
+        bool served = true;
+        for (int t = 0; t < 2; ++t)
+            for (int k = 0; k < TK_COUNT; ++k)
+                served = served && (P.term[t][k].empty() || k == TK_SD1 || k == TK_CR1 || k == TK_ZERO);
+        if (served)
+            for (int t = 0; t < 2; ++t)
+                build_whole_pass(P.cfv_levels[t], P.cfv_nlong[t], P.reach_levels[t], P.fr_off, P.fr_items, E, &P.whole[t]);
+    }
 
     double hsum = 0;
     for (int p = 0; p < np; ++p) hsum += P.H[p];

@@ -56,6 +56,8 @@ class Session {
     const CfvItem *cfv_items[SS_MAX_PLAYERS] = {};
     std::vector<std::pair<int, int>> cfv_lv[SS_MAX_PLAYERS];
     TreeRef tree[SS_MAX_PLAYERS] = {};
+    SmallRef small{};         // small heads-up subgames: iterations in one cooperative kernel
+    int small_blocks = 0;     // its grid; 0: the captured iterations run
     const TermItem *term_items[SS_MAX_PLAYERS][TK_COUNT] = {};
     const int *term_heads[SS_MAX_PLAYERS][TK_COUNT] = {};   // null for kinds without P.term_heads
     const int *root_fr[SS_MAX_PLAYERS] = {};
