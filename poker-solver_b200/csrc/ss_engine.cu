@@ -159,7 +159,9 @@ bool host_block_give(void *p) {
 
 
 int Session::init(const Problem &pb, const SolveConfig &cfg) {
-    int rc = build_plan(pb, &P);
+    // the passes of its own iterations: not for a batch's member or a check alone
+    const bool runs = !cfg.batch_member && !cfg.check_only;
+    int rc = build_plan(pb, &P, runs);
     if (rc != SS_OK) return rc;
     if (P.enum_work > kEnumLimitPerIter) {
         set_error("terminals with three or more counted opponents (or multiway showdowns) need " +
@@ -181,15 +183,6 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     CK(cudaSetDevice(device));
     keep_pool_warm(device);
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    if (!cfg.batch_member) {
-        // side streams of the session's own captured iterations (a batch
-        // member's launches are the batch's)
-        CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-        for (int k = 0; k < TK_COUNT; ++k) {
-            CK(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
-            CK(cudaEventCreateWithFlags(&ev_join[k], cudaEventDisableTiming));
-        }
-    }
     const int np = P.np;
     const size_t HS = static_cast<size_t>(P.HS);
     const size_t E = static_cast<size_t>(P.E), N = static_cast<size_t>(P.N);
@@ -358,7 +351,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     c.root_na = P.root_na;
     c.root_frozen = frozen_root;
     c.root_player = P.root_player;
-    if (!cfg.batch_member && !P.whole[0].items.empty() && !P.whole[1].items.empty())
+    if (!P.whole[0].items.empty() && !P.whole[1].items.empty())
         small_blocks = small_solve_blocks(c, &small);
     return reset();
 }
@@ -748,6 +741,7 @@ int solve(const Problem &pb, int iterations, const SolveConfig &cfg, SSOutput *o
 int exploitability(const Problem &pb, const float *avg, double *pct, double *nash, double *br,
                    double *cur, double *z) {
     SolveConfig cfg;
+    cfg.check_only = 1;
     Session *s = nullptr;
     int rc = session_create(pb, cfg, &s);
     if (rc != SS_OK) return rc;

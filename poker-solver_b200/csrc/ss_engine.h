@@ -371,7 +371,8 @@ struct Plan {
     double node_hands = 0;             // num_nodes x sum_p H_p
 };
 
-int build_plan(const Problem &pb, Plan *plan);
+// passes: also the one-launch passes (Plan::tree, Plan::whole)
+int build_plan(const Problem &pb, Plan *plan, bool passes = false);
 
 // 7-card rank of board (num_board == 5) plus two hole cards, reference
 // encoding (src/hand_eval.h:26-35, 138-156); 0 if any card repeats.
@@ -388,6 +389,7 @@ struct SolveConfig {
     float target_exploitability = -1.f;
     int check_every = 50;
     int compute_exploitability = 0;
+    int check_only = 0;      // the session only evaluates profiles
     int batch_member = 0;    // the session only runs inside a batch (no launches of its own iterations)
 };
 

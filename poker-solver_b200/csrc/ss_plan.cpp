@@ -260,7 +260,7 @@ void build_whole_pass(const std::vector<std::vector<CfvItem>> &cfv_levels, const
     W.o_roff = put(W.reach_off.data(), W.reach_off.size() * sizeof(int));
 }
 
-int build_plan(const Problem &pb, Plan *out) {
+int build_plan(const Problem &pb, Plan *out, bool passes) {
     Plan &P = *out;
     if (!validate(pb, P)) return SS_ERR_INVALID;
     const int np = P.np, N = P.N;
@@ -409,7 +409,7 @@ int build_plan(const Problem &pb, Plan *out) {
                 return P.fr_off[it.first_edge + it.na] - P.fr_off[it.first_edge];
             });
         }
-        build_tree_pass(P.cfv_levels[t], P.cfv_nlong[t], P.reach_levels[t], P.fr_off, P.fr_items, &P.tree[t]);
+        if (passes) build_tree_pass(P.cfv_levels[t], P.cfv_nlong[t], P.reach_levels[t], P.fr_off, P.fr_items, &P.tree[t]);
     }
 
     // board and hand tables
@@ -732,7 +732,7 @@ int build_plan(const Problem &pb, Plan *out) {
 
     // a small heads-up subgame runs whole iterations in one kernel: terminals
     // of the kinds it serves, and both players' passes within its shared memory
-    if (np == 2 && N <= kSmallNodes) {
+    if (passes && np == 2 && N <= kSmallNodes) {
         bool served = true;
         for (int t = 0; t < 2; ++t)
             for (int k = 0; k < TK_COUNT; ++k)

@@ -156,6 +156,48 @@ class Session {
                             term_heads[t][k], static_cast<int>(P.term_heads[t][k].size()));
     }
 
+    // The terminal launches of traverser t's pass, their bytes, and the one
+    // with the most work, which stays on the session stream (relative block
+    // times of full-range rivers and turns); returns their number.
+    int launch_kinds(int t, int kinds[TK_COUNT], int *main_k, double by[TK_COUNT]) const {
+        int nk = 0;
+        double main_w = 0;
+        for (int k = 0; k < TK_COUNT; ++k) {
+            const int n = static_cast<int>(P.term[t][k].size());
+            const int lk = light(t, k) ? static_cast<int>(TK_SD1) : k;
+            by[lk] += term_bytes[t][k];
+            if (n == 0 || lk != k) continue;
+            kinds[nk++] = k;
+            const double w = n * (k == TK_SD3 || k == TK_CR3 ? 64.0 : k == TK_SD2 || k == TK_ENUM ? 16.0 : 1.0);
+            if (*main_k < 0 || w > main_w) {
+                *main_k = k;
+                main_w = w;
+            }
+        }
+        return nk;
+    }
+
+    // the side streams and events that a captured iteration forks onto, made
+    // when the first one is captured
+    cudaError_t ensure_side() {
+        cudaError_t e = cudaSuccess;
+        for (int t = 0; t < P.np; ++t) {
+            int kinds[TK_COUNT], main_k = -1;
+            double by[TK_COUNT] = {};
+            const int nk = launch_kinds(t, kinds, &main_k, by);
+            if (nk <= 1) continue;
+            if (!ev_fork) e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
+            for (int i = 0; i < nk && e == cudaSuccess; ++i) {
+                const int k = kinds[i];
+                if (k == main_k || side[k]) continue;
+                e = cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking);
+                if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_join[k], cudaEventDisableTiming);
+            }
+            if (e != cudaSuccess) return e;
+        }
+        return e;
+    }
+
     // traverser t's part of iteration *iter + iter_add
     cudaError_t pass(int t, bool snapshot_root, int iter_add) {
         cudaError_t e = cudaSuccess;
@@ -166,23 +208,10 @@ class Session {
                                          P.H[P.root_player], dsmall, stream);
             if (e != cudaSuccess) return e;
         }
-        // the launches of this pass; the one with the most work stays on the
-        // session stream (relative block times of full-range rivers and turns)
-        int kinds[TK_COUNT], nk = 0, main_k = -1;
-        double main_w = 0, by[TK_COUNT] = {};
-        for (int k = 0; k < TK_COUNT; ++k) {
-            const int n = static_cast<int>(P.term[t][k].size());
-            const int lk = light(t, k) ? static_cast<int>(TK_SD1) : k;
-            by[lk] += term_bytes[t][k];
-            if (n == 0 || lk != k) continue;
-            kinds[nk++] = k;
-            const double w = n * (k == TK_SD3 || k == TK_CR3 ? 64.0 : k == TK_SD2 || k == TK_ENUM ? 16.0 : 1.0);
-            if (main_k < 0 || w > main_w) {
-                main_k = k;
-                main_w = w;
-            }
-        }
-        if (marks || nk <= 1 || !ev_fork) {
+        int kinds[TK_COUNT], main_k = -1;
+        double by[TK_COUNT] = {};
+        const int nk = launch_kinds(t, kinds, &main_k, by);
+        if (marks || nk <= 1) {
             // one kind after the other (the profile times each class)
             for (int i = 0; i < nk; ++i) {
                 const int k = kinds[i];
@@ -239,7 +268,8 @@ class Session {
 
     cudaError_t capture(int iters, bool last, cudaGraphExec_t *exec) {
         cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+        cudaError_t e = ensure_side();
+        if (e == cudaSuccess) e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
         cudaError_t body = cudaSuccess;
         for (int i = 0; i < iters && body == cudaSuccess; ++i) body = iteration(last && i == iters - 1, i + 1);
