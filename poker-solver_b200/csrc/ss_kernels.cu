@@ -2393,6 +2393,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
 // ---------------------------------------------------------------------------
 constexpr int SD2_S = 49;   // row stride of the sweep's card matrices (odd: conflict-free columns)
 constexpr int SD2_N = 48;   // cards a matrix covers (dense indices; a river deck has 47)
+constexpr int SD2_W = (1326 + 31) / 32;   // words of a position mask
+// live positions (of the opponent with more) up to which a sweep takes the sparse form.  A
+// river's 40 three-way showdowns, dense -> sparse form: 66 -> 51 us at 200 hands, 72 -> 70 at
+// 400, 74 -> 82 at 550, 84 -> 125 at all 1,081 (walking masks costs more than testing values)
+constexpr int SD2_SPARSE = 400;
 static_assert(kTermThreads == 256, "the sweep's thread roles assume 256 threads");
 
 // the opponents' reach by rank position; after the sweep the same space holds
@@ -2412,12 +2417,29 @@ template <class T>
 constexpr size_t sd2_smem(int span, int ncomb) {
     return SD2_S * SD2_S * 8 + 2 * SD2_S * SD2_S * sizeof(T) + 4 * 64 * 8 + 8 * 8 + static_cast<size_t>(span) * 32 +
            sd2_reach_bytes<T>(ncomb) + static_cast<size_t>(ncomb) * 2 + static_cast<size_t>(span) * 2 + 16 +
-           13 * 16;
+           2 * SD2_W * 4 + 2 * 48 * 8 + 17 * 16;
 }
 
 struct Sd2State {
     double *P, *u1, *u2, *w, *d, *sc;   // sc: F1, F2, Q, D
+    // the positions where each opponent's reach is not 0 (bit q % 32 of word q / 32): sparse
+    // ranges walk these, and a group where an opponent has none costs it no phase
+    unsigned *on1, *on2;
+    unsigned long long *row1, *row2;    // direct states: the cells of each matrix row that are not 0
 };
+
+// the first position >= q of `on` below hi, or hi (dense: q itself; the caller
+// skips the zeros)
+template <bool SP>
+__device__ __forceinline__ int sd2_next(const unsigned *on, int q, int hi) {
+    if (!SP) return q;
+    while (q < hi) {
+        const unsigned m = on[q >> 5] >> (q & 31);
+        if (m) return min(hi, q + __ffs(static_cast<int>(m)) - 1);
+        q = (q | 31) + 1;
+    }
+    return hi;
+}
 
 __device__ __forceinline__ int sd2_c1(unsigned short e) { return e & 255; }
 __device__ __forceinline__ int sd2_c2(unsigned short e) { return e >> 8; }
@@ -2449,19 +2471,20 @@ __device__ __forceinline__ double sd2_mass(Sd2State st, const T *M1, const T *M2
 // Add the hands of opponent `who` (0 or 1) at rank positions [lo, hi) to the
 // sweep state.  R: that opponent's reach by rank position; Mo: that
 // opponent's matrix, Mx: the other's (symmetric); uo / ux: their card sums.
-template <class T>
+template <bool SP, class T>
 __device__ __forceinline__ void sd2_add(Sd2State st, const unsigned short *dd, const T *R, T *Mo, const T *Mx,
                                         double *uo, const double *ux, int who, int lo, int hi) {
     const int tid = threadIdx.x;
+    const unsigned *on = who == 0 ? st.on1 : st.on2;
     if (tid < 4 * SD2_N) {
         // P = M1 M2: opponent 1's hand {x, y} adds r Mx[y][.] to row x and
         // r Mx[x][.] to row y; opponent 2's adds the same to columns x, y.
         // Thread (part, j) owns column (row) j of the rows (columns) x with
         // x % 4 == part: the four suits of a rank fall to different threads.
         const int part = tid / SD2_N, j = tid - part * SD2_N;
-        for (int q = lo; q < hi; ++q) {
+        for (int q = sd2_next<SP>(on, lo, hi); q < hi; q = sd2_next<SP>(on, q + 1, hi)) {
             const T rt = R[q];
-            if (rt == T(0)) continue;
+            if (!SP && rt == T(0)) continue;
             const double r = static_cast<double>(rt);
             const unsigned short e = dd[q];
             const int x = sd2_c1(e), y = sd2_c2(e);
@@ -2480,9 +2503,9 @@ __device__ __forceinline__ void sd2_add(Sd2State st, const unsigned short *dd, c
         // at x, y
         const int c = tid - 4 * SD2_N;
         double du = 0.0, dd_c = 0.0, dw = 0.0;
-        for (int q = lo; q < hi; ++q) {
+        for (int q = sd2_next<SP>(on, lo, hi); q < hi; q = sd2_next<SP>(on, q + 1, hi)) {
             const T rt = R[q];
-            if (rt == T(0)) continue;
+            if (!SP && rt == T(0)) continue;
             const double r = static_cast<double>(rt);
             const unsigned short e = dd[q];
             const int x = sd2_c1(e), y = sd2_c2(e);
@@ -2505,9 +2528,9 @@ __device__ __forceinline__ void sd2_add(Sd2State st, const unsigned short *dd, c
     } else if (tid == 5 * SD2_N) {
         // F (this opponent's total), Q = sum u1 u2, D = sum d / 2
         double F = st.sc[who], Q = st.sc[2], D = st.sc[3];
-        for (int q = lo; q < hi; ++q) {
+        for (int q = sd2_next<SP>(on, lo, hi); q < hi; q = sd2_next<SP>(on, q + 1, hi)) {
             const T rt = R[q];
-            if (rt == T(0)) continue;
+            if (!SP && rt == T(0)) continue;
             const double r = static_cast<double>(rt);
             const unsigned short e = dd[q];
             const int x = sd2_c1(e), y = sd2_c2(e);
@@ -2536,7 +2559,7 @@ __device__ __forceinline__ void sd2_add(Sd2State st, const unsigned short *dd, c
 // matrices, P = M1 M2 as FP64 3x3 tiles over the 48-card box, the card sums,
 // d = diag P, w = column sums + row sums of P, and the scalars, each summed
 // in a fixed order.  The caller syncs before; this syncs after.
-template <class T>
+template <bool SP, class T>
 __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, const T *R1, const T *R2,
                                                  const unsigned short *dd, int qend) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -2562,6 +2585,7 @@ __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, cons
         M1[i] = T(0);
         M2[i] = T(0);
     }
+    if (SP && tid < SD2_N) st.row1[tid] = st.row2[tid] = 0ull;
     __syncthreads();
     for (int q = tid; q < qend; q += kTermThreads) {
         const unsigned short e = dd[q];
@@ -2570,17 +2594,35 @@ __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, cons
         if (r1 != T(0)) {
             M1[x * SD2_S + y] = r1;
             M1[y * SD2_S + x] = r1;
+            if (SP) {
+                atomicOr(&st.row1[x], 1ull << y);
+                atomicOr(&st.row1[y], 1ull << x);
+            }
         }
         if (r2 != T(0)) {
             M2[x * SD2_S + y] = r2;
             M2[y * SD2_S + x] = r2;
+            if (SP) {
+                atomicOr(&st.row2[x], 1ull << y);
+                atomicOr(&st.row2[y], 1ull << x);
+            }
         }
     }
     __syncthreads();
     {
         const int i0 = (tid >> 4) * 3, j0 = (tid & 15) * 3;
         double acc[3][3] = {};
+        // sparse: without the k whose three cells of M1 or of M2 are 0 (their
+        // terms are exact +0)
+        unsigned long long m = 0ull;
+        if (SP)
+            m = (st.row1[i0] | st.row1[i0 + 1] | st.row1[i0 + 2]) & (st.row2[j0] | st.row2[j0 + 1] | st.row2[j0 + 2]);
         for (int k = 0; k < SD2_N; ++k) {
+            if (SP) {
+                if (!m) break;
+                k = __ffsll(static_cast<long long>(m)) - 1;
+                m &= m - 1;
+            }
             double xs[3], ys[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -2601,17 +2643,20 @@ __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, cons
     if (tid < SD2_N) {
         const int c = tid;
         double u = 0.0;
+#pragma unroll 12
         for (int r = 0; r < SD2_N; ++r) u += static_cast<double>(M1[r * SD2_S + c]);
         st.u1[c] = u;
         st.d[c] = st.P[c * SD2_S + c];
     } else if (tid >= 64 && tid < 64 + SD2_N) {
         const int c = tid - 64;
         double u = 0.0;
+#pragma unroll 12
         for (int r = 0; r < SD2_N; ++r) u += static_cast<double>(M2[r * SD2_S + c]);
         st.u2[c] = u;
     } else if (tid >= 128 && tid < 128 + SD2_N) {
         const int c = tid - 128;
         double w = 0.0;   // (M2 u1)(c) = sum_r P[r][c]
+#pragma unroll 12
         for (int r = 0; r < SD2_N; ++r) w += st.P[r * SD2_S + c];
         st.w[c] = w;
     }
@@ -2619,6 +2664,7 @@ __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, cons
     if (tid < SD2_N) {
         const int c = tid;
         double w = 0.0;   // (M1 u2)(c) = sum_r P[c][r]
+#pragma unroll 12
         for (int r = 0; r < SD2_N; ++r) w += st.P[c * SD2_S + r];
         st.w[c] += w;
     } else if (warp == kTermThreads / 32 - 1) {
@@ -2650,7 +2696,7 @@ __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, cons
 // holds any group hand.  Eight lanes per hand, each taking every eighth group
 // position, combined in a fixed order.  Classes of position q at
 // cls[4 (q - base)]: A, T1, opponent 2 present, (C).
-template <class T>
+template <bool SP, class T>
 __device__ __forceinline__ void sd2_phase_a(Sd2State st, const T *M1, const T *M2, const T *R1, const T *R2,
                                             const unsigned short *dd, const short *pt, double *cls, int base,
                                             int lo, int hi) {
@@ -2670,10 +2716,24 @@ __device__ __forceinline__ void sd2_phase_a(Sd2State st, const T *M1, const T *M
             const double u1a = st.u1[a], u1b = st.u1[b], u2a = st.u2[a], u2b = st.u2[b];
             const double m1ab = static_cast<double>(M1[a * SD2_S + b]), m2ab = static_cast<double>(M2[a * SD2_S + b]);
             double dle = 0.0, del = 0.0;
-            for (int q2 = lo + l8; q2 < hi; q2 += 8) {
+            // this lane's group positions: lo + l8 and every eighth after it
+            // (sparse: those of them where an opponent has reach, 32 at a time)
+            const unsigned eighth = 0x01010101u << ((lo + l8) & 7);
+            int base2 = lo & ~31, q2 = lo + l8 - 8;
+            unsigned m = SP ? (st.on1[base2 >> 5] | st.on2[base2 >> 5]) & eighth & (~0u << (lo & 31)) : 0u;
+            for (;;) {
+                if (SP) {
+                    while (!m && (base2 += 32) < hi) m = (st.on1[base2 >> 5] | st.on2[base2 >> 5]) & eighth;
+                    if (!m) break;
+                    q2 = base2 + __ffs(static_cast<int>(m)) - 1;
+                    m &= m - 1;
+                } else {
+                    q2 += 8;
+                }
+                if (q2 >= hi) break;
                 const T r1 = R1[q2], r2 = R2[q2];
                 any2 = any2 || r2 != T(0);
-                if (r1 == T(0) && r2 == T(0)) continue;
+                if (!SP && r1 == T(0) && r2 == T(0)) continue;
                 const unsigned short e2 = dd[q2];
                 const int x = sd2_c1(e2), y = sd2_c2(e2);
                 if (x == a || x == b || y == a || y == b) continue;
@@ -2709,6 +2769,60 @@ __device__ __forceinline__ void sd2_phase_mass(Sd2State st, const T *M1, const T
                                                const short *pt, double *cls, int base, int lo, int hi, int k) {
     for (int q = lo + threadIdx.x; q < hi; q += kTermThreads)
         if (pt[q - base] >= 0) cls[4 * (q - base) + k] = sd2_mass(st, M1, M2, sd2_c1(dd[q]), sd2_c2(dd[q]));
+}
+
+// The sweep over a block's runs: segments [s0, s1), the first at `sg`, then the
+// state of every hand.
+// Groups are short and their phases wait on one another, so a block's time is
+// its barriers and the serial walk over a group's hands, not arithmetic.  With
+// few live hands (SP: at most SD2_SPARSE) most groups hold none of an opponent:
+// such a group takes no phase and no barrier, walks touch live positions only,
+// and the products skip terms that are exact zeros.  The order of what is
+// summed is the same either way, so both give the same bits.  207 three-way
+// showdowns of a 4-player river with 66 of 101 hands live: 300 -> 129 us.
+template <bool SP, class T>
+__device__ __forceinline__ void sd2_run(const Sd2State &st, T *M1, T *M2, const T *R1, const T *R2,
+                                        const unsigned short *dd, const short *pt, double *cls,
+                                        const int4 *__restrict__ seg4, int4 sg, int s0, int s1, int run_hi, int nc) {
+    const int run_lo = sg.x;
+    // the runs start from the state of every hand ranked below them
+    sd2_direct_state<SP>(st, M1, M2, R1, R2, dd, run_lo);
+
+    // segment entries come from global memory a step ahead of their use
+    int4 nsg = s0 + 1 < s1 ? __ldg(seg4 + s0 + 1) : make_int4(0, 0, 0, 0);
+    // reads: the state has been read since the last barrier, so the next hands
+    // added wait for one
+    bool reads = false;
+    if (sg.z) {
+        sd2_phase_a<SP>(st, M1, M2, R1, R2, dd, pt, cls, run_lo, sg.x, sg.y);
+        reads = true;
+    }
+    for (int si = s0; si < s1; ++si) {
+        const int lo = sg.x, hi = sg.y;
+        const bool has = sg.z != 0, nhas = si + 1 < s1 && nsg.z != 0;
+        const bool any1 = sd2_next<SP>(st.on1, lo, hi) < hi, any2 = sd2_next<SP>(st.on2, lo, hi) < hi;
+        if ((any1 || any2) && reads) {
+            __syncthreads();
+            reads = false;
+        }
+        if (any1) {
+            sd2_add<SP>(st, dd, R1, M1, M2, st.u1, st.u2, 0, lo, hi);
+            __syncthreads();
+        }
+        if (any2) {
+            sd2_add<SP>(st, dd, R2, M2, M1, st.u2, st.u1, 1, lo, hi);
+            __syncthreads();
+        }
+        // C of this group and A of the next group: the same state
+        if (has) sd2_phase_mass(st, M1, M2, dd, pt, cls, run_lo, lo, hi, 3);
+        if (nhas) sd2_phase_a<SP>(st, M1, M2, R1, R2, dd, pt, cls, run_lo, nsg.x, nsg.y);
+        reads = reads || has || nhas;
+        sg = nsg;   // the next segment's entry is loaded a full step before its use
+        if (si + 2 < s1) nsg = __ldg(seg4 + si + 2);
+    }
+    if (reads) __syncthreads();
+    // the whole state, unless these runs end the rank order and have it
+    if (run_hi < nc) sd2_direct_state<SP>(st, M1, M2, R1, R2, dd, nc);
 }
 
 // One block per 2^lgm consecutive runs of a terminal's sweep (grid: items x
@@ -2773,6 +2887,10 @@ __global__ void __launch_bounds__(kTermThreads, 4) k_term_sd2(DevCtx c0, const D
     st.w = cv.take<double>(64);
     st.d = cv.take<double>(64);
     st.sc = cv.take<double>(8);
+    st.row1 = cv.take<unsigned long long>(SD2_N);
+    st.row2 = cv.take<unsigned long long>(SD2_N);
+    st.on1 = cv.take<unsigned>(SD2_W);
+    st.on2 = cv.take<unsigned>(SD2_W);
     double *cls = cv.take<double>(4 * span);   // per position of the run: A, T1, opponent 2 present, C
     char *rbuf = cv.take<char>(static_cast<int>(sd2_reach_bytes<T>(nc)));
     T *R1 = reinterpret_cast<T *>(rbuf);
@@ -2783,6 +2901,7 @@ __global__ void __launch_bounds__(kTermThreads, 4) k_term_sd2(DevCtx c0, const D
 
     // opponents' reach and the cards by rank position, and the last position
     // holding positive reach of either opponent
+    bool odd = false;   // a reach that is not finite: no term may be skipped
     if (tid == 0) *last_pos = -1;
     if (tid < 64) {
         st.u1[tid] = 0.0;
@@ -2797,9 +2916,17 @@ __global__ void __launch_bounds__(kTermThreads, 4) k_term_sd2(DevCtx c0, const D
         const int *pa = pos_hand + static_cast<size_t>(o1) * nc, *pb = pos_hand + static_cast<size_t>(o2) * nc;
         int lp = -1;
 #pragma unroll 4
-        for (int q = tid; q < nc; q += kTermThreads) {
-            const int ha = __ldg(pa + q), hb = __ldg(pb + q);
+        for (int q0 = 0; q0 < nc; q0 += kTermThreads) {
+            const int q = q0 + tid;
+            const int ha = q < nc ? __ldg(pa + q) : -1, hb = q < nc ? __ldg(pb + q) : -1;
             const T x = ha >= 0 ? ra[ha] : T(0), y = hb >= 0 ? rb[hb] : T(0);
+            odd = odd || !(x - x == T(0)) || !(y - y == T(0));
+            const unsigned m1 = __ballot_sync(0xffffffffu, x != T(0)), m2 = __ballot_sync(0xffffffffu, y != T(0));
+            if (q >= nc) continue;
+            if (lane == 0) {
+                st.on1[q >> 5] = m1;
+                st.on2[q >> 5] = m2;
+            }
             R1[q] = x;
             R2[q] = y;
             dd[q] = static_cast<unsigned short>(cb[q].d1 | (cb[q].d2 << 8));
@@ -2809,35 +2936,18 @@ __global__ void __launch_bounds__(kTermThreads, 4) k_term_sd2(DevCtx c0, const D
         const int *ph_t = pos_hand + static_cast<size_t>(trav) * nc + run_lo;
         for (int k = tid; k < run_hi - run_lo; k += kTermThreads) pt[k] = static_cast<short>(__ldg(ph_t + k));
     }
-    __syncthreads();
-    // this run starts from the state of every hand ranked below it
-    sd2_direct_state(st, M1, M2, R1, R2, dd, run_lo);
+    odd = __syncthreads_or(odd);
+    int live = 0;
+    for (int i = lane; i < (nc + 31) / 32; i += 32) live += max(__popc(st.on1[i]), __popc(st.on2[i]));
+    const bool sparse = !odd && __reduce_add_sync(0xffffffffu, live) <= SD2_SPARSE;
+    if (sparse)
+        sd2_run<true>(st, M1, M2, R1, R2, dd, pt, cls, seg4, sg, s0, s1, run_hi, nc);
+    else
+        sd2_run<false>(st, M1, M2, R1, R2, dd, pt, cls, seg4, sg, s0, s1, run_hi, nc);
 
-    // segment entries come from global memory a step ahead of their use
-    int4 nsg = s0 + 1 < s1 ? __ldg(seg4 + s0 + 1) : make_int4(0, 0, 0, 0);
-    if (sg.z) {
-        sd2_phase_a(st, M1, M2, R1, R2, dd, pt, cls, run_lo, sg.x, sg.y);
-        __syncthreads();
-    }
-    for (int si = s0; si < s1; ++si) {
-        const int lo = sg.x, hi = sg.y;
-        const bool has = sg.z != 0, nhas = si + 1 < s1 && nsg.z != 0;
-        sd2_add(st, dd, R1, M1, M2, st.u1, st.u2, 0, lo, hi);
-        __syncthreads();
-        sd2_add(st, dd, R2, M2, M1, st.u2, st.u1, 1, lo, hi);
-        __syncthreads();
-        // C of this group and A of the next group: the same state
-        if (has) sd2_phase_mass(st, M1, M2, dd, pt, cls, run_lo, lo, hi, 3);
-        if (nhas) sd2_phase_a(st, M1, M2, R1, R2, dd, pt, cls, run_lo, nsg.x, nsg.y);
-        if (has || nhas) __syncthreads();
-        sg = nsg;   // the next segment's entry is loaded a full step before its use
-        if (si + 2 < s1) nsg = __ldg(seg4 + si + 2);
-    }
-
-    // all hands added (directly, unless this run ends the rank order): Z, and
-    // the exact positive-pair count for hands whose mass is within the error
-    // bound of zero (masks over the 47-card matrices, in the reach space)
-    if (run_hi < nc) sd2_direct_state(st, M1, M2, R1, R2, dd, nc);
+    // all hands added: Z, and the exact positive-pair count for hands whose
+    // mass is within the error bound of zero (masks over the 47-card matrices,
+    // in the reach space)
     ulonglong2 *Bm = reinterpret_cast<ulonglong2 *>(rbuf);
     Cr2Cnt *cnt = reinterpret_cast<Cr2Cnt *>(rbuf + 53 * sizeof(ulonglong2));
     Cr2Scalars *sc2 = reinterpret_cast<Cr2Scalars *>(rbuf + 53 * sizeof(ulonglong2) + 53 * sizeof(Cr2Cnt));
