@@ -235,26 +235,53 @@ template <class T>
 __device__ __forceinline__ void gather_dev(int tid, const Opp3<T> &in, const Tables &t, const int *pos1, int lo1,
                                            int hi1, const int *pos2, int lo2, int hi2) {
     const int warp = tid >> 5, lane = tid & 31;
-    for (int c = warp; c < kS; c += 8) {
-        unsigned long long ma = 0ull, mb = 0ull;
-        for (int half = 0; half < 2; ++half) {
-            const int e = half * 32 + lane;
-            double a = 0.0, b = 0.0;
-            if (e < kS && c < in.deck && e < in.deck) {
-                const int j1 = in.pair1[c * 52 + e], j2 = in.pair2[c * 52 + e];
-                if (j1 < in.HS && (!pos1 || (pos1[j1] >= lo1 && pos1[j1] < hi1))) a = static_cast<double>(in.r1[j1]);
-                if (j2 < in.HS && (!pos2 || (pos2[j2] >= lo2 && pos2[j2] < hi2))) b = static_cast<double>(in.r2[j2]);
+    // four rows at a time, each kind of load for all of them before the next:
+    // two waits on memory per four rows, where half rows one by one made a
+    // build of 22 K cycles wait on memory for most of them
+    constexpr int kR = 4;
+    for (int c0 = warp; c0 < kS; c0 += 8 * kR) {
+        int j1[kR][2], j2[kR][2], q1[kR][2], q2[kR][2];
+        T a[kR][2], b[kR][2];
+#pragma unroll
+        for (int i = 0; i < kR; ++i)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int c = c0 + 8 * i, e = half * 32 + lane;
+                const bool on = c < in.deck && e < in.deck;
+                j1[i][half] = on ? in.pair1[c * 52 + e] : in.HS;
+                j2[i][half] = on ? in.pair2[c * 52 + e] : in.HS;
             }
-            if (e < kS) {
-                t.A[c * kS + e] = a;
-                t.B[c * kS + e] = b;
+#pragma unroll
+        for (int i = 0; i < kR; ++i)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const bool on1 = j1[i][half] < in.HS, on2 = j2[i][half] < in.HS;
+                a[i][half] = on1 ? in.r1[j1[i][half]] : T(0);
+                b[i][half] = on2 ? in.r2[j2[i][half]] : T(0);
+                q1[i][half] = pos1 && on1 ? pos1[j1[i][half]] : lo1;
+                q2[i][half] = pos2 && on2 ? pos2[j2[i][half]] : lo2;
             }
-            ma |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, a > 0.0)) << (32 * half);
-            mb |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, b > 0.0)) << (32 * half);
-        }
-        if (lane == 0) {
-            t.mA[c] = ma;
-            t.mB[c] = mb;
+#pragma unroll
+        for (int i = 0; i < kR; ++i) {
+            const int c = c0 + 8 * i;
+            if (c >= kS) break;
+            unsigned long long ma = 0ull, mb = 0ull;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int e = half * 32 + lane;
+                const double x = !pos1 || (q1[i][half] >= lo1 && q1[i][half] < hi1) ? static_cast<double>(a[i][half]) : 0.0;
+                const double y = !pos2 || (q2[i][half] >= lo2 && q2[i][half] < hi2) ? static_cast<double>(b[i][half]) : 0.0;
+                if (e < kS) {
+                    t.A[c * kS + e] = x;
+                    t.B[c * kS + e] = y;
+                }
+                ma |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, x > 0.0)) << (32 * half);
+                mb |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, y > 0.0)) << (32 * half);
+            }
+            if (lane == 0) {
+                t.mA[c] = ma;
+                t.mB[c] = mb;
+            }
         }
     }
 }
@@ -571,7 +598,8 @@ SSB_CR3_HD void hand_mass_cls(int a, int b, const Tables &t, const int *p3, int 
 // (no class of a pair uses them).  k_term_sd3 spreads a tie group's hands
 // and these slices over its warps; slices combined in a fixed order give the
 // same sums up to the order of the additions.
-SSB_CR3_HD void hand_mass_cls_slice(int a, int b, const Tables &t, const int *p3, int lo, int hi, long long k0,
+template <class Pos>
+SSB_CR3_HD void hand_mass_cls_slice(int a, int b, const Tables &t, const Pos *p3, int lo, int hi, long long k0,
                                     long long kstep, double out[2], long long cnt[2], bool want_count) {
     const HandPart hp = hand_part(a, b, t);
     HandCount hc{};
@@ -706,8 +734,9 @@ SSB_CR3_HD void one_opp_avoid6(const double *M, const double *u, const unsigned 
 // L1 mass, EE enumerates E1 x E2.  Third-opponent entries k0, k0 + kstep, ...
 // below hi, split by class as in hand_mass_cls_slice; a term without a tuple
 // adds nothing, so a class whose count is 0 has mass exactly 0.
+template <class Pos>
 SSB_CR3_HD void e_pair_slice(int pr, int a, int b, const Tables &t, const EHand *E1, int n1, const EHand *E2, int n2,
-                             const int *p3, int lo, int hi, long long k0, long long kstep, double out[2],
+                             const Pos *p3, int lo, int hi, long long k0, long long kstep, double out[2],
                              long long cnt[2]) {
     out[0] = out[1] = 0.0;
     cnt[0] = cnt[1] = 0;

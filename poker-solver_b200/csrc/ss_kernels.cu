@@ -3281,14 +3281,24 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
 }
 
 // Four-way showdowns (three live opponents): the traverser's class masses
-// (ss_cr3.cuh) in FP64.  One block per (terminal, 256 rank positions), one
-// thread per position (the traverser's hand there, if any).  The block
-// builds the tables of the first two opponents' full matrices once (every
-// tuple's mass, for the loss class and the exact zero), then walks the tie
-// groups that meet its positions and, for a group holding a traverser hand,
-// rebuilds them for the four pairs of the opponents' weaker / tying parts;
-// the group's threads add the third opponent's hands by class.  A class
-// mass within rounding of 0 takes its exact tuple count (0: exactly 0).
+// (ss_cr3.cuh) in FP64.  One block per (terminal, 256 rank positions).  The
+// block builds the tables of the first two opponents' full matrices once
+// (every tuple's mass, for the loss class and the exact zero), then walks the
+// tie groups that hold one of its traverser hands with the tables of the
+// weaker parts, and adds the third opponent's hands by class.  A class mass
+// within rounding of 0 takes its exact tuple count (0: exactly 0).
+//
+// A block is a chain of short phases between barriers, so what bounds it is
+// their latency: loads that wait on loads, and warps with nothing to do.  So
+// the block's rank positions (hands, reach, cards, groups) are read once into
+// shared memory, the table gathers have all their loads in flight together,
+// and a warp takes one (hand, pair of classes) at a time, of the hands that
+// are there and not of the positions, all pairs that read the same tables in
+// one round.  Blocks come chunk by chunk: the last chunk, the shortest, runs
+// last.  Measured per launch, 4-player rivers: 73 terminals with 66 of 101
+// hands live 410 -> 143 us, 13 with 390 of 600 live 1.9 -> 1.2 ms, 9 at full
+// ranges 4.1 -> 3.4 ms; before, one thread listed the third opponent's hands
+// and warps took one pair of classes at a time, position by position.
 constexpr int kSd3Positions = 1081;   // C(47, 2): rank positions on every river board
 constexpr int kSd3Warps = kTermThreads / 32;
 // a tie group whose tying parts hold at most this many positive-reach hands
@@ -3297,13 +3307,17 @@ constexpr int kSd3Warps = kTermThreads / 32;
 constexpr int kSd3MaxE = 64;
 // a table build in units of one D2 evaluation (the sparse steps' cost model)
 constexpr double kSd3BuildCost = 3000.0;
+template <class T>
 constexpr size_t sd3_smem(int HS) {
     return (4 * cr3::kS * cr3::kS + 4 * cr3::kS + 8) * sizeof(double) + 4 * cr3::kS * sizeof(int) +
            2 * cr3::kS * sizeof(unsigned long long) + 8 * sizeof(long long) +
-           static_cast<size_t>(HS) * (sizeof(double) + sizeof(unsigned short)) + 16 * 16 +
-           static_cast<size_t>(HS) * sizeof(int) + 16 + 3 * kTermThreads +
-           2 * kSd3Warps * (sizeof(double) + sizeof(long long)) + 64 + 2 * kSd3MaxE * sizeof(cr3::EHand) + 16 + 64;
+           static_cast<size_t>(HS) * (sizeof(double) + 2 * sizeof(short)) +
+           kTermThreads * (2 * sizeof(T) + 3 * sizeof(short) + 3) +
+           4 * kSd3Warps * (sizeof(double) + sizeof(long long)) + 2 * kSd3MaxE * sizeof(cr3::EHand) +
+           (4 * kSd3Warps + 4) * sizeof(int) + 4 * 16;
 }
+static_assert(2 * kSd3MaxE * sizeof(cr3::EHand) == kTermThreads * sizeof(double), "the masses share the lists' space");
+static_assert(sd3_smem<float>(kMaxHS) <= (228 * 1024 - 2 * 1024) / 2, "two blocks per SM");
 
 template <class T>
 __global__ void __launch_bounds__(kTermThreads, 2) k_term_sd3(DevCtx c0, const DevCtx *__restrict__ ctxs,
@@ -3311,15 +3325,16 @@ __global__ void __launch_bounds__(kTermThreads, 2) k_term_sd3(DevCtx c0, const D
                                                              int trav) {
     wait_prior_grid();
     extern __shared__ __align__(16) char smem[];
-    const int it = blockIdx.x / nchunk;
-    const int ch = blockIdx.x - it * nchunk;
+    const int n_items = gridDim.x / nchunk;
+    const int ch = blockIdx.x / n_items;
+    const int it = blockIdx.x - ch * n_items;
     const TermItem I = items[it];
     if (retired(ctxs, I.sg)) return;
     const DevCtx &c = ctxs ? ctxs[I.sg] : c0;
     const int HS = c.HS;
     if (HS > c0.HS || c.deck > cr3::kS - 1) return;
     const size_t hs = static_cast<size_t>(HS);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     T *out = val_rows<T>(c) + static_cast<size_t>(I.node) * hs;
     const int *tpos = c.sd_pos + static_cast<size_t>(trav) * hs;
     // the first chunk writes the hands without a rank position and the padding
@@ -3348,21 +3363,33 @@ __global__ void __launch_bounds__(kTermThreads, 2) k_term_sd3(DevCtx c0, const D
     t.mA = cv.take<unsigned long long>(cr3::kS);
     t.mB = cv.take<unsigned long long>(cr3::kS);
     t.isc = cv.take<long long>(8);
-    t.r3 = cv.take<double>(HS);
-    t.xy = cv.take<unsigned short>(HS);
-    int *p3 = cv.take<int>(HS);
-    // per warp: the two class partials of one (hand, slice) of a tie group
-    double *part = cv.take<double>(2 * kSd3Warps);
-    long long *partc = cv.take<long long>(2 * kSd3Warps);
-    // the traverser hand at each of the block's rank positions
+    // per warp: the two class partials of one (hand, slice); two sets, so that
+    // a round's sums are read while the next round writes
+    double *part = cv.take<double>(4 * kSd3Warps);
+    long long *partc = cv.take<long long>(4 * kSd3Warps);
+    // the block's rank positions: the first two opponents' reach (0: no hand)
+    // and dense cards, the tie group's end; the traverser's dense cards
+    T *pr1 = cv.take<T>(kTermThreads);
+    T *pr2 = cv.take<T>(kTermThreads);
+    unsigned short *pxy1 = cv.take<unsigned short>(kTermThreads);
+    unsigned short *pxy2 = cv.take<unsigned short>(kTermThreads);
+    short *phi = cv.take<short>(kTermThreads);
     unsigned char *ga = cv.take<unsigned char>(kTermThreads);
     unsigned char *gb = cv.take<unsigned char>(kTermThreads);
-    unsigned char *ghas = cv.take<unsigned char>(kTermThreads);
+    // the positions that hold a traverser hand: in order, as a mask, and how
+    // many before each of its words
+    unsigned char *gl = cv.take<unsigned char>(kTermThreads);
+    unsigned *hm = cv.take<unsigned>(kSd3Warps + 1);
+    int *hp = cv.take<int>(kSd3Warps + 1);
+    int *wc = cv.take<int>(kSd3Warps);
     // the current tie group's tying hands of the first two opponents, and their numbers
     cr3::EHand *elist1 = cv.take<cr3::EHand>(kSd3MaxE);
     cr3::EHand *elist2 = cv.take<cr3::EHand>(kSd3MaxE);
+    double *tot = reinterpret_cast<double *>(elist1);   // (before the groups) every tuple's mass, by position
     int *en = cv.take<int>(2);
-    const int lane = tid & 31, warp = tid >> 5;
+    t.r3 = cv.take<double>(HS);   // (the third opponent's range may hold a combo twice)
+    t.xy = cv.take<unsigned short>(HS);
+    short *p3 = cv.take<short>(HS);
     const T *reach = reach_rows<T>(c);
     const int o1 = I.opp_player[0], o2 = I.opp_player[1], o3 = I.opp_player[2];
     cr3::Opp3<T> in;
@@ -3375,65 +3402,189 @@ __global__ void __launch_bounds__(kTermThreads, 2) k_term_sd3(DevCtx c0, const D
     in.H3 = c.H[o3];
     in.HS = HS;
     in.deck = c.deck;
+    const int *code1 = c.hand_code + static_cast<size_t>(o1) * hs, *code2 = c.hand_code + static_cast<size_t>(o2) * hs;
+    const int *ph1 = c.pos_hand + static_cast<size_t>(o1) * nc, *ph2 = c.pos_hand + static_cast<size_t>(o2) * nc;
     const int *posA = c.sd_pos + static_cast<size_t>(o1) * hs;
     const int *posB = c.sd_pos + static_cast<size_t>(o2) * hs;
     const int *pre1 = c.pos_prefix + static_cast<size_t>(o1) * (nc + 1);
     const int *pre2 = c.pos_prefix + static_cast<size_t>(o2) * (nc + 1);
-    // this thread's rank position and the traverser's hand there
+    // this thread's rank position: the traverser's hand there, the first two
+    // opponents' hands, the tie group
     cr3::Sd3Thread st;
     cr3::sd3_thread_init(q0 + tid, qend, c.pos_hand + static_cast<size_t>(trav) * nc,
                          c.hand_code + static_cast<size_t>(trav) * hs, c.sd_combo, st);
-    ga[tid] = static_cast<unsigned char>(st.a);
-    gb[tid] = static_cast<unsigned char>(st.b);
-    ghas[tid] = st.h >= 0;
+    {
+        const int q = q0 + tid;
+        const int h1 = q < qend ? ph1[q] : -1, h2 = q < qend ? ph2[q] : -1;
+        pr1[tid] = h1 >= 0 ? in.r1[h1] : T(0);
+        pr2[tid] = h2 >= 0 ? in.r2[h2] : T(0);
+        const int e1 = h1 >= 0 ? code1[h1] : 0, e2 = h2 >= 0 ? code2[h2] : 0;
+        pxy1[tid] = static_cast<unsigned short>(((e1 >> 20) & 63) | (((e1 >> 26) & 63) << 8));
+        pxy2[tid] = static_cast<unsigned short>(((e2 >> 20) & 63) | (((e2 >> 26) & 63) << 8));
+        phi[tid] = q < qend ? static_cast<short>(c.sd_combo[q].hi) : 0;
+        ga[tid] = static_cast<unsigned char>(st.a);
+        gb[tid] = static_cast<unsigned char>(st.b);
+        const unsigned m = __ballot_sync(0xffffffffu, st.h >= 0);
+        if (lane == 0) hm[warp] = m;
+        if (tid == 0) hm[kSd3Warps] = 0u;
+    }
+    __syncthreads();
+    if (tid <= kSd3Warps) {
+        int n = 0;
+        for (int w = 0; w < tid; ++w) n += __popc(hm[w]);
+        hp[tid] = n;
+    }
+    __syncthreads();
+    const int nhand = hp[kSd3Warps];
+    if (nhand == 0) return;   // no row of this block's positions to write
+    // how many traverser hands the block has below its position j
+    auto rank_at = [&](int j) { return hp[j >> 5] + __popc(hm[j >> 5] & ((1u << (j & 31)) - 1u)); };
+    const int myrank = rank_at(tid);
+    if (st.h >= 0) gl[myrank] = static_cast<unsigned char>(tid);
+    // the third opponent's positive-reach live hands in hand order
+    int n3 = 0;
+    for (int base = 0; base < in.H3; base += kTermThreads) {
+        const int h = base + tid;
+        int code = 0x10000, p = -1;
+        T r = T(0);
+        if (h < in.H3) {
+            code = in.code3[h];
+            p = c.sd_pos[static_cast<size_t>(o3) * hs + h];
+            r = in.r3[h];
+        }
+        const bool ok = !(code & 0x10000) && p >= 0 && r > T(0);
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        if (lane == 0) wc[warp] = __popc(m);
+        __syncthreads();
+        int at = n3 + __popc(m & ((1u << lane) - 1u));
+        for (int w = 0; w < kSd3Warps; ++w) {
+            if (w < warp) at += wc[w];
+            n3 += wc[w];
+        }
+        if (ok) {
+            t.r3[at] = static_cast<double>(r);
+            t.xy[at] = static_cast<unsigned short>(((code >> 20) & 63) | (((code >> 26) & 63) << 8));
+            p3[at] = static_cast<short>(p);
+        }
+        __syncthreads();
+    }
+    if (tid == 0) t.isc[4] = n3;
     constexpr int kAll = 1 << 30;
-    auto build = [&](int lo1, int hi1, int lo2, int hi2) {
+    auto build = [&](int lo1, int hi1, int lo2, int hi2, bool first) {
         cr3::gather_dev(tid, in, t, posA, lo1, hi1, posB, lo2, hi2);
         __syncthreads();
+        if (first && tid == kTermThreads - 1) {   // (this warp has no part of the product)
+            double f3 = 0.0;
+#pragma unroll 8
+            for (int k = 0; k < n3; ++k) f3 += t.r3[k];
+            t.sc[4] = f3;
+        }
         cr3::build_step1(tid, t);
         __syncthreads();
         cr3::build_step2(tid, t);
         __syncthreads();
     };
-    cr3::compact_third(tid, in, t, c.sd_pos + static_cast<size_t>(o3) * hs, p3);
-    build(0, kAll, 0, kAll);
-    cr3::sd3_thread_total(st, t, p3);
+    build(0, kAll, 0, kAll, true);
+    // Every tuple's mass per traverser hand, the third opponent's hands added
+    // in their order: `lanes` threads per hand evaluate as many of its terms,
+    // then each adds all of them in turn.
+    {
+        const double zb = cr3::zero_bound(t);
+        int lanes = 32;
+        while (lanes > 1 && lanes * nhand > kTermThreads) lanes >>= 1;
+        const int hc = tid / lanes, l = tid - hc * lanes;
+        const bool on = hc < nhand;
+        const int j = on ? gl[hc] : 0, a = ga[j], b = gb[j];
+        const cr3::HandPart part_ab = cr3::hand_part(a, b, t);
+        double sum = 0.0;
+        for (int k0 = 0; k0 < n3; k0 += lanes) {
+            const int k = k0 + l;
+            double v = 0.0;
+            if (on && k < n3) {
+                const int x = t.xy[k] & 0xff, y = t.xy[k] >> 8;
+                if (x != a && x != b && y != a && y != b) v = cr3::d2_at(part_ab, a, b, x, y, t);
+            }
+            if (lanes == 1) {
+                sum = fma(t.r3[k0], v, sum);
+            } else {
+                for (int i = 0; i < lanes; ++i) {
+                    const double vi = __shfl_sync(0xffffffffu, v, i, lanes);
+                    if (k0 + i < n3) sum = fma(t.r3[k0 + i], vi, sum);
+                }
+            }
+        }
+        const bool near = on && fabs(sum) <= zb;
+        if (__any_sync(0xffffffffu, near)) {
+            long long n = 0;
+            if (near) {
+                const cr3::HandCount cab = cr3::hand_count_part(a, b, t);
+                for (int k = l; k < n3; k += lanes) {
+                    const int x = t.xy[k] & 0xff, y = t.xy[k] >> 8;
+                    if (x != a && x != b && y != a && y != b) n += cr3::c2_at(cab, a, b, x, y, t);
+                }
+            }
+            for (int o = lanes >> 1; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+            if (near && n == 0) sum = 0.0;
+        }
+        if (on && l == 0) tot[j] = sum;
+    }
     __syncthreads();
-    // The tie groups meeting [q0, qend), the same walk in every thread.  For
-    // each of a group's four pairs, its hands' class masses are sums over the
-    // third opponent's list: the group's hands and slices of that list are
-    // spread over the block's warps (per warps per hand, lanes splitting a
-    // slice), and each hand's owner thread combines its warps' partials in
-    // warp order.  A mass within rounding of 0 takes the exact tuple count
-    // (a second pass of the same shape over the 0/1 tables).
+    st.total = tot[tid];   // written, and used, where st.h >= 0
+    // The tie groups meeting [q0, qend), the same walk in every thread.  A
+    // class mass of a (hand, pair of the first two opponents' parts) is a sum
+    // over the third opponent's list: slices of that list over `per` warps,
+    // lanes splitting a slice, and the hand's owner thread combines its warps'
+    // partials in warp order.
     // the weaker parts' tables (positions [0, t_hi) of the first two
     // opponents), grown group by group while the groups' tying parts are short
     bool t_valid = false;
     int t_hi = 0;
+    int buf = 0;
+    int glo = c.sd_combo[q0].lo;   // the first group may begin below the block's positions
     for (int g = q0; g < qend;) {
-        const int lo = c.sd_combo[g].lo, hi = c.sd_combo[g].hi;
-        const bool mine = st.h >= 0 && st.glo == lo;
-        const int nmine = __syncthreads_count(mine);   // the traverser's hands of this group in the block
+        const int lo = glo, hi = phi[g - q0];
+        glo = hi;
+        const int j0 = max(lo, q0) - q0, ng = min(hi, qend) - q0 - j0;
+        const int k0 = rank_at(j0), nmine = rank_at(j0 + ng) - k0;   // the block's traverser hands in the group
+        if (k0 == nhand) break;   // none here or above
+        if (nmine == 0 && !t_valid) {
+            g = hi;
+            continue;
+        }
+        const int mine_at = st.h >= 0 && st.glo == lo ? myrank - k0 : -1;   // this thread's hand among them
         const bool any = nmine > 0;
+        __syncthreads();
         // the group's tying hands of the first two opponents with positive
         // reach, in rank order (warp 0: first opponent, warp 1: second)
         if (warp < 2) {
-            const int *ph = c.pos_hand + static_cast<size_t>(warp == 0 ? o1 : o2) * nc;
+            const int *ph = warp == 0 ? ph1 : ph2;
             const T *rr = warp == 0 ? in.r1 : in.r2;
-            const int *code = c.hand_code + static_cast<size_t>(warp == 0 ? o1 : o2) * hs;
+            const int *code = warp == 0 ? code1 : code2;
+            const T *pr = warp == 0 ? pr1 : pr2;
+            const unsigned short *pxy = warp == 0 ? pxy1 : pxy2;
             cr3::EHand *E = warp == 0 ? elist1 : elist2;
             int n = 0;
             for (int base = lo; base < hi; base += 32) {
                 const int q = base + lane;
-                const int hh = q < hi ? ph[q] : -1;
-                const T rv = hh >= 0 ? rr[hh] : T(0);
-                const bool ok = hh >= 0 && rv > T(0);
+                T rv = T(0);
+                int x = 0, y = 0;
+                if (q >= q0 && q < qend) {
+                    rv = q < hi ? pr[q - q0] : T(0);
+                    x = pxy[q - q0] & 0xff;
+                    y = pxy[q - q0] >> 8;
+                } else {   // a group reaching past the block's positions
+                    const int hh = q < hi ? ph[q] : -1;
+                    if (hh >= 0) {
+                        rv = rr[hh];
+                        const int hc = code[hh];
+                        x = (hc >> 20) & 63;
+                        y = (hc >> 26) & 63;
+                    }
+                }
+                const bool ok = rv > T(0);
                 const unsigned bal = __ballot_sync(0xffffffffu, ok);
                 const int at = n + __popc(bal & ((1u << lane) - 1u));
-                if (ok && at < kSd3MaxE) {
-                    const int hc = code[hh];
-                    E[at] = cr3::EHand{static_cast<double>(rv), (hc >> 20) & 63, (hc >> 26) & 63};
-                }
+                if (ok && at < kSd3MaxE) E[at] = cr3::EHand{static_cast<double>(rv), x, y};
                 n += __popc(bal);
             }
             if (lane == 0) en[warp] = n;
@@ -3451,107 +3602,161 @@ __global__ void __launch_bounds__(kTermThreads, 2) k_term_sd3(DevCtx c0, const D
             // ranges build; the direct pairs run first, while the tables
             // still hold the weaker parts
             if (!(t_valid && t_hi == lo)) {
-                build(0, lo, 0, lo);
+                build(0, lo, 0, lo, false);
                 t_valid = true;
                 t_hi = lo;
             }
-            const double work = static_cast<double>(nmine) * static_cast<double>(t.isc[4]);
+            const double work = static_cast<double>(nmine) * static_cast<double>(n3);
             auto go_direct = [&](int pr) {
                 if (!small) return false;
                 const double terms = pr == 1 ? n1 : pr == 2 ? n2 : 0.125 * n1 * n2;
                 return work * (0.8 * terms) <= kSd3BuildCost + work;
             };
-            int order[4] = {0, 0, 0, 0}, no = 1;
-            for (int pr = 1; pr < 4; ++pr)
-                if (go_direct(pr)) order[no++] = pr;
-            for (int pr = 1; pr < 4; ++pr)
-                if (!go_direct(pr)) order[no++] = pr;
-            const int j0 = max(lo, q0) - q0, ng = min(hi, qend) - q0 - j0;
-            const int per = ng >= kSd3Warps ? 1 : kSd3Warps / ng;   // warps per hand
-            const int hpr = kSd3Warps / per;                          // hands per round
+            // an opponent without a hand in its part of a pair: no tuple, both
+            // class masses exactly 0 (what the tables and the exact count
+            // would give), nothing to do
+            const int w1 = pre1[lo] - pre1[0], e1 = pre1[hi] - pre1[lo];
+            const int w2 = pre2[lo] - pre2[0], e2 = pre2[hi] - pre2[lo];
+            // pairs to take from the weaker parts' tables, and to build (two
+            // bits each, in order)
+            unsigned now = 0u, later = 0u;
+            int n_now = 0, n_later = 0;
+            for (int pr = 0; pr < 4; ++pr) {
+                if (((pr & 1) ? e1 : w1) == 0 || ((pr & 2) ? e2 : w2) == 0) continue;
+                if (pr == 0 || go_direct(pr))
+                    now |= static_cast<unsigned>(pr) << (2 * n_now++);
+                else
+                    later |= static_cast<unsigned>(pr) << (2 * n_later++);
+            }
+            const int per = ng >= kSd3Warps ? 1 : kSd3Warps / ng;   // warps per (hand, pair)
+            const int ipr = kSd3Warps / per;                          // (hand, pair) items per round
             const int r = warp / per, sl = warp - r * per;
-            const int jl = tid - j0;                                  // this thread's index in the group
-            auto walk = [&](int pr, bool direct, int base, bool want_count) {
-                const int j = j0 + base + r;
-                double o[2] = {0.0, 0.0};
-                long long n[2] = {0, 0};
-                if (r < hpr && base + r < ng && ghas[j]) {
-                    if (direct)
-                        cr3::e_pair_slice(pr, ga[j], gb[j], t, elist1, n1, elist2, n2, p3, lo, hi, sl * 32 + lane,
-                                          per * 32, o, n);
-                    else
-                        cr3::hand_mass_cls_slice(ga[j], gb[j], t, p3, lo, hi, sl * 32 + lane, per * 32, o, n,
-                                                 want_count);
-                }
-                for (int off = 16; off > 0; off >>= 1) {
-                    o[0] += __shfl_xor_sync(0xffffffffu, o[0], off);
-                    o[1] += __shfl_xor_sync(0xffffffffu, o[1], off);
-                    n[0] += __shfl_xor_sync(0xffffffffu, n[0], off);
-                    n[1] += __shfl_xor_sync(0xffffffffu, n[1], off);
-                }
-                if (lane == 0) {
-                    part[2 * warp] = o[0];
-                    part[2 * warp + 1] = o[1];
-                    partc[2 * warp] = n[0];
-                    partc[2 * warp + 1] = n[1];
-                }
-                __syncthreads();
-            };
-            for (int step = 0; step < 4; ++step) {
-                const int pr = order[step];
-                int lo1, hi1, lo2, hi2;
-                cr3::sd3_pair_bounds(pr, lo, hi, &lo1, &hi1, &lo2, &hi2);
-                // an opponent without a hand in its part of the pair: no
-                // tuple, both class masses exactly 0 (what the tables and the
-                // exact count would give), no tables to build
-                if (pre1[hi1] == pre1[lo1] || pre2[hi2] == pre2[lo2]) {
-                    if (mine) st.m[pr][0] = st.m[pr][1] = 0.0;
-                    continue;
-                }
-                // direct: a pair with a short tying part, from the weaker
-                // parts' tables and the lists (masses and exact counts in one
-                // walk); otherwise the pair's own tables
-                const bool direct = pr > 0 && go_direct(pr);
-                if (pr > 0 && !direct) {
-                    build(lo1, hi1, lo2, hi2);
-                    t_valid = false;   // the pair's tables replace the weaker parts'
-                }
+            // the class masses of n_pairs pairs: LL and built pairs (`built`)
+            // from the tables, tying pairs directly
+            auto walk = [&](unsigned pairs, int n_pairs, bool built) {
+                const int n_work = n_pairs * nmine;
                 const double zb = cr3::zero_bound(t);
-                bool near_zero = false;
-                for (int base = 0; base < ng; base += hpr) {
-                    walk(pr, direct, base, false);
-                    if (mine && jl >= base && jl < base + hpr) {
-                        double m0 = 0.0, m1 = 0.0;
-                        long long c0 = 0, c1 = 0;
-                        for (int k = 0; k < per; ++k) {
-                            m0 += part[2 * ((jl - base) * per + k)];
-                            m1 += part[2 * ((jl - base) * per + k) + 1];
-                            c0 += partc[2 * ((jl - base) * per + k)];
-                            c1 += partc[2 * ((jl - base) * per + k) + 1];
+                bool near = false;
+                int near_pr = 0;
+                for (int base = 0; base < n_work; base += ipr) {
+                    const int item = base + r;
+                    double o[2] = {0.0, 0.0};
+                    long long n[2] = {0, 0};
+                    if (r < ipr && item < n_work) {
+                        const int pi = item / nmine, j = gl[k0 + item - pi * nmine];
+                        const int pr = static_cast<int>(pairs >> (2 * pi)) & 3;
+                        const int a = ga[j], b = gb[j];
+                        const bool direct = pr > 0 && !built;
+                        if (direct)
+                            cr3::e_pair_slice(pr, a, b, t, elist1, n1, elist2, n2, p3, lo, hi, sl * 32 + lane,
+                                              per * 32, o, n);
+                        else
+                            cr3::hand_mass_cls_slice(a, b, t, p3, lo, hi, sl * 32 + lane, per * 32, o, n, false);
+                        for (int off = 16; off > 0; off >>= 1) {
+                            o[0] += __shfl_xor_sync(0xffffffffu, o[0], off);
+                            o[1] += __shfl_xor_sync(0xffffffffu, o[1], off);
                         }
-                        if (direct) {
-                            st.m[pr][0] = c0 == 0 ? 0.0 : m0;
-                            st.m[pr][1] = c1 == 0 ? 0.0 : m1;
-                        } else {
-                            st.m[pr][0] = m0;
-                            st.m[pr][1] = m1;
-                            near_zero = fabs(m0) <= zb || fabs(m1) <= zb;
+                        // one warp holds all of a hand's sum: the exact count at once
+                        const bool near0 = !direct && per == 1 && fabs(o[0]) <= zb;
+                        const bool near1 = !direct && per == 1 && fabs(o[1]) <= zb;
+                        if (near0 || near1) {
+                            double none[2];
+                            cr3::hand_mass_cls_slice(a, b, t, p3, lo, hi, lane, 32, none, n, true);
                         }
+                        if (direct || near0 || near1)
+                            for (int off = 16; off > 0; off >>= 1) {
+                                n[0] += __shfl_xor_sync(0xffffffffu, n[0], off);
+                                n[1] += __shfl_xor_sync(0xffffffffu, n[1], off);
+                            }
+                        if (near0 && n[0] == 0) o[0] = 0.0;
+                        if (near1 && n[1] == 0) o[1] = 0.0;
+                    }
+                    double *ps = part + buf * 2 * kSd3Warps;
+                    long long *cs = partc + buf * 2 * kSd3Warps;
+                    if (lane == 0) {
+                        ps[2 * warp] = o[0];
+                        ps[2 * warp + 1] = o[1];
+                        cs[2 * warp] = n[0];
+                        cs[2 * warp + 1] = n[1];
                     }
                     __syncthreads();
-                }
-                if (__syncthreads_or(near_zero)) {
-                    for (int base = 0; base < ng; base += hpr) {
-                        walk(pr, false, base, true);
-                        if (mine && jl >= base && jl < base + hpr)
-                            for (int cls = 0; cls < 2; ++cls) {
-                                long long n = 0;
-                                for (int k = 0; k < per; ++k) n += partc[2 * ((jl - base) * per + k) + cls];
-                                if (fabs(st.m[pr][cls]) <= zb && n == 0) st.m[pr][cls] = 0.0;
+                    if (mine_at >= 0)
+                        for (int pi = 0; pi < n_pairs; ++pi) {
+                            const int at = pi * nmine + mine_at - base;
+                            if (at < 0 || at >= ipr) continue;
+                            const int pr = static_cast<int>(pairs >> (2 * pi)) & 3;
+                            double m0 = 0.0, m1 = 0.0;
+                            long long c0 = 0, c1 = 0;
+                            for (int k = 0; k < per; ++k) {
+                                m0 += ps[2 * (at * per + k)];
+                                m1 += ps[2 * (at * per + k) + 1];
+                                c0 += cs[2 * (at * per + k)];
+                                c1 += cs[2 * (at * per + k) + 1];
                             }
+                            if (pr > 0 && !built) {
+                                if (c0 == 0) m0 = 0.0;
+                                if (c1 == 0) m1 = 0.0;
+                            } else if (per > 1 && (fabs(m0) <= zb || fabs(m1) <= zb)) {
+                                near = true;
+                                near_pr = pr;
+                            }
+#pragma unroll
+                            for (int p = 0; p < 4; ++p)
+                                if (p == pr) {
+                                    st.m[p][0] = m0;
+                                    st.m[p][1] = m1;
+                                }
+                        }
+                    buf ^= 1;
+                }
+                // a sum split over warps: the exact counts in a second pass
+                // (at most one of the pairs is from the tables: the first)
+                if (per > 1 && __syncthreads_or(near)) {
+                    for (int base = 0; base < nmine; base += ipr) {
+                        long long n[2] = {0, 0};
+                        if (r < ipr && base + r < nmine) {
+                            const int j = gl[k0 + base + r];
+                            double none[2];
+                            cr3::hand_mass_cls_slice(ga[j], gb[j], t, p3, lo, hi, sl * 32 + lane, per * 32, none, n,
+                                                     true);
+                            for (int off = 16; off > 0; off >>= 1) {
+                                n[0] += __shfl_xor_sync(0xffffffffu, n[0], off);
+                                n[1] += __shfl_xor_sync(0xffffffffu, n[1], off);
+                            }
+                        }
+                        long long *cs = partc + buf * 2 * kSd3Warps;
+                        if (lane == 0) {
+                            cs[2 * warp] = n[0];
+                            cs[2 * warp + 1] = n[1];
+                        }
                         __syncthreads();
+                        const int at = mine_at - base;
+                        if (near && at >= 0 && at < ipr) {
+                            long long c0 = 0, c1 = 0;
+                            for (int k = 0; k < per; ++k) {
+                                c0 += cs[2 * (at * per + k)];
+                                c1 += cs[2 * (at * per + k) + 1];
+                            }
+#pragma unroll
+                            for (int p = 0; p < 4; ++p)
+                                if (p == near_pr) {
+                                    if (fabs(st.m[p][0]) <= zb && c0 == 0) st.m[p][0] = 0.0;
+                                    if (fabs(st.m[p][1]) <= zb && c1 == 0) st.m[p][1] = 0.0;
+                                }
+                        }
+                        buf ^= 1;
                     }
                 }
+            };
+            if (n_now > 0) walk(now, n_now, false);
+            for (int i = 0; i < n_later; ++i) {
+                const int pr = static_cast<int>(later >> (2 * i)) & 3;
+                int lo1, hi1, lo2, hi2;
+                cr3::sd3_pair_bounds(pr, lo, hi, &lo1, &hi1, &lo2, &hi2);
+                __syncthreads();
+                build(lo1, hi1, lo2, hi2, false);
+                t_valid = false;   // the pair's tables replace the weaker parts'
+                walk(static_cast<unsigned>(pr), 1, true);
             }
         }
         // advance the weaker parts' tables past this group: its tying hands
@@ -4028,9 +4233,9 @@ cudaError_t launch_terms_t(const DevCtx &c, int kind, const TermItem *items, int
             if (c.HS > kMaxHS || c.ncomb > kSd3Positions) return cudaErrorInvalidValue;
             const int nc = (kSd3Positions + kTermThreads - 1) / kTermThreads;
             e = cudaFuncSetAttribute(k_term_sd3<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(sd3_smem(kMaxHS)));
+                                     static_cast<int>(sd3_smem<T>(kMaxHS)));
             if (e != cudaSuccess) return e;
-            SSB_LAUNCH(k_term_sd3<T>, n * nc, kTermThreads, sd3_smem(c.HS), s, c, ctxs, items, nc, trav);
+            SSB_LAUNCH(k_term_sd3<T>, n * nc, kTermThreads, sd3_smem<T>(c.HS), s, c, ctxs, items, nc, trav);
             break;
         }
         case TK_CR3: {
