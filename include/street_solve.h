@@ -139,7 +139,7 @@ typedef struct {
 
 typedef struct {
     int device;                   /* CUDA device ordinal (default 0) */
-    int graph_iterations;         /* CFR iterations per captured CUDA graph (default 10) */
+    int graph_iterations;         /* CFR iterations per captured CUDA graph, at most (default 10) */
     float target_exploitability;  /* stop at this exploitability, % of pot; <= 0: run all iterations */
     int check_every;              /* iterations between exploitability checks (default 50) */
     int compute_exploitability;   /* 1: report the final exploitability in SSSolveStats */

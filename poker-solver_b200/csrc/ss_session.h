@@ -66,7 +66,9 @@ class Session {
     // per (player, level) / (traverser, kind) minimum bytes, for the profile
     std::vector<double> reach_bytes[SS_MAX_PLAYERS], cfv_bytes[SS_MAX_PLAYERS];
     double term_bytes[SS_MAX_PLAYERS][TK_COUNT] = {};
-    cudaGraphExec_t gA = nullptr, gC = nullptr, gB = nullptr;  // G iters, 1 iter, 1 iter + snapshot
+    cudaGraphExec_t graph = nullptr;   // graph_len iterations
+    int graph_len = 0;
+    int direct_done = 0;               // iterations launched without a graph while there was none
     // best response state (allocated on first use, ensure_br)
     std::vector<float> host_w;          // range weights [np][HS]
     double *dbr = nullptr;              // reach_d [E + np][HS], val_d [N + 1][HS]
@@ -96,9 +98,7 @@ class Session {
     cudaEvent_t ev_fork = nullptr, ev_join[TK_COUNT] = {};
 
     ~Session() {
-        if (gA) cudaGraphExecDestroy(gA);
-        if (gB) cudaGraphExecDestroy(gB);
-        if (gC) cudaGraphExecDestroy(gC);
+        if (graph) cudaGraphExecDestroy(graph);
         for (int k = 0; k < TK_COUNT; ++k) {
             if (side[k]) cudaStreamDestroy(side[k]);
             if (ev_join[k]) cudaEventDestroy(ev_join[k]);
@@ -266,15 +266,22 @@ class Session {
         return e;
     }
 
+    // `iters` iterations launched one by one; the last one's root strategy is
+    // kept for the output
+    cudaError_t direct(int iters, bool last) {
+        cudaError_t e = ensure_side();
+        for (int i = 0; i < iters && e == cudaSuccess; ++i) e = iteration(last && i == iters - 1, i + 1);
+        if (e == cudaSuccess) e = mark(PC_OTHER, 0);
+        if (e == cudaSuccess) e = launch_bump(diter, iters, stream);
+        return e;
+    }
+
     cudaError_t capture(int iters, bool last, cudaGraphExec_t *exec) {
         cudaGraph_t g = nullptr;
         cudaError_t e = ensure_side();
         if (e == cudaSuccess) e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
-        cudaError_t body = cudaSuccess;
-        for (int i = 0; i < iters && body == cudaSuccess; ++i) body = iteration(last && i == iters - 1, i + 1);
-        if (body == cudaSuccess) body = mark(PC_OTHER, 0);
-        if (body == cudaSuccess) body = launch_bump(diter, iters, stream);
+        const cudaError_t body = direct(iters, last);
         e = cudaStreamEndCapture(stream, &g);
         if (body != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
