@@ -2395,8 +2395,8 @@ constexpr int SD2_S = 49;   // row stride of the sweep's card matrices (odd: con
 constexpr int SD2_N = 48;   // cards a matrix covers (dense indices; a river deck has 47)
 constexpr int SD2_W = (1326 + 31) / 32;   // words of a position mask
 // live positions (of the opponent with more) up to which a sweep takes the sparse form.  A
-// river's 40 three-way showdowns, dense -> sparse form: 66 -> 51 us at 200 hands, 72 -> 70 at
-// 400, 74 -> 82 at 550, 84 -> 125 at all 1,081 (walking masks costs more than testing values)
+// river's 40 three-way showdowns, dense -> sparse form: 61 -> 48 us at 200 hands, 65.5 -> 65.5
+// at 400, 66 -> 72 at 550, 74 -> 110 at all 1,081 (walking masks costs more than testing values)
 constexpr int SD2_SPARSE = 400;
 static_assert(kTermThreads == 256, "the sweep's thread roles assume 256 threads");
 
@@ -2497,53 +2497,52 @@ __device__ __forceinline__ void sd2_add(Sd2State st, const unsigned short *dd, c
                 *p += r * static_cast<double>(Mx[x * SD2_S + j]);
             }
         }
-    } else if (tid < 5 * SD2_N) {
-        // card c: this opponent's card sum u(c), d(c) = sum_b M1[c][b] M2[c][b]
-        // and w(c) = (M2 u1 + M1 u2)(c): the hand changes Mo at (x, y) and uo
-        // at x, y
-        const int c = tid - 4 * SD2_N;
+        return;
+    }
+    // Warps 6 and 7.  Card c: this opponent's card sum u(c), d(c) = sum_b
+    // M1[c][b] M2[c][b] and w(c) = (M2 u1 + M1 u2)(c): the hand changes Mo at
+    // (x, y) and uo at x, y.  The lane after the last card takes F (this
+    // opponent's total), Q = sum u1 u2 and D = sum d / 2 in the same steps (a
+    // branch of its own, and one for Mo's cells, ran after the cards': 500
+    // cycles per hand where the other warps took 200 to 250).
+    const int c = tid - 4 * SD2_N;
+    const bool all = c == SD2_N;
+    if (c <= SD2_N) {
         double du = 0.0, dd_c = 0.0, dw = 0.0;
+        if (all) {
+            du = st.sc[who];
+            dw = st.sc[2];
+            dd_c = st.sc[3];
+        }
         for (int q = sd2_next<SP>(on, lo, hi); q < hi; q = sd2_next<SP>(on, q + 1, hi)) {
             const T rt = R[q];
             if (!SP && rt == T(0)) continue;
             const double r = static_cast<double>(rt);
             const unsigned short e = dd[q];
             const int x = sd2_c1(e), y = sd2_c2(e);
-            const double mx = static_cast<double>(Mx[c * SD2_S + x]), my = static_cast<double>(Mx[c * SD2_S + y]);
-            dw += r * (mx + my);
-            if (c == x) {
+            const bool mine = all || c == x || c == y;
+            const double mx = static_cast<double>(Mx[(all ? y : c) * SD2_S + x]);
+            const double my = static_cast<double>(Mx[(all ? x : c) * SD2_S + y]);
+            const double uy = ux[c == x || all ? y : x];
+            dw = fma(r, all ? ux[x] + uy : mx + my, dw);
+            if (mine) {
                 du += r;
-                dd_c += r * my;
-                dw += r * ux[y];
-            }
-            if (c == y) {
-                du += r;
-                dd_c += r * mx;
-                dw += r * ux[x];
+                dd_c = fma(r, c == y ? mx : my, dd_c);
+                if (!all) dw = fma(r, uy, dw);
             }
         }
-        uo[c] += du;
-        st.d[c] += dd_c;
-        st.w[c] += dw;
-    } else if (tid == 5 * SD2_N) {
-        // F (this opponent's total), Q = sum u1 u2, D = sum d / 2
-        double F = st.sc[who], Q = st.sc[2], D = st.sc[3];
-        for (int q = sd2_next<SP>(on, lo, hi); q < hi; q = sd2_next<SP>(on, q + 1, hi)) {
-            const T rt = R[q];
-            if (!SP && rt == T(0)) continue;
-            const double r = static_cast<double>(rt);
-            const unsigned short e = dd[q];
-            const int x = sd2_c1(e), y = sd2_c2(e);
-            Q += r * (ux[x] + ux[y]);
-            D += r * static_cast<double>(Mx[x * SD2_S + y]);
-            F += r;
+        if (all) {
+            st.sc[who] = du;
+            st.sc[2] = dw;
+            st.sc[3] = dd_c;
+        } else {
+            uo[c] += du;
+            st.d[c] += dd_c;
+            st.w[c] += dw;
         }
-        st.sc[who] = F;
-        st.sc[2] = Q;
-        st.sc[3] = D;
-    } else {
-        constexpr int kFirst = 5 * SD2_N + 1, kStep = kTermThreads - kFirst;
-        for (int q = lo + tid - kFirst; q < hi; q += kStep) {
+    }
+    if (c < 32)
+        for (int q = lo + c; q < hi; q += 32) {
             const T r = R[q];
             if (r == T(0)) continue;
             const unsigned short e = dd[q];
@@ -2551,7 +2550,6 @@ __device__ __forceinline__ void sd2_add(Sd2State st, const unsigned short *dd, c
             Mo[x * SD2_S + y] = r;
             Mo[y * SD2_S + x] = r;
         }
-    }
 }
 
 // The sweep state for the opponents' hands at rank positions [0, qend),
@@ -2690,12 +2688,13 @@ __device__ __forceinline__ void sd2_direct_state(Sd2State st, T *M1, T *M2, cons
 }
 
 // For the traverser's hands at positions [lo, hi) (a tie group), on the state
-// before the group: A = D(L, L); T1 = D(L, E) + D(E, L), summing over
+// before the group: T1 = D(L, E) + D(E, L), summing over
 // opponent 2's group hands (opponent 1's weaker hands avoiding four cards)
 // and over opponent 1's (opponent 2's avoiding four cards); whether opponent 2
 // holds any group hand.  Eight lanes per hand, each taking every eighth group
 // position, combined in a fixed order.  Classes of position q at
-// cls[4 (q - base)]: A, T1, opponent 2 present, (C).
+// cls[4 (q - base)]: A = D(L, L), T1, opponent 2 present, C; A and C are
+// sd2_phase_mass's.
 template <bool SP, class T>
 __device__ __forceinline__ void sd2_phase_a(Sd2State st, const T *M1, const T *M2, const T *R1, const T *R2,
                                             const unsigned short *dd, const short *pt, double *cls, int base,
@@ -2755,7 +2754,6 @@ __device__ __forceinline__ void sd2_phase_a(Sd2State st, const T *M1, const T *M
         const unsigned bal = __ballot_sync(0xffffffffu, any2);
         if (mine && l8 == 0) {
             double *k4 = cls + 4 * (q - base);
-            k4[0] = sd2_mass(st, M1, M2, a, b);
             k4[1] = t1;
             k4[2] = ((bal >> tbit) & 0xffu) ? 1.0 : 0.0;
         }
@@ -2763,11 +2761,12 @@ __device__ __forceinline__ void sd2_phase_a(Sd2State st, const T *M1, const T *M
 }
 
 // mass on the current state for the traverser's hands at [lo, hi), into
-// class slot k
+// class slot k; thread `first` takes the first hand, so that a short group's
+// masses fall to warps that its T1 leaves idle
 template <class T>
 __device__ __forceinline__ void sd2_phase_mass(Sd2State st, const T *M1, const T *M2, const unsigned short *dd,
-                                               const short *pt, double *cls, int base, int lo, int hi, int k) {
-    for (int q = lo + threadIdx.x; q < hi; q += kTermThreads)
+                                               const short *pt, double *cls, int base, int lo, int hi, int k, int first) {
+    for (int q = lo + ((threadIdx.x - first) & (kTermThreads - 1)); q < hi; q += kTermThreads)
         if (pt[q - base] >= 0) cls[4 * (q - base) + k] = sd2_mass(st, M1, M2, sd2_c1(dd[q]), sd2_c2(dd[q]));
 }
 
@@ -2785,6 +2784,7 @@ __device__ __forceinline__ void sd2_run(const Sd2State &st, T *M1, T *M2, const 
                                         const unsigned short *dd, const short *pt, double *cls,
                                         const int4 *__restrict__ seg4, int4 sg, int s0, int s1, int run_hi, int nc) {
     const int run_lo = sg.x;
+    constexpr int kMassA = 5 * 32, kMassC = 7 * 32;   // first threads of the masses
     // the runs start from the state of every hand ranked below them
     sd2_direct_state<SP>(st, M1, M2, R1, R2, dd, run_lo);
 
@@ -2795,6 +2795,7 @@ __device__ __forceinline__ void sd2_run(const Sd2State &st, T *M1, T *M2, const 
     bool reads = false;
     if (sg.z) {
         sd2_phase_a<SP>(st, M1, M2, R1, R2, dd, pt, cls, run_lo, sg.x, sg.y);
+        sd2_phase_mass(st, M1, M2, dd, pt, cls, run_lo, sg.x, sg.y, 0, kMassA);
         reads = true;
     }
     for (int si = s0; si < s1; ++si) {
@@ -2814,8 +2815,11 @@ __device__ __forceinline__ void sd2_run(const Sd2State &st, T *M1, T *M2, const 
             __syncthreads();
         }
         // C of this group and A of the next group: the same state
-        if (has) sd2_phase_mass(st, M1, M2, dd, pt, cls, run_lo, lo, hi, 3);
-        if (nhas) sd2_phase_a<SP>(st, M1, M2, R1, R2, dd, pt, cls, run_lo, nsg.x, nsg.y);
+        if (has) sd2_phase_mass(st, M1, M2, dd, pt, cls, run_lo, lo, hi, 3, kMassC);
+        if (nhas) {
+            sd2_phase_mass(st, M1, M2, dd, pt, cls, run_lo, nsg.x, nsg.y, 0, kMassA);
+            sd2_phase_a<SP>(st, M1, M2, R1, R2, dd, pt, cls, run_lo, nsg.x, nsg.y);
+        }
         reads = reads || has || nhas;
         sg = nsg;   // the next segment's entry is loaded a full step before its use
         if (si + 2 < s1) nsg = __ldg(seg4 + si + 2);
