@@ -381,7 +381,7 @@ constexpr int kSmallIters = 128;
 // 2 at 200 of them.  Building and destroying graphs of 10, 1 and 1 iterations
 // took 6 ms of a 3-player river's 69 and 12 ms of a 4-player river's 32.
 constexpr int kDirectIters = 16;
-static int graph_length(int iters, int most) {
+int graph_length(int iters, int most) {
     int len = 1;
     while (len < most && 64 * (len + 1) * len <= iters) ++len;
     return len;

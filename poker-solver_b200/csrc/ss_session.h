@@ -36,6 +36,9 @@ inline int term_class(int kind) {
     }
 }
 
+// iterations of a captured graph where `iters` are run, at most `most`
+int graph_length(int iters, int most);
+
 class Session {
   public:
     Plan P;

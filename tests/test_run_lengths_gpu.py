@@ -41,3 +41,19 @@ def test_cuts_of_a_run(runs, most):
     assert np.array_equal(avg, np.asarray(ref["avg_strategies"]).ravel())
     assert np.array_equal(rs, np.asarray(ref["root_strategy"]).ravel())
     sg.free()
+
+
+@pytest.mark.parametrize("iterations,most", [(1, 10), (40, 10), (150, 10), (390, 10), (390, 2)])
+def test_batches_of_any_length(iterations, most):
+    """Several players and kinds of terminals side by side, over graphs of 1 to
+    3 iterations and what is left over."""
+    subs = [make(c) for c in ((3, 5, [1.0], 1, 9, 0), (2, 5, [0.5, 1.0], 1, 40, 0), (4, 5, [1.0], 1, 17, 0),
+                              (2, 4, [1.0], 1, 33, 0))]
+    refs = [noalloc_solve(sg, iterations) for sg in subs]
+    rc, got = wl.batch_solve(subs, iterations, graph_iterations=most)
+    assert rc == 0, wl.ssg.last_error(subs[0].lib)
+    for ref, r in zip(refs, got):
+        for k in ("avg_strategies", "root_strategy", "root_ev"):
+            assert np.array_equal(r[k], ref[k]), k
+    for sg in subs:
+        sg.free()
