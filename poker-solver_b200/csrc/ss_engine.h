@@ -241,7 +241,7 @@ inline int sd2_merge_of(int n_terms) {
     return lg;
 }
 
-// Folds and leaves with three counted opponents use the conditioning closed
+// Folds and leaves with three counted opponents use the contraction closed
 // form (TK_CR3) once every counted range holds at least this many hands and
 // the first two hold no combo twice; smaller ranges enumerate (TK_ENUM).
 constexpr int kCr3MinHands = 16;
