@@ -546,7 +546,8 @@ SSB_CR3_HD void phase_gather_cls(int tid, int nt, const Opp3<T> &in, const Table
 }
 
 // the third opponent's positive-reach live hands in hand order with their
-// rank positions (one item; run once per block)
+// rank positions (for the host checks: the kernel lists them with the whole
+// block, in the same order)
 template <class T>
 SSB_CR3_HD void compact_third(int tid, const Opp3<T> &in, const Tables &t, const int *pos3, int *p3) {
     if (tid != 0) return;
@@ -851,7 +852,9 @@ SSB_CR3_HD void sd3_thread_init(int q, int qend, const int *pos_hand_t, const in
     }
 }
 
-// after the full pair's tables: the total, exact 0 when no tuple exists
+// after the full pair's tables: the total, exact 0 when no tuple exists (for
+// the host checks: the kernel spreads a hand's terms over lanes and adds them
+// in the same order)
 SSB_CR3_HD void sd3_thread_total(Sd3Thread &s, const Tables &t, const int *p3) {
     if (s.h < 0) return;
     double o[3];
