@@ -1562,7 +1562,9 @@ constexpr size_t sd1_smem() {
 // Latency-bound: a heads-up river launches tens of these blocks and waits for
 // one.  1024 threads: eight warps scan the rank positions while the other 24
 // take the cards' lists, and every table that no kernel writes is read before
-// the wait for the previous kernel where a register can hold it.
+// the wait for the previous kernel where a register can hold it.  (Not of a
+// member that has left the batch: its tables are freed.  The live flag is
+// written by a copy, which the kernels' order cannot overtake.)
 constexpr int kSd1Threads = 1024;
 constexpr int kSd1Scan = 256;   // threads of the rank-order scan (fixes its summation order)
 template <class T>
@@ -1583,10 +1585,11 @@ __device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__r
     const bool dup = c.dup[o] != 0;
     const int *ph = c.pos_hand + static_cast<size_t>(o) * nc;
     const int *tpos = c.sd_pos + static_cast<size_t>(trav) * HS;
-    const int ph0 = tid < nc ? __ldg(ph + tid) : -1;
-    const int q0 = tid < Ht ? __ldg(tpos + tid) : -1;
+    const bool gone = retired(ctxs, I.sg);
+    const int ph0 = !gone && tid < nc ? __ldg(ph + tid) : -1;
+    const int q0 = !gone && tid < Ht ? __ldg(tpos + tid) : -1;
     wait_prior_grid();
-    if (retired(ctxs, I.sg)) return;
+    if (gone) return;
     const T *r = reach_rows<T>(c) + static_cast<size_t>(I.opp_row[0]) * HS;
     if (!dup) {
         // the opponent's reach by rank position, gathered
