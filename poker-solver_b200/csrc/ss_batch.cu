@@ -16,6 +16,7 @@
 // member's FP64 exploitability at block ends, and retires a member when it
 // reaches the target (or the iteration cap), freeing its memory for the next
 // requests.  Latency = submission to retirement.
+#include "ss_runs.h"
 #include "ss_session.h"
 
 #include <algorithm>
@@ -207,8 +208,8 @@ class Batch {
     std::vector<Launch> seq, br_seq;
     cudaGraphExec_t graph = nullptr, br_graph = nullptr;
     // a pass's terminal launches write disjoint value rows and only read reach:
-    // they run side by side (most fill a part of the chip, or end in a tail of
-    // few blocks): a mixed batch of 16 requests 277 -> 228 ms, with the shorter
+    // they run side by side (ss_runs.h; most fill a part of the chip, or end in a
+    // tail of few blocks): a mixed batch of 16 requests 277 -> 228 ms, with the shorter
     // graphs of run()
     static constexpr int kSides = 5;
     cudaStream_t side[kSides] = {};
@@ -278,14 +279,14 @@ class Batch {
         return SS_OK;
     }
 
+    static bool terminal(const Launch &L) { return L.type == L_TERM || L.type == L_BR_TERM; }
+
     // the launches of `q` in order, each run of terminal launches forked over
     // the side streams (the last one, with the most work, stays on the stream)
     cudaError_t run_all(const std::vector<Launch> &q) {
         cudaError_t e = cudaSuccess;
         for (size_t i = 0; i < q.size() && e == cudaSuccess;) {
-            size_t j = i + 1;
-            if (q[i].type == L_TERM || q[i].type == L_BR_TERM)
-                while (j < q.size() && q[j].type == q[i].type) ++j;
+            const size_t j = run_end(q, i, terminal);
             const int sides = std::min<int>(kSides, static_cast<int>(j - i) - 1);
             if (sides > 0) e = cudaEventRecord(ev_fork, stream);
             for (int k = 0; k < sides && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(side[k], ev_fork, 0);
@@ -564,18 +565,10 @@ class Batch {
         // within a run of terminal launches: by work, the most last (block times as
         // in Session::launch_kinds)
         for (std::vector<Launch> *q : {&seq, &br_seq})
-            for (size_t i = 0, j; i < q->size(); i = j) {
-                j = i + 1;
-                const int type = (*q)[i].type;
-                if (type != L_TERM && type != L_BR_TERM) continue;
-                while (j < q->size() && (*q)[j].type == type) ++j;
-                auto weight = [](const Launch &L) {
-                    const int k = L.kind;
-                    return L.n * (k == TK_SD3 || k == TK_CR3 ? 64.0 : k == TK_SD2 || k == TK_ENUM ? 16.0 : 1.0);
-                };
-                std::stable_sort(q->begin() + static_cast<std::ptrdiff_t>(i), q->begin() + static_cast<std::ptrdiff_t>(j),
-                                 [&](const Launch &x, const Launch &y) { return weight(x) < weight(y); });
-            }
+            order_runs(q, terminal, [](const Launch &L) {
+                const int k = L.kind;
+                return L.n * (k == TK_SD3 || k == TK_CR3 ? 64.0 : k == TK_SD2 || k == TK_ENUM ? 16.0 : 1.0);
+            });
         built_work = live_work = 0;
         for (int i : act) built_work += work[i];
         live_work = built_work;
