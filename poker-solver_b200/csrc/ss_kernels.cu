@@ -3154,8 +3154,9 @@ __global__ void __launch_bounds__(32 * kEnumWarps) k_term_enum(DevCtx c0, const 
 // item's blocks write every member's row, each with its own factor.  Bound by
 // the FP64 pipe and shared memory: per hand and card 34 FP64 operations and
 // 23 shared-memory wavefronts per warp, beside two 48 x 48 products per block.
-// A hand whose mass is within rounding of 0 is looked at exactly, and 0 when
-// it has no tuple (the reference adds only positive products).
+// A hand whose mass is small beside the product of the three sums is summed
+// again by conditioning, to keep its digits, and 0 when it has no tuple (the
+// reference adds only positive products).
 //
 // 384 threads take the 1128 hands of a turn in three rounds of 98 %, and the
 // tables of a 48-card deck (105 KB) leave two blocks per SM (512 and 576
@@ -3245,7 +3246,7 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
     const int lanes = Ht * 4 <= kCr3Threads ? 4 : Ht * 2 <= kCr3Threads ? 2 : 1;
     const int per = kCr3Threads / lanes, mine = tid / lanes, part = tid % lanes;   // hands per round
     const int first = ch * per, step = nchunk * per;
-    unsigned near = 0;   // this thread's hands (by round) within rounding of 0
+    unsigned near = 0;   // this thread's hands (by round) to sum again
     int round = 0;
 #pragma unroll 1
     for (int h0 = first; h0 < HS; h0 += step, ++round) {
@@ -3265,7 +3266,7 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
         write(h, m);
     }
     if (!__syncthreads_or(near != 0)) return;
-    // a warp per hand within rounding of 0, 32 third-opponent hands at a time;
+    // a warp per hand to sum again, 32 third-opponent hands at a time;
     // the list of those hands takes C's space
     int *n_near = reinterpret_cast<int *>(t.C);
     unsigned short *list = reinterpret_cast<unsigned short *>(n_near + 4);
@@ -3280,10 +3281,10 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
     const int lane = tid & 31;
     for (int i = tid >> 5; i < *n_near; i += kCr3Threads / 32) {
         const int h = list[i], hc = __ldg(code_t + h), a = dense(hc, 20), b = dense(hc, 26);
-        bool any = false;
-        for (int j = lane; !any && j - lane < H3; j += 32)
-            any = __any_sync(0xffffffffu, j < H3 && tri::tuple_with(a, b, k, r3[j], __ldg(code3 + j)));
-        if (!any && lane == 0) write(h, 0.0);
+        double m = 0.0;
+        for (int j = lane; j < H3; j += 32) m += tri::tuple_mass(a, b, t, k, r3[j], __ldg(code3 + j));
+        m = warp_sum(m);
+        if (lane == 0) write(h, m);
     }
 }
 

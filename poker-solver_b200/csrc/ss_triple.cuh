@@ -302,15 +302,49 @@ SSB_TRI_HD double hand_finish(int a, int b, const Tables &t, const Part &part) {
 
 SSB_TRI_HD double hand_mass(int a, int b, const Tables &t) { return hand_finish(a, b, t, hand_part(a, b, t, 0, 1)); }
 
-// A computed mass at or below this may be an empty set of tuples (every term
-// is at most a few F_A F_B F_C, its rounding far below the factor here)
-SSB_TRI_HD double zero_bound(const Tables &t) { return 1e-9 * t.sc[FA] * t.sc[FB] * t.sc[FC]; }
+// Up to this bound a computed mass is summed again by conditioning on the
+// third opponent's hand (pair_mass): the contraction subtracts what hands that
+// share a card with the traverser add to the sums, so its error is a few
+// hundred roundings of F_A F_B F_C (below 1e-13 of that product), whatever is
+// left of it.  At 1e-6 of the product that is 1e-7 of the mass at most (3e-12
+// was seen at 8e-6, 120 hands).  Conditioning leaves those hands out instead, so a
+// third range whose weight lies on cards of the traverser's costs no digits;
+// it also finds the empty sets, whose mass is exactly 0.
+SSB_TRI_HD double zero_bound(const Tables &t) { return 1e-6 * t.sc[FA] * t.sc[FB] * t.sc[FC]; }
+
+// The mass of the first two opponents' pairs of disjoint hands that avoid the
+// four cards {a, b, x, y}: the two-opponent form, D2 in ss_cr3.cuh.
+SSB_TRI_HD double pair_mass(int a, int b, int x, int y, const Tables &t) {
+    const int s[4] = {a, b, x, y};
+    const double *v = t.v;
+    double fa = t.sc[FA], fb = t.sc[FB], q = t.sc[QAB], e = t.sc[EAB];
+    for (int i = 0; i < 4; ++i) {
+        const int c = s[i];
+        double ua = v[UA * kVS + c], ub = v[UB * kVS + c];
+        fa -= ua;
+        fb -= ub;
+        q -= v[AUB * kVS + c] + v[BUA * kVS + c];
+        e -= v[DAB * kVS + c];
+        for (int j = 0; j < 4; ++j) {
+            const double A = t.A[c * t.S + s[j]], B = t.B[c * t.S + s[j]];
+            ua -= A;
+            ub -= B;
+            q += t.AB[c * t.S + s[j]];
+            if (j > i) {
+                fa += A;
+                fb += B;
+                e += A * B;
+            }
+        }
+        q -= ua * ub;
+    }
+    return fa * fb - q + e;
+}
 
 // Whether a tuple of positive reach is disjoint and avoids {a, b} (exact):
 // tuple_with asks it for one hand of the third opponent, by the two-opponent
 // count on the positive cells of A and B (row masks mA, mB; row and vector
-// counts as in the mass).  Only hands near zero mass come here, and the first
-// third-opponent hand with a tuple ends it.
+// counts as in the mass).  Only hands near zero mass come here.
 struct Counts {
     unsigned long long *mA, *mB;   // [kVS]
     int *nA, *nB, *nW, *nD;        // [kVS]: row counts, (I_B n_A + I_A n_B), common cells
@@ -387,6 +421,14 @@ SSB_TRI_HD bool tuple_with(int a, int b, const Counts &k, T r, int code) {
         q -= static_cast<long long>(na) * nb;
     }
     return fa * fb - q + e > 0;
+}
+
+// what one hand of the third opponent adds to the mass of {a, b}; exactly 0
+// without a tuple
+template <class T>
+SSB_TRI_HD double tuple_mass(int a, int b, const Tables &t, const Counts &k, T r, int code) {
+    if (!tuple_with(a, b, k, r, code)) return 0.0;
+    return static_cast<double>(r) * pair_mass(a, b, (code >> 20) & 63, (code >> 26) & 63, t);
 }
 
 }  // namespace tri
