@@ -119,6 +119,12 @@ constexpr int kCfvLongFrontier = 48;
 // (k_cfv), chains per edge of such an item (k_tree)
 constexpr int kCfvSplit = 4;
 
+// Short value/regret items have one thread per (item, pair of hands), in blocks
+// of kCfvThreads numbered in 32 bits: a level with more of them (3.2 million
+// items of 1326 hands) is cut into launches of this many items.
+constexpr int kCfvThreads = 128;
+inline int cfv_items_per_launch(int pairs) { return (0x7fffffff / kCfvThreads * kCfvThreads) / pairs; }
+
 // Order one level's value/regret items short, then long (stable within each
 // class); returns the number of long items.
 template <class Item, class FrontierRows>

@@ -4096,11 +4096,12 @@ cudaError_t launch_cfv(const DevCtx &c, const CfvItem *items, int n, int n_long,
     if (n <= 0 || H <= 0) return cudaSuccess;
     n_long = n_long < 0 ? 0 : n_long > n ? n : n_long;
     const int n_short = n - n_long;
-    if (n_short > 0) {
-        const int pairs = (H + 1) / 2;
-        const long long threads = static_cast<long long>(n_short) * pairs;
+    const int pairs = (H + 1) / 2, most = cfv_items_per_launch(pairs);
+    for (long long at = 0; at < n_short; at += most) {
+        const int now = static_cast<int>(std::min<long long>(n_short - at, most));
+        const long long threads = static_cast<long long>(now) * pairs;
         SSB_LAUNCH(k_cfv<1>, static_cast<unsigned>((threads + kCfvThreads - 1) / kCfvThreads), kCfvThreads, 0, s, c, ctxs,
-                   items, n_short, pairs, H, trav, iter_add);
+                   items + at, now, pairs, H, trav, iter_add);
     }
     if (n_long > 0) {
         const int nc = (H + 63) / 64;

@@ -76,8 +76,6 @@ struct alignas(8) AvgItem {
 // threads per block of the per-hand kernels; each thread covers 4 hands
 constexpr int kHandThreads = 64;
 constexpr int kHandsPerBlock = kHandThreads * 4;
-// threads per block of the value/regret kernel (2 hands each)
-constexpr int kCfvThreads = 128;
 // threads per block of the per-terminal kernels
 constexpr int kTermThreads = 256;
 
