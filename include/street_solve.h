@@ -313,6 +313,13 @@ int ss_session_exploitability(SSSession *session, double *exploitability_pct, do
 int ss_session_narrow(SSSession *session, int player, int node, unsigned int action_mask, int num_hands,
                       const int *hand_cards, double *weights, int *applied);
 
+/* EXTENSION: how often a block of the session's iterations asks for the others
+ * at a grid-wide wait before it gives up (default: a few seconds' worth; 0: at
+ * once).  Once a wait has run out, every call that waits for the session or
+ * reads its state returns SS_ERR_CUDA until ss_session_reset; other sessions
+ * are not affected.  Sessions without such waits ignore it. */
+int ss_session_set_wait_limit(SSSession *session, unsigned int polls);
+
 /* EXTENSION: release the session. */
 void ss_session_destroy(SSSession *session);
 

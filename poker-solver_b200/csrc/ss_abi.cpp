@@ -324,6 +324,12 @@ int ss_session_narrow(SSSession *s, int player, int node, unsigned int action_ma
 
 void *ss_session_stream(SSSession *s) { return s ? ssb::session_stream(s->impl) : nullptr; }
 
+int ss_session_set_wait_limit(SSSession *s, unsigned int polls) {
+    if (!s) return SS_ERR_INVALID;
+    ssb::session_set_wait_limit(s->impl, polls);
+    return SS_OK;
+}
+
 void ss_session_destroy(SSSession *s) {
     if (!s) return;
     ssb::session_destroy(s->impl);

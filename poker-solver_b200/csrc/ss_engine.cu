@@ -295,8 +295,11 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     nVal = N * HS;
     CK(cudaMallocAsync(reinterpret_cast<void **>(&dstate), (2 * nR + nReach + nVal) * sizeof(float), stream));
     CK(cudaMemsetAsync(dstate, 0, (2 * nR + nReach + nVal) * sizeof(float), stream));
-    CK(cudaMallocAsync(reinterpret_cast<void **>(&diter), 2 * sizeof(int), stream));   // iteration, grid barrier
+    // iteration, grid barrier, fault word
+    CK(cudaMallocAsync(reinterpret_cast<void **>(&diter), 3 * sizeof(int), stream));
     small.barrier = reinterpret_cast<unsigned *>(diter + 1);
+    small.fault = reinterpret_cast<unsigned *>(diter + 2);
+    small.polls = kGridPolls;
     float *R = dstate, *S = R + nR, *reach = S + nR, *val = reach + nReach;
     {
         std::vector<float> w(static_cast<size_t>(np) * HS, 0.f);
@@ -360,7 +363,8 @@ int Session::reset() {
     CK(cudaSetDevice(device));
     CK(cudaMemsetAsync(dstate, 0, 2 * nR * sizeof(float), stream));
     CK(cudaMemsetAsync(c.val, 0, nVal * sizeof(float), stream));
-    CK(cudaMemsetAsync(diter, 0, sizeof(int), stream));
+    CK(cudaMemsetAsync(diter, 0, 3 * sizeof(int), stream));
+    small_fault = 0;
     CK(cudaMemsetAsync(dsmall, 0, (n_rs + P.HS) * sizeof(float), stream));
     for (int p = 0; p < P.np; ++p) CK(reach(p));  // all regrets zero: uniform (or frozen) play
     iterations = 0;
@@ -399,6 +403,7 @@ int Session::run(int iters) {
         return SS_ERR_UNSUPPORTED;
     }
     CK(cudaSetDevice(device));
+    if (small_fault) return small_fault_error();
     if (small_blocks > 0) {
         for (int done = 0; done < iters;) {
             const int n = std::min(kSmallIters, iters - done);
@@ -436,6 +441,26 @@ int Session::run(int iters) {
     return SS_OK;
 }
 
+// A barrier of k_small_solve that gives up leaves regrets, sums and the counter
+// of some blocks behind: whatever reads the state afterwards reports it, until
+// the state is reset.
+int Session::small_fault_error() {
+    set_error("a bounded wait in the session's iterations ran out: its state is lost until it is reset");
+    return SS_ERR_CUDA;
+}
+
+cudaError_t Session::fetch_small_fault() {
+    if (small_blocks == 0 || small_fault) return cudaSuccess;
+    return cudaMemcpyAsync(&small_fault, small.fault, sizeof(small_fault), cudaMemcpyDeviceToHost, stream);
+}
+
+int Session::sync() {
+    CK(cudaSetDevice(device));
+    CK(fetch_small_fault());
+    CK(cudaStreamSynchronize(stream));
+    return small_fault ? small_fault_error() : SS_OK;
+}
+
 int Session::output(SSOutput *out) {
     std::memset(out, 0, sizeof(*out));
     CK(cudaSetDevice(device));
@@ -470,19 +495,22 @@ int Session::output(SSOutput *out) {
         e = cudaMemcpyAsync(h_rev, d_rev, static_cast<size_t>(P.H[tl]) * sizeof(float),
                             cudaMemcpyDeviceToHost, stream);
     cudaFreeAsync(davg, stream);
+    if (e == cudaSuccess) e = fetch_small_fault();
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     unsigned fault = 0;
     if (e == cudaSuccess) e = read_device_fault(&fault, stream);
-    if (e != cudaSuccess || fault) {
+    if (e != cudaSuccess || fault || small_fault) {
         std::free(h_rs);
         std::free(h_rev);
         host_block_give(h_avg);
         std::free(h_ids);
         if (e != cudaSuccess)
             set_error(std::string("CUDA: ") + cudaGetErrorString(e));
-        else
+        else if (fault)
             set_error("a kernel recorded a device fault (code " + std::to_string(fault) +
-                      "): a bounded wait in it ran out or it got a subgame it does not serve");
+                      "): the tensor-core product's completion wait ran out or it got a subgame it does not serve");
+        else
+            return small_fault_error();
         return SS_ERR_CUDA;
     }
     for (int i = 0; i < P.num_dec; ++i) h_ids[i] = P.dec_nodes[i];
@@ -500,6 +528,10 @@ int Session::output(SSOutput *out) {
 
 int Session::profile(SSKernelProfile *prof) {
     std::memset(prof, 0, sizeof(*prof));
+    if (small_blocks > 0) {
+        const int rc = sync();
+        if (rc != SS_OK) return rc;
+    }
     CK(cudaSetDevice(device));
     std::vector<Mark> ms;
     marks = &ms;
@@ -645,7 +677,9 @@ int Session::exploitability(const float *host_avg, double *pct, double *nash, do
     CK(launch_br_root(c, br_row, 1, P.H[0], P.E, 0, 1, br_sc + 2 * SS_MAX_PLAYERS, stream));
     double sc[2 * SS_MAX_PLAYERS + 2] = {};
     CK(cudaMemcpyAsync(sc, br_sc, sizeof(sc), cudaMemcpyDeviceToHost, stream));
+    if (!host_avg) CK(fetch_small_fault());
     CK(cudaStreamSynchronize(stream));
+    if (!host_avg && small_fault) return small_fault_error();
     nashconv_from_sums(sc, pct, nash, br, cur, deal_mass);
     return SS_OK;
 }
@@ -686,11 +720,7 @@ int session_create(const Problem &pb, const SolveConfig &cfg, Session **out) {
 
 int session_run(Session *s, int iters) { return s->run(iters); }
 
-int session_sync(Session *s) {
-    CK(cudaSetDevice(s->device));
-    CK(cudaStreamSynchronize(s->stream));
-    return SS_OK;
-}
+int session_sync(Session *s) { return s->sync(); }
 
 int session_reset(Session *s) { return s->reset(); }
 int session_iterations(const Session *s) { return s->iterations; }
@@ -703,6 +733,7 @@ int session_exploitability(Session *s, const float *host_avg, double *pct, doubl
                            double *cur, double *z) {
     return s->exploitability(host_avg, pct, nash, br, cur, z);
 }
+void session_set_wait_limit(Session *s, unsigned polls) { s->small.polls = polls; }
 void session_destroy(Session *s) { delete s; }
 void *session_stream(Session *s) { return static_cast<void *>(s->stream); }
 

@@ -414,6 +414,7 @@ int session_profile(Session *s, SSKernelProfile *prof);
 int session_profile_launches(const Session *s, SSLaunchRecord *rec, int max_records, int *num_records);
 void session_destroy(Session *s);
 void *session_stream(Session *s);
+void session_set_wait_limit(Session *s, unsigned polls);
 int session_exploitability(Session *s, const float *host_avg, double *pct, double *nash, double *br,
                            double *cur, double *z);
 // ss_narrow.cu: the reference's range update from the session's average strategy

@@ -1758,13 +1758,12 @@ __global__ void __launch_bounds__(kSd1Threads, 2) k_term_light(DevCtx c0, const 
 // nodes and 90 hands 35.8 -> 20.3; turn of 1,081 nodes and 1128 hands 58.6 ->
 // 42.5.
 // --------------------------------------------------------------------------
-constexpr unsigned kFaultGridWait = 4u;   // k_small_solve: a grid barrier's wait ran out
-constexpr unsigned kGridPolls = 4u << 20; // polls of the barrier (seconds) before a block gives up
 constexpr int kSmallThreads = kSd1Threads;
 
 // All blocks of the (cooperative) grid; count starts at 0 and grows by
-// gridDim.x per barrier.  False when the wait ran out: the caller returns.
-__device__ bool grid_barrier(unsigned *count) {
+// gridDim.x per barrier.  False when the wait ran out: the fault word is set
+// and the caller returns.
+__device__ bool grid_barrier(unsigned *count, unsigned *fault, unsigned limit) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1772,10 +1771,10 @@ __device__ bool grid_barrier(unsigned *count) {
         asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(count) : "memory");
         const unsigned target = (before / gridDim.x + 1u) * gridDim.x;
         unsigned now = before + 1u, polls = 0;
-        while (static_cast<int>(now - target) < 0 && ++polls < kGridPolls)
+        while (static_cast<int>(now - target) < 0 && polls++ < limit)
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(count) : "memory");
         ok = static_cast<int>(now - target) >= 0;
-        if (!ok) atomicOr(&g_ss_fault, kFaultGridWait);
+        if (!ok) atomicOr(fault, 1u);
     }
     __syncthreads();
     return ok != 0;
@@ -2228,6 +2227,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
     const size_t HS = static_cast<size_t>(c.HS);
     const bool river = s.n_sd1[0] + s.n_sd1[1] > 0, folds = s.n_cr1[0] + s.n_cr1[1] > 0;
     const int hand = threadIdx.x & (kTreeHands - 1), h = blockIdx.x * kTreeHands + hand;
+    if (*s.fault) return;   // an earlier launch gave up: its rows are no state to go on from
     float weight0 = 0.f, weight1 = 0.f;
     // tables and the block's rows
     for (int p = 0; p < 2; ++p) {
@@ -2328,7 +2328,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
                 }
                 if (job + static_cast<int>(gridDim.x) < jobs) __syncthreads();   // the next job's space
             }
-            if (!grid_barrier(s.barrier)) return;
+            if (!grid_barrier(s.barrier, s.fault, s.polls)) return;
             float *R = reinterpret_cast<float *>(smem + s.at.R[t]), *S = reinterpret_cast<float *>(smem + s.at.S[t]);
             // the root strategy before the last traverser's pass
             if (snapshot && it == iters && t == 1) {
@@ -2356,7 +2356,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
             float *rv = reinterpret_cast<float *>(work);
             whole_pass(c, s.tree[t], smem + s.at.tab[t], R, S, rv, rv + s.tree[t].n_rows * kTreeHands, h, h < c.H[t],
                        t ? weight1 : weight0, base + it, it == iters);
-            if (!grid_barrier(s.barrier)) return;
+            if (!grid_barrier(s.barrier, s.fault, s.polls)) return;
         }
     }
     rows(true);

@@ -115,7 +115,10 @@ struct SmallRef {
     const TermItem *sd1[2], *cr1[2], *zero[2];
     int n_sd1[2], n_cr1[2], n_zero[2];
     unsigned *barrier;   // grid barrier count
+    unsigned *fault;     // not 0 once a barrier's wait ran out; the session's own
+    unsigned polls;      // of a barrier before a block gives up
 };
+constexpr unsigned kGridPolls = 4u << 20;   // seconds
 // Lays out s.at and returns the blocks of the cooperative grid; 0 where the
 // device or the shared memory cannot run it.
 int small_solve_blocks(const DevCtx &c, SmallRef *s);

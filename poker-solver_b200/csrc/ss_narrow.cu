@@ -174,7 +174,8 @@ int session_narrow(Session *s, int player, int node, unsigned action_mask, int n
         set_error("ss_session_narrow: action mask outside the node's actions");
         return SS_ERR_INVALID;
     }
-    int rc = SS_OK;
+    int rc = s->small_blocks > 0 ? s->sync() : SS_OK;   // lost sums narrow nothing
+    if (rc != SS_OK) return rc;
     char *buf = nullptr;
     int flag = 0;
     const size_t cb = static_cast<size_t>(n) * 2 * sizeof(int), wb = static_cast<size_t>(n) * sizeof(double);

@@ -61,6 +61,7 @@ class Session {
     TreeRef tree[SS_MAX_PLAYERS] = {};
     SmallRef small{};         // small heads-up subgames: iterations in one cooperative kernel
     int small_blocks = 0;     // its grid; 0: the captured iterations run
+    unsigned small_fault = 0; // its fault word as last read: set until the state is reset
     const TermItem *term_items[SS_MAX_PLAYERS][TK_COUNT] = {};
     const int *term_heads[SS_MAX_PLAYERS][TK_COUNT] = {};   // null for kinds without P.term_heads
     const int *root_fr[SS_MAX_PLAYERS] = {};
@@ -305,6 +306,9 @@ class Session {
     int reset();
     int run(int iters);
     int output(SSOutput *out);
+    int sync();
+    int small_fault_error();          // the error of a session whose wait ran out
+    cudaError_t fetch_small_fault();  // queues the read of the fault word (small sessions)
     int profile(SSKernelProfile *prof);
     int profile_launches(SSLaunchRecord *rec, int max_records, int *num_records) const;
 };
