@@ -2422,6 +2422,12 @@ constexpr size_t sd2_smem(int span, int ncomb) {
            sd2_reach_bytes<T>(ncomb) + static_cast<size_t>(ncomb) * 2 + static_cast<size_t>(span) * 2 + 16 +
            2 * SD2_W * 4 + 2 * 48 * 8 + 17 * 16;
 }
+// Rank positions of any board.  The attribute that allows a launch its shared
+// memory is one per kernel, for all host threads: it is set to what the largest
+// launch takes, never to this launch's size, which another thread's may exceed
+// by the time that it launches.
+constexpr int kMaxSpan = 1326;
+static_assert(sd2_smem<double>(kMaxSpan, kMaxSpan) <= 227 * 1024, "one block fits");
 
 struct Sd2State {
     double *P, *u1, *u2, *w, *d, *sc;   // sc: F1, F2, Q, D
@@ -4225,7 +4231,8 @@ cudaError_t launch_terms_t(const DevCtx &c, int kind, const TermItem *items, int
             // runs per block: about two waves of four blocks per SM at most
             const int lgm = sd2_merge_of(n);
             const size_t sm = sd2_smem<T>(c.sd_span[lgm], c.ncomb);
-            e = cudaFuncSetAttribute(k_term_sd2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+            e = cudaFuncSetAttribute(k_term_sd2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(sd2_smem<T>(kMaxSpan, kMaxSpan)));
             if (e != cudaSuccess) return e;
             SSB_LAUNCH(k_term_sd2<T>, n * (kSd2Chunks >> lgm), kTermThreads, sm, s, c, ctxs, items, trav, lgm, nullptr);
             break;
@@ -4288,8 +4295,8 @@ cudaError_t launch_sd2_mapped_t(const DevCtx &c, const TermItem *items, const in
                                 int trav, cudaStream_t s, const DevCtx *ctxs) {
     if (nblocks <= 0) return cudaSuccess;
     const size_t sm = sd2_smem<T>(c.sd_span[lg_max], c.ncomb);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_term_sd2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+    cudaError_t e = cudaFuncSetAttribute(k_term_sd2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(sd2_smem<T>(kMaxSpan, kMaxSpan)));
     if (e != cudaSuccess) return e;
     SSB_LAUNCH(k_term_sd2<T>, nblocks, kTermThreads, sm, s, c, ctxs, items, trav, 0, bmap);
     return cudaGetLastError();
