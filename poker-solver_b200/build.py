@@ -22,7 +22,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
 ENGINE = ["ss_tree.cpp", "ss_plan.cpp", "ss_kernels.cu", "ss_engine.cu", "ss_rank_kernels.cu", "ss_noalloc.cu", "ss_batch.cu",
           "ss_leaf_plan.cpp", "ss_leaf.cu", "ss_stage.cu", "ss_narrow.cu", "fs_tree.cpp", "fs_engine.cu", "fs_abi.cpp"]
-HEADERS = ["ss_engine.h", "ss_kernels.h", "ss_rank.cuh", "ss_session.h", "ss_leaf.h", "ss_leaf.cuh", "ss_stage.h", "ss_runs.h", "fs_engine.h",
+HEADERS = ["ss_engine.h", "ss_kernels.h", "ss_rank.cuh", "ss_session.h", "ss_leaf.h", "ss_leaf.cuh", "ss_stage.h", "ss_runs.h", "ss_shares.h", "fs_engine.h",
            "ss_cr2_tc.cuh", "ss_cr3.cuh", "ss_triple.cuh"]
 VARIANTS = {"libstreet_solve.so": 200, "libstreet_solve_wide.so": 1326}
 

@@ -2,12 +2,11 @@
 #include "ss_stage.h"
 
 #include "ss_engine.h"
+#include "ss_shares.h"
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 namespace ssb {
 
@@ -76,24 +75,13 @@ cudaError_t staged(Way way, void *dst, const void *src, size_t bytes, cudaStream
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) {
         const size_t share = (bytes / nt + kPiece - 1) / kPiece * kPiece;   // whole pieces; the last takes the rest
-        std::vector<cudaError_t> got(nt, cudaSuccess);
-        std::vector<std::thread> threads;
-        auto run = [&](int i) {
+        cudaError_t got[kMaxThreads] = {};
+        run_shares<kMaxThreads>(nt, [&](int i) {
             const size_t at = std::min(bytes, share * i), end = i + 1 == nt ? bytes : std::min(bytes, share * (i + 1));
             if (at < end)
                 got[i] = move_share(way, device, static_cast<char *>(dst) + at, static_cast<const char *>(src) + at,
                                     end - at, buf + 2 * kPiece * i, s);
-        };
-        threads.reserve(nt);
-        int started = 1;
-        try {
-            for (; started < nt; ++started) threads.emplace_back(run, started);
-        } catch (const std::system_error &) {
-            // no more threads: this one takes the shares left
-        }
-        run(0);
-        for (int i = started; i < nt; ++i) run(i);
-        for (std::thread &t : threads) t.join();
+        });
         for (cudaError_t g : got)
             if (e == cudaSuccess) e = g;
     }
