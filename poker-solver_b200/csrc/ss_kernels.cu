@@ -1559,15 +1559,18 @@ constexpr size_t sd1_smem() {
 // A traverser hand with no compatible positive-reach opponent hand gets
 // exactly 0 (positive-reach masks per card, as in the two-opponent kernels).
 //
-// Latency-bound: a heads-up river launches tens of these blocks and waits for
-// one.  1024 threads: eight warps scan the rank positions while the other 24
-// take the cards' lists, and every table that no kernel writes is read before
-// the wait for the previous kernel where a register can hold it.  (Not of a
-// member that has left the batch: its tables are freed.  The live flag is
-// written by a copy, which the kernels' order cannot overtake.)
+// NT = kSd1Threads is for few showdowns, whose launch waits for one block: eight
+// warps scan the rank positions while the other 24 take the cards' lists, and
+// every table that no kernel writes is read before the wait for the previous
+// kernel where a register can hold it.  (Not of a member that has left the
+// batch: its tables are freed.  The live flag is written by a copy, which the
+// kernels' order cannot overtake.)  NT = kTermThreads is for many, where five
+// small blocks per SM do more than two large ones: one step after the other,
+// the reach scattered hand by hand (a narrow range touches its own hands, not
+// every position).  Same sums in the same order.
 constexpr int kSd1Threads = 1024;
 constexpr int kSd1Scan = 256;   // threads of the rank-order scan (fixes its summation order)
-template <class T>
+template <int NT, class T>
 __device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__restrict__ ctxs,
                                              const TermItem *__restrict__ item, int trav, char *smem) {
     Carve cv{smem};
@@ -1586,26 +1589,33 @@ __device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__r
     const int *ph = c.pos_hand + static_cast<size_t>(o) * nc;
     const int *tpos = c.sd_pos + static_cast<size_t>(trav) * HS;
     const bool gone = retired(ctxs, I.sg);
-    const int ph0 = !gone && tid < nc ? __ldg(ph + tid) : -1;
-    const int q0 = !gone && tid < Ht ? __ldg(tpos + tid) : -1;
+    constexpr bool kFew = NT > kSd1Scan;
+    const int ph0 = kFew && !gone && tid < nc ? __ldg(ph + tid) : -1;
+    const int q0 = kFew && !gone && tid < Ht ? __ldg(tpos + tid) : -1;
     wait_prior_grid();
     if (gone) return;
     const T *r = reach_rows<T>(c) + static_cast<size_t>(I.opp_row[0]) * HS;
-    if (!dup) {
+    if (kFew && !dup) {
         // the opponent's reach by rank position, gathered
-        for (int q = tid; q < nc; q += kSd1Threads) {
+        for (int q = tid; q < nc; q += NT) {
             const int j = q == tid ? ph0 : __ldg(ph + q);
             Rr[q] = j >= 0 ? r[j] : T(0);
         }
     } else {
-        for (int i = tid; i < nc; i += kSd1Threads) Rr[i] = T(0);
+        for (int i = tid; i < nc; i += NT) Rr[i] = T(0);
         __syncthreads();
         const int *pos = c.sd_pos + static_cast<size_t>(o) * HS;
-        for (int j = tid; j < c.H[o]; j += kSd1Threads)
-            if (pos[j] >= 0) atomicAdd(&Rr[pos[j]], r[j]);
+        for (int j = tid; j < c.H[o]; j += NT) {
+            const int q = pos[j];
+            if (q < 0) continue;
+            if (dup)
+                atomicAdd(&Rr[q], r[j]);
+            else
+                Rr[q] = r[j];
+        }
     }
     __syncthreads();
-    if (warp < kSd1Scan / 32) {
+    if (!kFew || warp < kSd1Scan / 32) {
         // exclusive prefix over rank positions: each thread scans a contiguous chunk
         const int per = (nc + kSd1Scan - 1) / kSd1Scan;
         const int b0 = tid * per, b1 = min(nc, b0 + per);
@@ -1631,10 +1641,12 @@ __device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__r
             for (int w = 0; w < kSd1Scan / 32; ++w) tot += wsum[w];
             Pp[nc] = tot;
         }
-    } else {
+    }
+    if (!kFew || warp >= kSd1Scan / 32) {
         // per card: exclusive prefix sums over its combos in rank order, and
         // the mask of partner cards whose combo holds positive reach
-        for (int card = warp - kSd1Scan / 32; card < 52; card += (kSd1Threads - kSd1Scan) / 32) {
+        constexpr int kFirst = kFew ? kSd1Scan / 32 : 0;
+        for (int card = warp - kFirst; card < 52; card += NT / 32 - kFirst) {
             const short *L = c.sd_card_list + card * 52;
             const short *Pt = c.sd_card_partner + card * 52;
             const int i0 = 2 * lane, i1 = 2 * lane + 1;
@@ -1673,9 +1685,9 @@ __device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__r
     // its class exactly, as in the reference's sum
     const double cw = static_cast<double>(I.pot - I.bet), ct = static_cast<double>(I.pot * 0.5f - I.bet);
     const double cl = -static_cast<double>(I.bet);
-    for (int h = tid; h < HS; h += kSd1Threads) {
+    for (int h = tid; h < HS; h += NT) {
         double v = 0.0;
-        const int q = h == tid ? q0 : h < Ht ? __ldg(tpos + h) : -1;
+        const int q = kFew && h == tid ? q0 : h < Ht ? __ldg(tpos + h) : -1;
         if (q >= 0) {
             const SdCombo s = c.sd_combo[q];
             const unsigned long long B1 = B[s.c1], B2 = B[s.c2];
@@ -1693,11 +1705,11 @@ __device__ __forceinline__ void sd1_terminal(const DevCtx &c0, const DevCtx *__r
     }
 }
 
-template <class T>
-__global__ void __launch_bounds__(kSd1Threads, 2) k_term_sd1(DevCtx c0, const DevCtx *__restrict__ ctxs,
-                                                          const TermItem *__restrict__ items, int trav) {
+template <int NT, class T>
+__global__ void __launch_bounds__(NT, NT == kSd1Threads ? 2 : 5) k_term_sd1(DevCtx c0, const DevCtx *__restrict__ ctxs,
+                                                                          const TermItem *__restrict__ items, int trav) {
     extern __shared__ __align__(16) char smem[];
-    sd1_terminal<T>(c0, ctxs, items + blockIdx.x, trav, smem);
+    sd1_terminal<NT, T>(c0, ctxs, items + blockIdx.x, trav, smem);
 }
 
 // Two-way showdowns, one-opponent folds and zero rows of a river in one
@@ -1715,7 +1727,7 @@ __global__ void __launch_bounds__(kSd1Threads, 2) k_term_light(DevCtx c0, const 
     extern __shared__ __align__(16) char smem[];
     int b = blockIdx.x;
     if (b < n_sd1) {
-        sd1_terminal<float>(c0, ctxs, sd1 + b, trav, smem);
+        sd1_terminal<kSd1Threads, float>(c0, ctxs, sd1 + b, trav, smem);
         return;
     }
     wait_prior_grid();
@@ -4221,11 +4233,11 @@ cudaError_t launch_terms_t(const DevCtx &c, int kind, const TermItem *items, int
             break;
         }
         case TK_SD1:
-            if (sd1_smem<T>() > 48 * 1024)
-                e = cudaFuncSetAttribute(k_term_sd1<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(sd1_smem<T>()));
-            if (e != cudaSuccess) return e;
-            SSB_LAUNCH(k_term_sd1<T>, n, kSd1Threads, sd1_smem<T>(), s, c, ctxs, items, trav);
+            static_assert(sd1_smem<T>() <= 48 * 1024, "no attribute needed");
+            if (n <= kSd1Few)
+                SSB_LAUNCH((k_term_sd1<kSd1Threads, T>), n, kSd1Threads, sd1_smem<T>(), s, c, ctxs, items, trav);
+            else
+                SSB_LAUNCH((k_term_sd1<kTermThreads, T>), n, kTermThreads, sd1_smem<T>(), s, c, ctxs, items, trav);
             break;
         case TK_SD2: {
             // runs per block: about two waves of four blocks per SM at most

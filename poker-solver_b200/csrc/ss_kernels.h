@@ -78,6 +78,12 @@ constexpr int kHandThreads = 64;
 constexpr int kHandsPerBlock = kHandThreads * 4;
 // threads per block of the per-terminal kernels
 constexpr int kTermThreads = 256;
+// two-way showdowns up to which a launch has blocks of 1024 threads: two per
+// SM, so that all run at once.  Microseconds per launch with small / large
+// blocks, 90 hands: 8.3 / 6.0 at 47, 10.4 / 8.2 at 188, 11.3 / 12.5 at 376,
+// 44.8 / 65.6 at 3008; 1081 hands: 13.2 / 8.1, 17.4 / 13.1, 18.8 / 19.0, 85.5 /
+// 104.7.
+constexpr int kSd1Few = 2 * 148;
 
 // With ctxs (a device array) every item reads the context of its subgame
 // (item.sg) and covers that subgame's hands of `player` / `trav`; without,

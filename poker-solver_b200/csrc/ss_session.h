@@ -145,9 +145,11 @@ class Session {
     }
 
     // Where traverser t has two-way showdowns, its one-opponent folds and zero
-    // rows ride in their launch (rivers: tens of short blocks of each kind).
+    // rows ride in their launch (rivers: tens of short blocks of each kind), as
+    // long as that launch has large blocks.
     bool light(int t, int k) const {
-        return !P.term[t][TK_SD1].empty() && (k == TK_SD1 || k == TK_CR1 || k == TK_ZERO);
+        const size_t n = P.term[t][TK_SD1].size();
+        return n > 0 && n <= kSd1Few && (k == TK_SD1 || k == TK_CR1 || k == TK_ZERO);
     }
 
     // traverser t's terminals of kind k (grouped kinds: one block per head)
