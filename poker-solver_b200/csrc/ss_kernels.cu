@@ -3179,10 +3179,10 @@ __global__ void __launch_bounds__(32 * kEnumWarps) k_term_enum(DevCtx c0, const 
 // 384 threads take the 1128 hands of a turn in three rounds of 98 %, and the
 // tables of a 48-card deck (105 KB) leave two blocks per SM (512 and 576
 // threads spill: 1.4x slower).  Measured on the 4-player turn (5,681 nodes,
-// 2,696 terminals): 8.4 ms per launch by conditioning, 0.5 ms in the first
-// iterations, 0.9 ms where play has become near pure and many hands need the
-// exact look; at 32 hands, where the tables are the work, 0.18 ms by
-// conditioning and 0.146 ms (0.22 before sparse products and split hands).
+// 2,696 terminals), a mean launch of 60 iterations by conditioning on every
+// third hand and now: 8.35 and 0.69 ms at full ranges, 390 and 224 us at 200
+// hands, 158 and 133 us at 60, 118 and 104 us at 24, where the tables are the
+// work (165 and 133 us at 60 and 24 while every pair of cards was looked up).
 constexpr int kCr3Threads = 384;
 static_assert(kMaxHS <= 14 * (kCr3Threads / 4), "a thread's rounds fit a mask");
 // blocks a launch is brought to by sharing a group's hands between blocks (each
@@ -3229,9 +3229,14 @@ __global__ void __launch_bounds__(kCr3Threads, 2) k_term_cr3(DevCtx c0, const De
     const int *code3 = c.hand_code + static_cast<size_t>(o3) * hs;
     const int H3 = c.H[o3];
     const bool dup3 = c.dup[o3] != 0;
-    tri::phase_gather(tid, kCr3Threads, t, r1, r2, r3, c.pair_idx + static_cast<size_t>(o1) * 52 * 52,
-                      c.pair_idx + static_cast<size_t>(o2) * 52 * 52, c.pair_idx + static_cast<size_t>(o3) * 52 * 52,
-                      HS, !dup3);
+    tri::phase_clear(tid, kCr3Threads, t);
+    __syncthreads();
+    {
+        const T *const r[3] = {r1, r2, r3};
+        const int *const code[3] = {c.hand_code + static_cast<size_t>(o1) * hs, c.hand_code + static_cast<size_t>(o2) * hs, code3};
+        const int H[3] = {c.H[o1], c.H[o2], H3};
+        tri::phase_scatter(tid, kCr3Threads, t, r, code, H, !dup3);
+    }
     __syncthreads();
     if (dup3) {
         tri::phase_gather_third(tid, kCr3Threads, t, r3, code3, H3);

@@ -70,55 +70,61 @@ SSB_TRI_HD Tables tables(double *mem, int n) {
     return t;
 }
 
-// phase 1: the matrices from the opponents' pair tables ([52][52] dense pair
-// -> range index, HS if none); the dummy row and column are zero.  Without
-// `third` (a third range that repeats a combo) C is left to
-// phase_gather_third.  On the device a warp fills whole rows and takes the
-// row's nonzero cells from ballots; on the host one item is a row.
+// phase 1: the matrices of the opponents' hands with reach, written hand by
+// hand over cleared ones (3 x 1128 hands at most; looking every pair of cards
+// up took 9 K cycles of a block).  The first two ranges repeat no combo.
+// Without `third` (a third range that does) C is left to phase_gather_third.
+// t.m: the nonzero cells of each row.
+SSB_TRI_HD void phase_clear(int tid, int nt, const Tables &t) {
+    for (int i = tid; i < 3 * t.S * t.S; i += nt) t.A[i] = 0.0;   // A, B, C lie in a row
+    for (int i = tid; i < 3 * kVS; i += nt) t.m[i] = 0ull;
+}
+SSB_TRI_HD void mark(unsigned long long *row, int x) {
+#if defined(__CUDA_ARCH__)
+    atomicOr(reinterpret_cast<unsigned *>(row) + (x >> 5), 1u << (x & 31));   // (64 bits would be a loop)
+#else
+    *row |= 1ull << x;
+#endif
+}
 template <class T>
-SSB_TRI_HD void cell(const Tables &t, int x, int y, const T *r1, const T *r2, const T *r3, const int *pair1,
-                     const int *pair2, const int *pair3, int HS, bool third, double v[3]) {
-    v[0] = v[1] = v[2] = 0.0;
-    if (x < t.n && y < t.n) {
-        const int j1 = pair1[x * 52 + y], j2 = pair2[x * 52 + y], j3 = third ? pair3[x * 52 + y] : HS;
-        if (j1 < HS) v[0] = static_cast<double>(r1[j1]);
-        if (j2 < HS) v[1] = static_cast<double>(r2[j2]);
-        if (j3 < HS && r3[j3] > T(0)) v[2] = static_cast<double>(r3[j3]);
-    }
-    if (y <= t.n) {
-        t.A[x * t.S + y] = v[0];
-        t.B[x * t.S + y] = v[1];
-        t.C[x * t.S + y] = v[2];
+SSB_TRI_HD void phase_scatter(int tid, int nt, const Tables &t, const T *const r[3], const int *const code[3],
+                              const int H[3], bool third) {
+    const int n = H[0] + H[1] + (third ? H[2] : 0);
+#pragma unroll 4
+    for (int i = tid; i < n; i += nt) {
+        const int o = i < H[0] ? 0 : i < H[0] + H[1] ? 1 : 2;
+        const int h = i - (o > 0 ? H[0] : 0) - (o > 1 ? H[1] : 0);
+        const int c = (o == 0 ? code[0] : o == 1 ? code[1] : code[2])[h];
+        const T v = (o == 0 ? r[0] : o == 1 ? r[1] : r[2])[h];
+        if ((c & 0x10000) || v == T(0) || (o == 2 && !(v > T(0)))) continue;   // touches the board, or nothing to add
+        const int x = (c >> 20) & 63, y = (c >> 26) & 63;
+        double *M = o == 0 ? t.A : o == 1 ? t.B : t.C;
+        M[x * t.S + y] = M[y * t.S + x] = static_cast<double>(v);
+        mark(t.m + o * kVS + x, y);
+        mark(t.m + o * kVS + y, x);
     }
 }
+// The same from the pair tables ([52][52] dense pair -> range index, HS if
+// none), row by row: what the host checks hold the scatter against.
 template <class T>
 SSB_TRI_HD void phase_gather(int tid, int nt, const Tables &t, const T *r1, const T *r2, const T *r3,
                              const int *pair1, const int *pair2, const int *pair3, int HS, bool third) {
-#if defined(__CUDA_ARCH__)
-    const int lane = tid & 31;
-#pragma unroll 2
-    for (int x = tid >> 5; x <= t.n; x += nt >> 5) {
-        unsigned long long m[3] = {0ull, 0ull, 0ull};
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            double v[3];
-            cell(t, x, half * 32 + lane, r1, r2, r3, pair1, pair2, pair3, HS, third, v);
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-                m[i] |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, v[i] != 0.0)) << (32 * half);
-        }
-        if (lane < 3) t.m[lane * kVS + x] = lane == 0 ? m[0] : lane == 1 ? m[1] : m[2];
-    }
-#else
     for (int x = tid; x <= t.n; x += nt) {
         for (int i = 0; i < 3; ++i) t.m[i * kVS + x] = 0ull;
         for (int y = 0; y <= t.n; ++y) {
-            double v[3];
-            cell(t, x, y, r1, r2, r3, pair1, pair2, pair3, HS, third, v);
+            double v[3] = {0.0, 0.0, 0.0};
+            if (x < t.n && y < t.n) {
+                const int j1 = pair1[x * 52 + y], j2 = pair2[x * 52 + y], j3 = third ? pair3[x * 52 + y] : HS;
+                if (j1 < HS) v[0] = static_cast<double>(r1[j1]);
+                if (j2 < HS) v[1] = static_cast<double>(r2[j2]);
+                if (j3 < HS && r3[j3] > T(0)) v[2] = static_cast<double>(r3[j3]);
+            }
+            t.A[x * t.S + y] = v[0];
+            t.B[x * t.S + y] = v[1];
+            t.C[x * t.S + y] = v[2];
             for (int i = 0; i < 3; ++i) t.m[i * kVS + x] |= static_cast<unsigned long long>(v[i] != 0.0) << y;
         }
     }
-#endif
 }
 
 // phase 1 continued, for a third range that repeats a combo: its hands add up
@@ -232,15 +238,33 @@ SSB_TRI_HD void phase_vectors(int tid, int nt, const Tables &t) {
     }
 }
 
-// phase 4: the scalars, one item each
+// phase 4: the scalars, each in sum4's order; on the device four lanes take the
+// four partial sums (one thread per scalar: 3 K cycles of waiting for it)
 SSB_TRI_HD void phase_scalars(int tid, int nt, const Tables &t) {
-    for (int k = tid; k < N_SCAL; k += nt) {
+    auto term = [&](int k, int c) {
         const int p = k == QAB || k == QAC ? UA : k == QBC ? UB : -1, q = k == QAB ? UB : UC;
         const int one = k < 3 ? UA + k : k >= EAB && k <= EBC ? DAB + (k - EAB) : k == SH ? HH : TABC;
-        const double s = p >= 0 ? sum4(t.n, [&](int c) { return t.v[p * kVS + c] * t.v[q * kVS + c]; })
-                                : sum4(t.n, [&](int c) { return t.v[one * kVS + c]; });
-        t.sc[k] = k < 3 || (k >= EAB && k <= EBC) ? 0.5 * s : s;
+        return p >= 0 ? t.v[p * kVS + c] * t.v[q * kVS + c] : t.v[one * kVS + c];
+    };
+    auto put = [&](int k, double s) { t.sc[k] = k < 3 || (k >= EAB && k <= EBC) ? 0.5 * s : s; };
+#if defined(__CUDA_ARCH__)
+    const int part = tid & 3, n4 = t.n & ~3;
+    for (int base = (tid >> 5) * 8; base < N_SCAL; base += nt >> 2) {
+        const int k = base + ((tid & 31) >> 2);
+        double s = 0.0;
+        if (k < N_SCAL) {
+#pragma unroll 4
+            for (int c = part; c < n4; c += 4) s += term(k, c);
+            if (part == 0)
+                for (int c = n4; c < t.n; ++c) s += term(k, c);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (part == 0 && k < N_SCAL) put(k, s);
     }
+#else
+    for (int k = tid; k < N_SCAL; k += nt) put(k, sum4(t.n, [&](int c) { return term(k, c); }));
+#endif
 }
 
 // The mass of one traverser hand with dense cards (a, b): the sums over the
@@ -358,39 +382,70 @@ SSB_TRI_HD int popc(unsigned long long x) {
 #endif
 }
 SSB_TRI_HD void phase_masks(int tid, int nt, const Tables &t, const Counts &k) {
+    auto put = [&](int c, unsigned long long a, unsigned long long b) {
+        k.mA[c] = a;
+        k.mB[c] = b;
+        k.nA[c] = popc(a);
+        k.nB[c] = popc(b);
+        k.nD[c] = popc(a & b);
+    };
+#if defined(__CUDA_ARCH__)
+    const int lane = tid & 31;   // a warp per row
+    for (int c = tid >> 5; c <= t.n; c += nt >> 5) {
+        unsigned long long a = 0ull, b = 0ull;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int x = half * 32 + lane;
+            a |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, x < t.n && t.A[c * t.S + x] > 0.0)) << (32 * half);
+            b |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, x < t.n && t.B[c * t.S + x] > 0.0)) << (32 * half);
+        }
+        if (lane == 0) put(c, a, b);
+    }
+#else
     for (int c = tid; c <= t.n; c += nt) {
         unsigned long long a = 0ull, b = 0ull;
         for (int x = 0; x < t.n; ++x) {
             a |= static_cast<unsigned long long>(t.A[c * t.S + x] > 0.0) << x;
             b |= static_cast<unsigned long long>(t.B[c * t.S + x] > 0.0) << x;
         }
-        k.mA[c] = a;
-        k.mB[c] = b;
-        k.nA[c] = popc(a);
-        k.nB[c] = popc(b);
-        k.nD[c] = popc(a & b);
+        put(c, a, b);
     }
+#endif
 }
 SSB_TRI_HD void phase_counts(int tid, int nt, const Tables &t, const Counts &k) {
+    // whole numbers, below 52^3
+    auto w = [&](int c, int x) {
+        return x >= t.n ? 0 : ((k.mB[c] >> x) & 1ull ? k.nA[x] : 0) + ((k.mA[c] >> x) & 1ull ? k.nB[x] : 0);
+    };
+    auto total = [&](int i, int c) {
+        return c >= t.n ? 0 : i == 0 ? k.nA[c] : i == 1 ? k.nB[c] : i == 2 ? k.nA[c] * k.nB[c] : k.nD[c];
+    };
+    auto put = [&](int i, int s) { k.s[i] = i == 2 ? s : s / 2; };
+#if defined(__CUDA_ARCH__)
+    const int lane = tid & 31;   // a warp per sum
+    for (int c = tid >> 5; c <= t.n + 4; c += nt >> 5) {
+        const bool row = c <= t.n;
+        const int i = c - t.n - 1;
+        const int s = __reduce_add_sync(0xffffffffu, row ? w(c, lane) + w(c, lane + 32) : total(i, lane) + total(i, lane + 32));
+        if (lane > 0) continue;
+        if (row)
+            k.nW[c] = s;
+        else
+            put(i, s);
+    }
+#else
     for (int c = tid; c <= t.n; c += nt) {
-        int w = 0;
-        for (int x = 0; x < t.n; ++x)
-            w += ((k.mB[c] >> x) & 1ull ? k.nA[x] : 0) + ((k.mA[c] >> x) & 1ull ? k.nB[x] : 0);
-        k.nW[c] = w;
+        int s = 0;
+        for (int x = 0; x < t.n; ++x) s += w(c, x);
+        k.nW[c] = s;
     }
-    if (tid == nt - 1) {
-        long long fa = 0, fb = 0, q = 0, e = 0;
-        for (int c = 0; c < t.n; ++c) {
-            fa += k.nA[c];
-            fb += k.nB[c];
-            q += static_cast<long long>(k.nA[c]) * k.nB[c];
-            e += k.nD[c];
+    if (tid == nt - 1)
+        for (int i = 0; i < 4; ++i) {
+            int s = 0;
+            for (int c = 0; c < t.n; ++c) s += total(i, c);
+            put(i, s);
         }
-        k.s[0] = fa / 2;
-        k.s[1] = fb / 2;
-        k.s[2] = q;
-        k.s[3] = e / 2;
-    }
+#endif
 }
 template <class T>
 SSB_TRI_HD bool tuple_with(int a, int b, const Counts &k, T r, int code) {
