@@ -447,9 +447,10 @@ __global__ void __launch_bounds__(kFsThreads) k_fs_tables(const int *__restrict_
         }
 }
 
-// Terminals: one warp per terminal and no block barriers (a block per terminal
-// spent its time waiting at three of them: 764 us for 113,488 folds, 640 us
-// for 152,880 showdowns of 200 hands; now 182 and 374 us).  What the terminals of a block share
+// Terminals, where a launch has many: one warp per terminal and no block
+// barriers (a block per terminal spends its time waiting at three of them: 764 us
+// for 113,488 folds, 640 us for 152,880 showdowns of 200 hands; a warp each 182
+// and 374 us).  What the terminals of a block share
 // sits in shared memory: the ranges' tables (folds), one river board's tables
 // (showdowns).  Every sum keeps a fixed order: positions or hands in runs per
 // lane, lists in list order.
@@ -565,8 +566,9 @@ __global__ void __launch_bounds__(kFsThreads) k_fs_fold(const FsTermItem *__rest
 // holding one of its two cards (their own prefix sums along each card's
 // list); value = (W - L) x half_pot, FP64 sums.  The same on 0/1 counts
 // gives exactly 0 where no positive-reach opponent hand wins or loses.
-// One block per river board: its terminals [bstart[b], bstart[b + 1]) are
-// consecutive items.
+// A river board's terminals [bstart[b], bstart[b + 1]) are consecutive items,
+// shared by `split` blocks (a tree from the turn or the river on has few boards
+// with many terminals each).
 //
 // Bound by shared-memory wavefronts, so the zero test keeps no counts beside
 // the sums: a W or L above 1e-9 of the opponent's whole reach cannot be the
@@ -583,7 +585,7 @@ constexpr size_t fs_sd_smem() {
            (FS_MAX_HANDS + 2 * FS_MAX_HANDS + 64 + FS_MAX_HANDS) * sizeof(short) + 16;
 }
 __global__ void __launch_bounds__(kFsThreads) k_fs_showdown(const FsTermItem *__restrict__ items,
-                                                           const int *__restrict__ bstart, int trav,
+                                                           const int *__restrict__ bstart, int split, int trav,
                                                            const float *__restrict__ reach, FsTables T,
                                                            float *__restrict__ out, int scaled) {
     extern __shared__ __align__(16) char smem[];
@@ -597,7 +599,10 @@ __global__ void __launch_bounds__(kFsThreads) k_fs_showdown(const FsTermItem *__
     const int Ho = opp == 0 ? T.H0 : T.H1, Ht = trav == 0 ? T.H0 : T.H1;
     const size_t hs = static_cast<size_t>(T.HS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const size_t bo = static_cast<size_t>(blockIdx.x) * 2 + opp, bt = static_cast<size_t>(blockIdx.x) * 2 + trav;
+    const int board = blockIdx.x / split, share = blockIdx.x - board * split;
+    const int first = bstart[board] + share * kFsWarps, end = bstart[board + 1];
+    if (first >= end) return;
+    const size_t bo = static_cast<size_t>(board) * 2 + opp, bt = static_cast<size_t>(board) * 2 + trav;
     for (int i = tid; i < 52 * kFsRun; i += kFsThreads) cmask[i] = 0u;
     if (tid < Ho) {
         const int o = T.sd_ord[bo * hs + tid];
@@ -615,7 +620,7 @@ __global__ void __launch_bounds__(kFsThreads) k_fs_showdown(const FsTermItem *__
         for (int k = off[tid]; k < off[tid + 1]; ++k) cmask[tid * kFsRun + list[k] % kFsRun] |= 1u << (list[k] / kFsRun);
     __syncthreads();
     FsSdWarp &W = all[warp];
-    for (int i = bstart[blockIdx.x] + warp; i < bstart[blockIdx.x + 1]; i += kFsWarps) {
+    for (int i = first + warp; i < end; i += split * kFsWarps) {
         const FsTermItem &I = items[i];
         const float *row = reach + static_cast<size_t>(I.opp_row) * hs;
         // the opponent's reach by position (0 where the board blocks the
@@ -704,6 +709,179 @@ __global__ void __launch_bounds__(kFsThreads) k_fs_showdown(const FsTermItem *__
         }
         __syncwarp();
     }
+}
+
+// The same values (same sums, same order) by a block per terminal, for launches
+// of few of them, which wait for one terminal and not for all: the hands and
+// the cards of a terminal are spread over the block, and nothing is brought to
+// shared memory but what the terminal computes.
+__global__ void __launch_bounds__(kFsThreads) k_fs_fold_few(const FsTermItem *__restrict__ items, int trav,
+                                                           const float *__restrict__ reach, FsTables T,
+                                                           float *__restrict__ out, int scaled) {
+    __shared__ double r_o[FS_MAX_HANDS];
+    __shared__ double u[52], tot[kFsWarps];
+    __shared__ int cu[52], ctot[kFsWarps];
+    const FsTermItem I = items[blockIdx.x];
+    const int opp = 1 - trav;
+    const int Ho = opp == 0 ? T.H0 : T.H1, Ht = trav == 0 ? T.H0 : T.H1;
+    const size_t hs = static_cast<size_t>(T.HS);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int *cl = T.f_clist + opp * 2 * T.HS, *coff = T.f_coff + opp * 53;
+    double f = 0.0;
+    if (tid < Ho) {
+        const int code = T.hand_cards[opp * T.HS + tid];
+        const float r = reach[static_cast<size_t>(I.opp_row) * hs + tid];
+        bool blocked = false;
+        for (int k = 0; k < I.nb; ++k) blocked |= (code & 0xff) == I.board[k] || ((code >> 8) & 0xff) == I.board[k];
+        f = blocked ? 0.0 : static_cast<double>(r);
+        r_o[tid] = f;
+    }
+    const int hc = tid < Ht ? T.hand_cards[trav * T.HS + tid] : 0, so = tid < Ht ? T.f_same[trav * T.HS + tid] : -1;
+    const int n = __popc(__ballot_sync(0xffffffffu, f > 0.0));
+    for (int k = 16; k > 0; k >>= 1) f += __shfl_xor_sync(0xffffffffu, f, k);
+    if (lane == 0) {
+        tot[warp] = f;
+        ctot[warp] = n;
+    }
+    __syncthreads();
+    if (tid < 52) {
+        double s = 0.0;
+        int m = 0;
+        for (int k = coff[tid]; k < coff[tid + 1]; ++k) {
+            const double r = r_o[cl[k]];
+            s += r;
+            m += r > 0.0 ? 1 : 0;
+        }
+        u[tid] = s;
+        cu[tid] = m;
+    }
+    __syncthreads();
+    static_assert(FS_MAX_HANDS <= kFsThreads, "a thread per hand");
+    if (tid >= Ht) return;
+    double F = 0.0;
+    int CF = 0;
+    for (int w = 0; w < kFsRun; ++w) {
+        F += tot[w];
+        CF += ctot[w];
+    }
+    const int a = hc & 0xff, b = (hc >> 8) & 0xff;
+    double same = 0.0;
+    int csame = 0;
+    if (!T.dup[opp]) {
+        same = so >= 0 ? r_o[so] : 0.0;
+        csame = same > 0.0 ? 1 : 0;
+    } else {
+        for (int k = coff[a]; k < coff[a + 1]; ++k) {
+            const int o = cl[k], oc = T.hand_cards[opp * T.HS + o];
+            if ((oc & 0xff) != b && ((oc >> 8) & 0xff) != b) continue;
+            same += r_o[o];
+            csame += r_o[o] > 0.0 ? 1 : 0;
+        }
+    }
+    const int cnt = CF - cu[a] - cu[b] + csame;
+    const double mass = cnt == 0 ? 0.0 : F - u[a] - u[b] + same;
+    out[static_cast<size_t>(I.node) * hs + tid] = static_cast<float>(mass) * I.payoff * (scaled ? I.scale : 1.0f);
+}
+
+__global__ void __launch_bounds__(kFsThreads) k_fs_showdown_few(const FsTermItem *__restrict__ items, int trav,
+                                                               const float *__restrict__ reach, FsTables T,
+                                                               float *__restrict__ out, int scaled) {
+    __shared__ double P[FS_MAX_HANDS + 1], PC[2 * FS_MAX_HANDS + 52];
+    __shared__ int Pn[FS_MAX_HANDS + 1], PCn[2 * FS_MAX_HANDS + 52];   // the same sums over positive reach
+    __shared__ float x_s[32 * kFsRun];
+    const FsTermItem &I = items[blockIdx.x];
+    const int opp = 1 - trav;
+    const int Ho = opp == 0 ? T.H0 : T.H1, Ht = trav == 0 ? T.H0 : T.H1;
+    const size_t hs = static_cast<size_t>(T.HS);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const size_t bo = static_cast<size_t>(I.sboard) * 2 + opp, bt = static_cast<size_t>(I.sboard) * 2 + trav;
+    const int *coff = T.sd_coff + bo * 53;
+    // the opponent's reach by position (0 where the board blocks the hand)
+    if (tid < 32 * kFsRun) {
+        const int o = tid < Ho ? T.sd_ord[bo * hs + tid] : -1;
+        x_s[tid] = o >= 0 && T.sd_str[bo * hs + o] != 0u ? reach[static_cast<size_t>(I.opp_row) * hs + o] : 0.f;
+    }
+    const bool live = tid < Ht && T.sd_str[bt * hs + tid] != 0u;
+    const int4 hp = live ? reinterpret_cast<const int4 *>(T.sd_hpos)[bt * hs + tid] : make_int4(0, 0, 0, 0);
+    static_assert(32 * kFsRun <= kFsThreads && FS_MAX_HANDS <= kFsThreads, "a thread per hand");
+    __syncthreads();
+    if (warp == 0) {
+        const int k0 = lane * kFsRun;
+        double s = 0.0;
+        int n = 0;
+#pragma unroll
+        for (int j = 0; j < kFsRun; ++j) {
+            s += static_cast<double>(x_s[k0 + j]);
+            n += x_s[k0 + j] > 0.f ? 1 : 0;
+        }
+        double incl = s;
+        int nincl = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const double v = __shfl_up_sync(0xffffffffu, incl, d);
+            const int m = __shfl_up_sync(0xffffffffu, nincl, d);
+            if (lane >= d) {
+                incl += v;
+                nincl += m;
+            }
+        }
+        double run = incl - s;
+        int nrun = nincl - n;
+#pragma unroll
+        for (int j = 0; j < kFsRun; ++j)
+            if (k0 + j < Ho) {
+                P[k0 + j] = run;
+                Pn[k0 + j] = nrun;
+                run += static_cast<double>(x_s[k0 + j]);
+                nrun += x_s[k0 + j] > 0.f ? 1 : 0;
+            }
+        if (lane == 31) {
+            P[Ho] = incl;
+            Pn[Ho] = nincl;
+        }
+    } else if (tid >= 64 && tid < 64 + 52) {
+        const int c = tid - 64, b0 = coff[c], b1 = coff[c + 1];
+        const int *cl = T.sd_clist + bo * 2 * hs;
+        double q = 0.0;
+        int m = 0;
+        PC[b0 + c] = 0.0;
+        PCn[b0 + c] = 0;
+        for (int k = b0; k < b1; ++k) {
+            const float v = x_s[cl[k]];
+            q += static_cast<double>(v);
+            m += v > 0.f ? 1 : 0;
+            PC[k + c + 1] = q;
+            PCn[k + c + 1] = m;
+        }
+    }
+    __syncthreads();
+    if (tid >= Ht) return;
+    float v = 0.f;
+    if (live) {
+        const int lo = hp.x & 0xffff, hi = hp.x >> 16;
+        const int c1 = hp.y & 0xff, c2 = (hp.y >> 8) & 0xff;
+        const int b1 = coff[c1] + c1, e1 = coff[c1 + 1] + c1;
+        const int b2 = coff[c2] + c2, e2 = coff[c2 + 1] + c2;
+        const int l1lo = hp.z & 0xffff, l1hi = hp.z >> 16, l2lo = hp.w & 0xffff, l2hi = hp.w >> 16;
+        double w = P[lo] - PC[b1 + l1lo] - PC[b2 + l2lo];
+        double l = (P[Ho] - P[hi]) - (PC[e1] - PC[b1 + l1hi]) - (PC[e2] - PC[b2 + l2hi]);
+        if (Pn[lo] - PCn[b1 + l1lo] - PCn[b2 + l2lo] == 0) w = 0.0;
+        if ((Pn[Ho] - Pn[hi]) - (PCn[e1] - PCn[b1 + l1hi]) - (PCn[e2] - PCn[b2 + l2hi]) == 0) l = 0.0;
+        v = static_cast<float>((w - l) * static_cast<double>(I.half_pot));
+    }
+    out[static_cast<size_t>(I.node) * hs + tid] = v * (scaled ? I.scale : 1.0f);
+}
+
+// Terminals of a launch up to which each has a block.  Microseconds per launch
+// by block / by warp, 200 hands: folds 3.6 / 5.6 at 4, 5.1 / 6.1 at 292, 6.3 /
+// 6.1 at 484, 40 / 13.9 at 5,596; showdowns 3.7 / 9.5 at 5, 8.6 / 15.4 at 1,296,
+// 18.2 / 21.1 at 3,792, 30.7 / 30.0 at 6,480, 72 / 63 at 16,656.  40 hands: folds
+// 4.4 / 4.4 at 292, showdowns 9.3 / 9.6 at 3,120, 17.2 / 13.4 at 6,480.
+constexpr int kFsFewFolds = 2 * 148, kFsFewShowdowns = 4096;
+// blocks that share a river board's showdowns: as many as it takes to have two
+// per SM, while a warp gets a terminal or more
+inline int fs_split(int showdowns, int boards) {
+    return std::max(1, std::min((2 * 148 + boards - 1) / boards, showdowns / (boards * kFsWarps)));
 }
 
 // the regret-matched strategy of every decision node of player p into
@@ -933,18 +1111,22 @@ class Solve {
     }
 
     cudaError_t terms(int t, float *out, int scaled) {
-        const int nf = P.nfold[t], boards = static_cast<int>(P.bstart.size()) - 1;
-        if (nf > 0) {
+        const int nf = P.nfold[t], ns = static_cast<int>(P.term[t].size()) - nf, boards = static_cast<int>(P.bstart.size()) - 1;
+        if (nf > 0 && nf <= kFsFewFolds) {
+            k_fs_fold_few<<<nf, kFsThreads, 0, stream>>>(term_items[t], t, c.reach, tab, out, scaled);
+        } else if (nf > 0) {
             // eight resident blocks per SM, each over many terminals
             const int grid = std::min((nf + kFsWarps - 1) / kFsWarps, 8 * 148);
             k_fs_fold<<<grid, kFsThreads, 0, stream>>>(term_items[t], nf, t, c.reach, tab, out, scaled);
         }
-        if (boards > 0) {
+        if (ns > 0 && ns <= kFsFewShowdowns) {
+            k_fs_showdown_few<<<ns, kFsThreads, 0, stream>>>(term_items[t] + nf, t, c.reach, tab, out, scaled);
+        } else if (ns > 0) {
             cudaError_t e = cudaFuncSetAttribute(k_fs_showdown, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(fs_sd_smem()));
             if (e != cudaSuccess) return e;
-            k_fs_showdown<<<boards, kFsThreads, fs_sd_smem(), stream>>>(term_items[t] + nf, bstart, t, c.reach, tab, out,
-                                                                       scaled);
+            k_fs_showdown<<<boards * fs_split(ns, boards), kFsThreads, fs_sd_smem(), stream>>>(
+                term_items[t] + nf, bstart, fs_split(ns, boards), t, c.reach, tab, out, scaled);
         }
         return cudaGetLastError();
     }
