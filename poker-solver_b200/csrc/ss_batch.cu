@@ -270,9 +270,17 @@ class Batch {
         }
     }
 
+    // the side streams that the longest run of terminal launches forks onto
     int ensure_sides() {
-        if (!ev_fork) BCK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-        for (int i = 0; i < kSides; ++i) {
+        size_t longest = 1;
+        for (const std::vector<Launch> *q : {&seq, &br_seq})
+            for (size_t i = 0, j; i < q->size(); i = j) {
+                j = run_end(*q, i, terminal);
+                longest = std::max(longest, j - i);
+            }
+        const int sides = std::min<int>(kSides, static_cast<int>(longest) - 1);
+        if (sides > 0 && !ev_fork) BCK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+        for (int i = 0; i < sides; ++i) {
             if (!side[i]) BCK(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
             if (!ev_join[i]) BCK(cudaEventCreateWithFlags(&ev_join[i], cudaEventDisableTiming));
         }
