@@ -191,7 +191,7 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
     Blob b;
     size_t o_heads[SS_MAX_PLAYERS][TK_COUNT] = {};
     size_t o_reach[SS_MAX_PLAYERS], o_cfv[SS_MAX_PLAYERS], o_term[SS_MAX_PLAYERS][TK_COUNT],
-        o_rootfr[SS_MAX_PLAYERS], o_tree[SS_MAX_PLAYERS], o_whole[2] = {};
+        o_rootfr[SS_MAX_PLAYERS], o_tree[SS_MAX_PLAYERS], o_whole[2] = {}, o_small[2] = {};
     for (int p = 0; p < np; ++p) {
         std::vector<ReachItem> all;
         for (auto &lv : P.reach_levels[p]) {
@@ -228,7 +228,14 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
         }
         o_rootfr[p] = b.add(P.root_fr[p]);
         o_tree[p] = b.add(P.tree[p].blob);
-        if (p < 2) o_whole[p] = b.add(P.whole[p].blob);
+        if (p < 2) {
+            o_whole[p] = b.add(P.whole[p].blob);
+            std::vector<int> heads;
+            for (size_t i = 0; !P.whole[p].items.empty() && i < P.term[p][TK_CR1].size(); ++i)
+                if (!P.term[p][TK_CR1][i].follow) heads.push_back(static_cast<int>(i));
+            o_small[p] = b.add(heads);
+            small.n_cr1[p] = static_cast<int>(heads.size());
+        }
     }
     const size_t o_fr_off = b.add(P.fr_off);
     const size_t o_fr_items = b.add(P.fr_items);
@@ -275,9 +282,9 @@ int Session::init(const Problem &pb, const SolveConfig &cfg) {
                                      static_cast<int>(W.reach_off.size()) - 1};
             small.sd1[p] = term_items[p][TK_SD1];
             small.cr1[p] = term_items[p][TK_CR1];
+            small.cr1_head[p] = reinterpret_cast<const int *>(dbase + o_small[p]);
             small.zero[p] = term_items[p][TK_ZERO];
             small.n_sd1[p] = static_cast<int>(P.term[p][TK_SD1].size());
-            small.n_cr1[p] = static_cast<int>(P.term[p][TK_CR1].size());
             small.n_zero[p] = static_cast<int>(P.term[p][TK_ZERO].size());
         }
     }

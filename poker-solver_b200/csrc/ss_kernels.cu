@@ -1983,7 +1983,6 @@ __device__ __forceinline__ void small_sd1(const DevCtx &c, const SmallHand *hand
 // shared memory) by kTermThreads threads with barrier `bar`.
 __device__ __forceinline__ void small_cr1(const DevCtx &c, const unsigned *hands, const short *pair,
                                           const TermItem *__restrict__ I0, int trav, char *smem, int tid, int bar) {
-    if (I0->follow) return;
     constexpr int kRounds = (kMaxHS + kTermThreads - 1) / kTermThreads;
     auto sync = [bar] { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kTermThreads) : "memory"); };
     const int ng = I0->gextra + 1, lane = tid & 31;
@@ -2311,12 +2310,19 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
         first_sd1[threadIdx.x] = s.sd1[threadIdx.x][blockIdx.x];
     const int base = *c.iter;
     const int group = threadIdx.x / kTermThreads, tid = threadIdx.x % kTermThreads;
+    // the first fold or leaf of either traverser is the same every iteration
+    int first_cr1[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int i = (static_cast<int>(blockIdx.x) - s.n_sd1[t]) * s.per_job[t] + group;
+        first_cr1[t] = i >= 0 && i < s.n_cr1[t] ? __ldg(s.cr1_head[t] + i) : 0;
+    }
     char *work = smem + s.at.phase;
     __syncthreads();
     for (int it = 1; it <= iters; ++it) {
         for (int t = 0; t < 2; ++t) {
             const int n_sd1 = s.n_sd1[t], n_cr1 = s.n_cr1[t], n_zero = s.n_zero[t];
-            const int cr1_jobs = (n_cr1 + kLightGroups - 1) / kLightGroups;
+            const int per_job = s.per_job[t], cr1_jobs = (n_cr1 + per_job - 1) / per_job;
             const int jobs = n_sd1 + cr1_jobs + (n_zero + kLightGroups - 1) / kLightGroups;
             for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
                 if (job < n_sd1) {
@@ -2326,10 +2332,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
                               reinterpret_cast<const short *>(smem + s.at.list),
                               reinterpret_cast<const int *>(smem + s.at.clen), job == static_cast<int>(blockIdx.x) ? first_sd1[t] : s.sd1[t][job], t, work);
                 } else if (job < n_sd1 + cr1_jobs) {
-                    const int i = (job - n_sd1) * kLightGroups + group;
-                    if (i < n_cr1)
+                    const int i = (job - n_sd1) * per_job + group;
+                    if (group < per_job && i < n_cr1)
                         small_cr1(c, reinterpret_cast<const unsigned *>(smem + s.at.fold[t]),
-                                  reinterpret_cast<const short *>(smem + s.at.pair[1 - t]), s.cr1[t] + i, t,
+                                  reinterpret_cast<const short *>(smem + s.at.pair[1 - t]),
+                                  s.cr1[t] + (job == static_cast<int>(blockIdx.x) ? first_cr1[t] : __ldg(s.cr1_head[t] + i)), t,
                                   work + group * small_fold_space(c.HS), tid, group + 1);
                 } else {
                     const int i = (job - n_sd1 - cr1_jobs) * kLightGroups + group;
@@ -4151,7 +4158,15 @@ cudaError_t launch_tree(const DevCtx &c, const TreeRef &t, int H, cudaStream_t s
     return cudaGetLastError();
 }
 
-// The grid: a block per 8 hands and per terminal job, at most one per SM.
+// The grid: a block per 8 hands and per terminal job, at most one per SM.  A
+// block takes one group of folds or leaves at a time if that needs no more
+// blocks than the hands do or than half the SMs (so that two sessions run side
+// by side), else two or four.  Groups, not items: the three other continuation
+// choices of a leaf follow its first, and items taken four by four left three
+// of four thread groups idle.  Microseconds per iteration in fours of items and
+// so: heads-up turn of 1,081 nodes 42.2 and 38.9, of 391 nodes and 300 hands
+// 25.6 and 25.9 (half the blocks), river of 51 nodes and 1,081 hands 19.7 and
+// 18.0.
 int small_solve_blocks(const DevCtx &c, SmallRef *ref) {
     SmallRef &s = *ref;
     int dev = 0, coop = 0, sms = 0, optin = 0, per_sm = 0;
@@ -4170,8 +4185,12 @@ int small_solve_blocks(const DevCtx &c, SmallRef *ref) {
     }
     int widest = 1;
     for (int t = 0; t < 2; ++t) {
-        const int jobs = s.n_sd1[t] + (s.n_cr1[t] + kLightGroups - 1) / kLightGroups +
-                         (s.n_zero[t] + kLightGroups - 1) / kLightGroups;
+        const int zeros = (s.n_zero[t] + kLightGroups - 1) / kLightGroups;
+        auto jobs_of = [&](int per) { return s.n_sd1[t] + (s.n_cr1[t] + per - 1) / per + zeros; };
+        const int most = std::max((std::max(c.H[0], c.H[1]) + kTreeHands - 1) / kTreeHands, sms / 2);
+        s.per_job[t] = 1;
+        while (s.per_job[t] < kLightGroups && jobs_of(s.per_job[t]) > most) s.per_job[t] *= 2;
+        const int jobs = jobs_of(s.per_job[t]);
         const int chunks = (c.H[t] + kTreeHands - 1) / kTreeHands;
         if (chunks > sms) return 0;   // a block owns 8 hands for the whole launch
         widest = std::max({widest, jobs, chunks});
