@@ -36,6 +36,15 @@ inline int term_class(int kind) {
     }
 }
 
+// A small subgame that is launched kernel by kernel (Session::crowded): one of
+// more node-hand pairs (nodes x both ranges) than this level by level, a smaller
+// one with its tree passes.  Eight sessions at once, microseconds per iteration
+// of one with tree passes / by level: 6.4 / 18 (51 nodes, 2,162 hands: 110 K
+// pairs), 14.9 / 24 (141, 2,162: 305 K), 32 / 22.6 (1,081, 2,256: 2.4 M).
+constexpr double kLevelsAbove = 6e5;
+// threads of its tree passes then: two blocks per SM
+constexpr int kTreeBeside = 512;
+
 // iterations of a captured graph where `iters` are run, at most `most`
 int graph_length(int iters, int most);
 
@@ -62,6 +71,9 @@ class Session {
     SmallRef small{};         // small heads-up subgames: iterations in one cooperative kernel
     int small_blocks = 0;     // its grid; 0: the captured iterations run
     unsigned small_fault = 0; // its fault word as last read: set until the state is reset
+    int sms = 0;
+    cudaEvent_t ev_done = nullptr;   // after the iterations queued last (small subgames)
+    bool in_flight = false;          // it was recorded and not yet seen to be reached (under the list's lock)
     const TermItem *term_items[SS_MAX_PLAYERS][TK_COUNT] = {};
     const int *term_heads[SS_MAX_PLAYERS][TK_COUNT] = {};   // null for kinds without P.term_heads
     const int *root_fr[SS_MAX_PLAYERS] = {};
@@ -102,6 +114,7 @@ class Session {
     cudaEvent_t ev_fork = nullptr, ev_join[TK_COUNT] = {};
 
     ~Session() {
+        leave_flights();
         if (graph) cudaGraphExecDestroy(graph);
         for (int k = 0; k < TK_COUNT; ++k) {
             if (side[k]) cudaStreamDestroy(side[k]);
@@ -144,12 +157,17 @@ class Session {
         return cudaSuccess;
     }
 
+    // A small subgame is launched kernel by kernel only beside others (crowded),
+    // so what counts there is the time on all SMs together: level by level, which
+    // is spread over short blocks, unless the tree pass is short.
+    bool levels() const { return small_blocks > 0 && P.node_hands > kLevelsAbove; }
+
     // Where traverser t has two-way showdowns, its one-opponent folds and zero
     // rows ride in their launch (rivers: tens of short blocks of each kind), as
     // long as that launch has large blocks.
     bool light(int t, int k) const {
         const size_t n = P.term[t][TK_SD1].size();
-        return n > 0 && n <= kSd1Few && (k == TK_SD1 || k == TK_CR1 || k == TK_ZERO);
+        return !levels() && n > 0 && n <= kSd1Few && (k == TK_SD1 || k == TK_CR1 || k == TK_ZERO);
     }
 
     // traverser t's terminals of kind k (grouped kinds: one block per head)
@@ -242,10 +260,11 @@ class Session {
         // the large value/regret levels, then the small levels of values and
         // reach in one launch, then the large reach levels
         const TreePass &T = P.tree[t];
+        const bool tree_pass = tree[t].n_stages > 0 && !levels();
         double tree_by = 0;
         int items = 0;
         for (size_t l = 0; l < cfv_lv[t].size(); ++l) {
-            if (static_cast<int>(l) >= T.cfv_from) {
+            if (tree_pass && static_cast<int>(l) >= T.cfv_from) {
                 tree_by += cfv_bytes[t][l];
                 items += cfv_lv[t][l].second;
                 continue;
@@ -256,13 +275,13 @@ class Session {
                                P.H[t], stream, nullptr, -1, iter_add);
             if (e != cudaSuccess) return e;
         }
-        if (tree[t].n_stages > 0) {
+        if (tree_pass) {
             for (int l = 0; l < T.reach_to; ++l) tree_by += reach_bytes[t][l];
             e = mark(PC_CFV, tree_by, items);
             if (e == cudaSuccess) e = launch_tree(c, tree[t], P.H[t], stream, iter_add);
             if (e != cudaSuccess) return e;
         }
-        return reach(t, static_cast<size_t>(T.reach_to));
+        return reach(t, tree_pass ? static_cast<size_t>(T.reach_to) : 0);
     }
 
     // iteration *iter + iter_add
@@ -307,6 +326,10 @@ class Session {
                             double *deal_mass) const;
     int reset();
     int run(int iters);
+    int run_launches(int iters);      // iterations kernel by kernel
+    bool crowded();                   // small subgames: whether its grid does not fit beside those in flight
+    int join_flights();               // marks what was just queued as in flight
+    void leave_flights();
     int output(SSOutput *out);
     int sync();
     int small_fault_error();          // the error of a session whose wait ran out
