@@ -1030,6 +1030,39 @@ def anchor_gpu(seed, device, solves=20):
             "kind": "ss_solve_gpu from host buffers (e2e), one B200"}
 
 
+def _context_usable():
+    """Whether the CUDA context still works after a failed leg (a sticky error,
+    such as an illegal address, ends every later call of the process)."""
+    import torch
+    try:
+        torch.cuda.synchronize()
+        torch.zeros(1, device="cuda").cpu()
+        return True
+    except RuntimeError:
+        return False
+
+
+class Legs:
+    """The legs beside the headline.  A leg that fails leaves its error in its
+    place and the next one runs, unless it took the CUDA context with it: the
+    legs after that are not run and say so."""
+
+    def __init__(self, forms, usable):
+        self.forms, self.usable, self.lost = forms, usable, None
+
+    def run(self, name, fn):
+        if name not in self.forms:
+            return None
+        if self.lost:
+            return {"error": f"not run: the CUDA context was lost in the leg {self.lost!r}"}
+        try:
+            return fn()
+        except Exception as e:  # the solver's line is printed whatever happens here
+            if not self.usable():
+                self.lost = name
+            return {"error": f"{type(e).__name__}: {e}"}
+
+
 def main():
     args = parse()
     if args.ncu_summary:
@@ -1076,49 +1109,22 @@ def main():
 
     forms = set(args.forms.split(","))
     res = run_ours(args, world, rank, local)
-    batched = served = None
-    if rank == 0 and world == 1 and "batched" in forms:
-        try:
-            batched = run_batched(args.batch_size, args.seed, local)
-        except Exception as e:  # the solver's line is printed whatever happens here
-            batched = {"error": f"{type(e).__name__}: {e}"}
-    if rank == 0 and world == 1 and "served" in forms:
-        try:
-            served = run_served([float(r) for r in args.rates.split(",")], args.served_requests, args.seed, local)
-        except Exception as e:  # the solver's line is printed whatever happens here
-            served = {"error": f"{type(e).__name__}: {e}"}
-    hu = None
-    if rank == 0 and world == 1 and "hu_river" in forms:
-        try:
-            hu = run_hu_river(args.seed, local)
-        except Exception as e:  # the solver's line is printed whatever happens here
-            hu = {"error": f"{type(e).__name__}: {e}"}
-    leaf = None
-    if rank == 0 and world == 1 and "leaf" in forms and args.workload == "turn3":
-        try:
-            leaf = run_leaf_producer(args.seed)
-        except Exception as e:  # the solver's line is printed whatever happens here
-            leaf = {"error": f"{type(e).__name__}: {e}"}
-    four = None
-    if rank == 0 and world == 1 and "four" in forms:
-        try:
-            four = run_four_player(args.seed, local)
-        except Exception as e:  # the solver's line is printed whatever happens here
-            four = {"error": f"{type(e).__name__}: {e}"}
-    flop = None
-    if rank == 0 and world == 1 and "flop" in forms:
-        try:
-            flop = run_flop(args.seed, local)
-        except Exception as e:  # the solver's line is printed whatever happens here
-            flop = {"error": f"{type(e).__name__}: {e}"}
-    anchor = None
-    if rank == 0 and world == 1 and "anchor" in forms and args.workload == "turn3":
-        try:
-            anchor = {"gpu": anchor_gpu(args.seed, local), "reference": anchor_reference(args.seed)}
-            if anchor["reference"]:
-                anchor["speedup"] = anchor["gpu"]["solves_per_s"] / anchor["reference"]["solves_per_s"]
-        except Exception as e:  # the solver's line is printed whatever happens here
-            anchor = {"error": f"{type(e).__name__}: {e}"}
+    legs = Legs(forms if rank == 0 and world == 1 else (), _context_usable)
+    turn3 = args.workload == "turn3"
+    batched = legs.run("batched", lambda: run_batched(args.batch_size, args.seed, local))
+    served = legs.run("served", lambda: run_served([float(r) for r in args.rates.split(",")], args.served_requests,
+                                                   args.seed, local))
+    hu = legs.run("hu_river", lambda: run_hu_river(args.seed, local))
+    leaf = legs.run("leaf", lambda: run_leaf_producer(args.seed)) if turn3 else None
+    four = legs.run("four", lambda: run_four_player(args.seed, local))
+    flop = legs.run("flop", lambda: run_flop(args.seed, local))
+
+    def run_anchor():
+        r = {"gpu": anchor_gpu(args.seed, local), "reference": anchor_reference(args.seed)}
+        if r["reference"]:
+            r["speedup"] = r["gpu"]["solves_per_s"] / r["reference"]["solves_per_s"]
+        return r
+    anchor = legs.run("anchor", run_anchor) if turn3 else None
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and args.workload == "turn3":
         r = reference_cpu(args.seed, budget_s=20.0)
@@ -1158,7 +1164,7 @@ def main():
             dist.destroy_process_group()
     except Exception:
         pass
-    return 0
+    return 1 if legs.lost else 0
 
 
 if __name__ == "__main__":
