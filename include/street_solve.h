@@ -277,7 +277,9 @@ int ss_session_iterations(const SSSession *session);
 int ss_session_output(SSSession *session, SSOutput *output);
 
 /* EXTENSION: run one more iteration as a graph with event nodes between the
- * kernel classes and report their device times and minimum bytes. */
+ * kernel classes and report their device times and minimum bytes.  (A small
+ * heads-up session, whose iterations otherwise run in one kernel, runs this one
+ * kernel by kernel, as it does beside many others.) */
 int ss_session_profile(SSSession *session, SSKernelProfile *profile);
 
 /* EXTENSION: the launches of the iteration the last ss_session_profile call

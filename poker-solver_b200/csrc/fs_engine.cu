@@ -14,9 +14,10 @@
 //     opponent's decisions and through chance nodes, whose average becomes a
 //     weight 1 / cards dealt folded into each frontier row when it is written
 //     (the items' `scale`), so k_cfv sums rows unchanged;
-//   * terminals: one warp per terminal over the opponent's reach row, with the
-//     ranges' tables or the river board's in the block's shared memory: sums
-//     per card and in strength order, then O(1) per traverser hand;
+//   * terminals: sums per card and in strength order over the opponent's reach
+//     row, then O(1) per traverser hand; one warp per terminal with the ranges'
+//     tables or the river board's in the block's shared memory, one block per
+//     terminal where a launch has few;
 //   * strengths and the tables by strength: once per solve for every river
 //     board of the tree on the device (k_fs_tables), instead of once per
 //     showdown node;

@@ -26,10 +26,12 @@
 // whose rows, columns and vectors are zero, so it drops out of every sum
 // (opponent hands never hold board cards).
 //
-// Each phase is a function of (thread index, thread count) whose work items
-// are independent within the phase; the kernel separates phases with block
-// barriers, and a host build runs them one after another (the check in
-// tests/native/cr3_emul.cpp).
+// k_term_sd3 runs gather_dev, build_step1, build_step2 and add_hands between
+// block barriers, and hand_part / d2_at, hand_count_part / c2_at,
+// hand_mass_cls_slice and e_pair_slice per hand.  The other functions are a host
+// form of the same sums -- phases of independent work items, one thread index at
+// a time, and whole sums per hand -- that tests/native builds compare with
+// enumeration; of the kernel's own, they share the per-hand ones.
 #pragma once
 
 #include <cmath>

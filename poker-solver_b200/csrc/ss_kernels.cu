@@ -1,11 +1,14 @@
 // ss_kernels.cu -- sm_100a kernels of the single-street Linear-CFR solver.
 //
-// Per-hand kernels (reach, cfv): one block per (work item, 256-hand chunk),
-// each thread owns 4 consecutive hands and moves them with 128-bit loads and
-// stores; rows are HS floats (HS a multiple of 32), so every warp touches
-// 512 contiguous bytes per row.
+// Per-hand kernels, over rows of HS floats (HS a multiple of 32): reach in
+// units of one work item and 256 hands, four to a block, four consecutive hands
+// per thread (128-bit loads and stores); values and regrets one pair of hands
+// per thread, items back to back; the small levels near the root in one launch
+// with eight hands per block (k_tree); a small heads-up subgame's whole
+// iterations in one cooperative kernel (k_small_solve).
 //
-// Per-terminal kernels: one block per terminal node.  The block stages the
+// Per-terminal kernels: one block per terminal node (several for a long
+// showdown sweep or a large range).  The block stages the
 // counted opponents' reach at that node in shared memory as 52x52 combo
 // matrices (or as a strength-sorted vector for showdowns), reduces them to
 // per-card aggregates, and then evaluates the exact card-removal formula for
@@ -1765,10 +1768,10 @@ __global__ void __launch_bounds__(kSd1Threads, 2) k_term_light(DevCtx c0, const 
 // kernel writes; what crosses the blocks is the reach rows (to the other
 // player's terminals) and the terminal rows, one L2 round trip each per phase.
 // Summation orders and expressions are those of the separate kernels.
-// Per iteration: heads-up river of 51 nodes and 1081 hands 34.4 us as launches,
-// 19.2 so (terminals 4.5 us, tree 3.3 us, two barriers 1.5 us each, twice); 141
-// nodes and 90 hands 35.8 -> 20.3; turn of 1,081 nodes and 1128 hands 58.6 ->
-// 42.5.
+// Per iteration: heads-up river of 51 nodes and 1081 hands 34.9 us as launches,
+// 18.0 so (with four items per block 19.5: terminals 4.5 us, tree 3.3 us, two
+// barriers 1.5 us each, twice); 141 nodes and 90 hands 35.5 -> 19.7; turn of
+// 1,081 nodes and 1128 hands 59 -> 38.9.
 // --------------------------------------------------------------------------
 constexpr int kSmallThreads = kSd1Threads;
 

@@ -9,8 +9,10 @@
 //
 // The pieces' buffers come from the library's pool of page-locked blocks
 // (host_block_take: bounded, shared by all threads, handed back on return);
-// nothing else outlives the call.  Both return when the host range is free to
-// reuse (up) or filled (down); the device side is ordered on the stream.
+// nothing else outlives the call.  Down returns when the host range is filled,
+// up when it is free to reuse, unless it is page-locked and small enough for the
+// plain call (then, as with that call, when the stream has got there); the
+// device side is ordered on the stream.
 #pragma once
 
 #include <cuda_runtime.h>
