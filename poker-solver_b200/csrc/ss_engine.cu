@@ -580,7 +580,8 @@ int Session::output(SSOutput *out) {
     if (e == cudaSuccess) e = fetch_small_fault();
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     unsigned fault = 0;
-    if (e == cudaSuccess) e = read_device_fault(&fault, stream);
+    // (the tensor-core product's word: a small subgame has no such terminals)
+    if (e == cudaSuccess && small_blocks == 0) e = read_device_fault(&fault, stream);
     if (e != cudaSuccess || fault || small_fault) {
         std::free(h_rs);
         std::free(h_rev);

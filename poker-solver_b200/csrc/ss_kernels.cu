@@ -2317,15 +2317,15 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
     int first_cr1[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        const int i = (static_cast<int>(blockIdx.x) - s.n_sd1[t]) * s.per_job[t] + group;
-        first_cr1[t] = i >= 0 && i < s.n_cr1[t] ? __ldg(s.cr1_head[t] + i) : 0;
+        const int j = static_cast<int>(blockIdx.x) - s.n_sd1[t], i = j + group * s.cr1_jobs[t];
+        first_cr1[t] = j >= 0 && i < s.n_cr1[t] ? __ldg(s.cr1_head[t] + i) : 0;
     }
     char *work = smem + s.at.phase;
     __syncthreads();
     for (int it = 1; it <= iters; ++it) {
         for (int t = 0; t < 2; ++t) {
             const int n_sd1 = s.n_sd1[t], n_cr1 = s.n_cr1[t], n_zero = s.n_zero[t];
-            const int per_job = s.per_job[t], cr1_jobs = (n_cr1 + per_job - 1) / per_job;
+            const int cr1_jobs = s.cr1_jobs[t];
             const int jobs = n_sd1 + cr1_jobs + (n_zero + kLightGroups - 1) / kLightGroups;
             for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
                 if (job < n_sd1) {
@@ -2335,8 +2335,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
                               reinterpret_cast<const short *>(smem + s.at.list),
                               reinterpret_cast<const int *>(smem + s.at.clen), job == static_cast<int>(blockIdx.x) ? first_sd1[t] : s.sd1[t][job], t, work);
                 } else if (job < n_sd1 + cr1_jobs) {
-                    const int i = (job - n_sd1) * per_job + group;
-                    if (group < per_job && i < n_cr1)
+                    const int i = job - n_sd1 + group * cr1_jobs;
+                    if (i < n_cr1)
                         small_cr1(c, reinterpret_cast<const unsigned *>(smem + s.at.fold[t]),
                                   reinterpret_cast<const short *>(smem + s.at.pair[1 - t]),
                                   s.cr1[t] + (job == static_cast<int>(blockIdx.x) ? first_cr1[t] : __ldg(s.cr1_head[t] + i)), t,
@@ -4161,15 +4161,14 @@ cudaError_t launch_tree(const DevCtx &c, const TreeRef &t, int H, cudaStream_t s
     return cudaGetLastError();
 }
 
-// The grid: a block per 8 hands and per terminal job, at most one per SM.  A
-// block takes one group of folds or leaves at a time if that needs no more
-// blocks than the hands do or than half the SMs (so that two sessions run side
-// by side), else two or four.  Groups, not items: the three other continuation
-// choices of a leaf follow its first, and items taken four by four left three
-// of four thread groups idle.  Microseconds per iteration in fours of items and
-// so: heads-up turn of 1,081 nodes 42.2 and 38.9, of 391 nodes and 300 hands
-// 25.6 and 25.9 (half the blocks), river of 51 nodes and 1,081 hands 19.7 and
-// 18.0.
+// The grid: a block per 8 hands and per terminal job, at most one per SM.  The
+// groups of folds or leaves are dealt one by one to as many blocks as that leaves
+// within what the hands ask for, or half the SMs if that is more (so that two
+// sessions run side by side), up to four to a block at a time.  Groups, not items:
+// the three other continuation choices of a leaf follow its first, and items
+// taken four by four left three of four thread groups idle.  Microseconds per
+// iteration in fours of items and so: heads-up turn of 1,081 nodes 42.2 and
+// 38.9, river of 51 nodes and 1,081 hands 19.7 and 18.0.
 int small_solve_blocks(const DevCtx &c, SmallRef *ref) {
     SmallRef &s = *ref;
     int dev = 0, coop = 0, sms = 0, optin = 0, per_sm = 0;
@@ -4189,11 +4188,10 @@ int small_solve_blocks(const DevCtx &c, SmallRef *ref) {
     int widest = 1;
     for (int t = 0; t < 2; ++t) {
         const int zeros = (s.n_zero[t] + kLightGroups - 1) / kLightGroups;
-        auto jobs_of = [&](int per) { return s.n_sd1[t] + (s.n_cr1[t] + per - 1) / per + zeros; };
         const int most = std::max((std::max(c.H[0], c.H[1]) + kTreeHands - 1) / kTreeHands, sms / 2);
-        s.per_job[t] = 1;
-        while (s.per_job[t] < kLightGroups && jobs_of(s.per_job[t]) > most) s.per_job[t] *= 2;
-        const int jobs = jobs_of(s.per_job[t]);
+        const int fewest = (s.n_cr1[t] + kLightGroups - 1) / kLightGroups;
+        s.cr1_jobs[t] = std::max(fewest, std::min(s.n_cr1[t], most - s.n_sd1[t] - zeros));
+        const int jobs = s.n_sd1[t] + s.cr1_jobs[t] + zeros;
         const int chunks = (c.H[t] + kTreeHands - 1) / kTreeHands;
         if (chunks > sms) return 0;   // a block owns 8 hands for the whole launch
         widest = std::max({widest, jobs, chunks});

@@ -121,7 +121,7 @@ struct SmallRef {
     const TermItem *sd1[2], *cr1[2], *zero[2];
     const int *cr1_head[2];   // the folds or leaves that start a group (TermItem::follow is not set)
     int n_sd1[2], n_cr1[2], n_zero[2];   // n_cr1: of cr1_head
-    int per_job[2];           // groups of folds or leaves that one block takes at a time
+    int cr1_jobs[2];          // blocks that the groups of folds or leaves are dealt to
     unsigned *barrier;   // grid barrier count
     unsigned *fault;     // not 0 once a barrier's wait ran out; the session's own
     unsigned polls;      // of a barrier before a block gives up
