@@ -2241,7 +2241,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_c
     const size_t HS = static_cast<size_t>(c.HS);
     const bool river = s.n_sd1[0] + s.n_sd1[1] > 0, folds = s.n_cr1[0] + s.n_cr1[1] > 0;
     const int hand = threadIdx.x & (kTreeHands - 1), h = blockIdx.x * kTreeHands + hand;
-    if (*s.fault) return;   // an earlier launch gave up: its rows are no state to go on from
+    // an earlier launch gave up: its rows are no state to go on from.  (One thread
+    // asks for the block: this launch's own blocks may set the word meanwhile, and
+    // the named barriers below count on every thread.)
+    if (__syncthreads_or(threadIdx.x == 0 && *s.fault != 0u)) return;
     float weight0 = 0.f, weight1 = 0.f;
     // tables and the block's rows
     for (int p = 0; p < 2; ++p) {

@@ -98,3 +98,13 @@ def test_server_iterates_past_released_members():
         assert a["stats"]["iterations_run"] == m["stats"]["iterations_run"]
     for sg in subs:
         sg.free()
+
+
+def test_small_solve_stops_block_by_block():
+    """k_small_solve waits at barriers that count threads, so whatever makes it
+    return before them is decided once for the block: its early returns follow a
+    block-wide vote or a grid barrier's shared answer."""
+    src = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "ss_kernels.cu")).read())
+    body = re.search(r"k_small_solve\(const __grid_constant__.*?\{(.*?)^\}", src, re.M | re.S).group(1)
+    returns = [line.strip() for line in body.split("\n") if re.search(r"\breturn;", line)]
+    assert returns and all("__syncthreads_or(" in r or "grid_barrier(" in r for r in returns), returns
